@@ -57,9 +57,8 @@ struct MatView {
     const int32_t *col;
     const float *val;
     const int32_t *rlen;  // entries of each row (coarse matrices), null: the slice width
-    const __half *hval;   // FP16 copy of val read by the cycle's fine-level kernels, or null
 };
-MatView view(const AmgMatrix &A) { return {A.n, A.slice_off, A.col, A.val, A.rlen, nullptr}; }
+MatView view(const AmgMatrix &A) { return {A.n, A.slice_off, A.col, A.val, A.rlen}; }
 
 // Rows longer than this (hub aggregates: a fracture intersection or a channel that couples to
 // every aggregate along it) are skipped by the thread-per-row kernels and handled by a block
@@ -844,12 +843,9 @@ __global__ void k_dense_gemv(Gate gate, const float *__restrict__ inv, int64_t n
 // (A x)_i.  On the fine level (no row lengths: 7-8 entries per row) the first 8 slots are
 // loaded together, then gathered together, so each thread keeps 8 independent loads in flight
 // instead of one dependent load chain per slot; coarse rows (longer, irregular) loop.
-// the fine level's row: slots loaded 8 at a time, values from FP32 or their FP16 copy
-template <bool HALF>
 // The slots are a stream read once per pass: loaded evict-first (ld.global.cs) so that they
 // do not push the gathered vector out of L2.
 __device__ __forceinline__ float fine_dot(const MatView &A, int64_t base, int w, int ln, const float *__restrict__ x) {
-    auto value = [&](int64_t slot) { return HALF ? __half2float(__ldcs(A.hval + slot)) : __ldcs(A.val + slot); };
     constexpr int kB = 8;
     int32_t c[kB];
     float v[kB];
@@ -857,7 +853,7 @@ __device__ __forceinline__ float fine_dot(const MatView &A, int64_t base, int w,
     for (int k = 0; k < kB; ++k) {
         const int64_t slot = base + (int64_t)k * kS + ln;
         c[k] = k < w ? __ldcs(A.col + slot) : 0;
-        v[k] = k < w ? value(slot) : 0.f;
+        v[k] = k < w ? __ldcs(A.val + slot) : 0.f;
     }
     float g[kB];
 #pragma unroll
@@ -867,7 +863,7 @@ __device__ __forceinline__ float fine_dot(const MatView &A, int64_t base, int w,
     for (int k = 0; k < kB; ++k) y += v[k] * g[k];
     for (int j = kB; j < w; ++j) {
         const int64_t slot = base + (int64_t)j * kS + ln;
-        y += value(slot) * x[__ldcs(A.col + slot)];
+        y += __ldcs(A.val + slot) * x[__ldcs(A.col + slot)];
     }
     return y;
 }
@@ -884,7 +880,7 @@ __device__ __forceinline__ float row_dot(const MatView &A, int64_t i, const floa
         }
         return y;
     }
-    return A.hval ? fine_dot<true>(A, base, w, ln, x) : fine_dot<false>(A, base, w, ln, x);
+    return fine_dot(A, base, w, ln, x);
 }
 
 // Coarse rows are long (tens of entries), so one thread walking a row issues a long chain of
@@ -1003,8 +999,9 @@ __global__ void __launch_bounds__(256) k_sm_step(Gate gate, MatView A, const flo
     x_out[i] = x_in[i] + dn;
 }
 
-// The fine level's first two Chebyshev steps from x = 0 in one pass (unit diagonal):
-// x1 = c0 b (so A x1 = c0 A b), d = c1 c0 b + c2 (b - c0 A b), x_out = x1 + d
+// The fine level's first two Chebyshev steps from x = 0 in one pass (unit diagonal), FP32 values
+// (half_fine = 0; k_fine otherwise): x1 = c0 b (so A x1 = c0 A b), d = c1 c0 b + c2 (b - c0 A b),
+// x_out = x1 + d
 __global__ void k_sm_first_step(Gate gate, MatView A, const float *__restrict__ b, float *__restrict__ x_out,
                                 float *__restrict__ d, float c0, float c1, float c2, const int32_t *__restrict__ agg) {
     if (closed(gate)) return;
@@ -1044,8 +1041,7 @@ __global__ void k_sm_first_step_w(Gate gate, MatView A, const float *__restrict_
     for (int j = 0; j < wd; ++j) {
         const int64_t slot = base + (int64_t)j * kS + ln;
         const int32_t c = __ldg(A.col + slot);
-        const float v = A.hval ? __half2float(A.hval[slot]) : __ldg(A.val + slot);
-        y += v * (w[c] * b[c]);
+        y += __ldg(A.val + slot) * (w[c] * b[c]);
     }
     const float wi = w[i];
     const float x1 = c0 * wi * bi;
@@ -1228,6 +1224,136 @@ __global__ void __launch_bounds__(256) k_coarse_dots(Gate gate, MatView A, const
     }
 }
 
+// The fine level's update arithmetic, rounding for rounding the same in every kernel that has it
+// (explicit fma: the compiler's choice of contractions depends on the code around).
+// x1 = c0 w b, d = c1 x1 + c2 w (b - c0 y): the sequence's first two steps, y = (S^ W b)_i
+__device__ __forceinline__ float fine_first(float b, float w, float y, float c0, float c1, float c2, float &x1) {
+    x1 = __fmul_rn(__fmul_rn(c0, w), b);
+    return __fmaf_rn(__fmul_rn(c2, w), __fmaf_rn(-c0, y, b), __fmul_rn(c1, x1));
+}
+// d = c1 d + c2 w (b - y): a later step, y = (S^ x)_i
+__device__ __forceinline__ float fine_step(float b, float w, float y, float d, float c1, float c2) {
+    return __fmaf_rn(__fmul_rn(c2, w), __fadd_rn(b, -y), __fmul_rn(c1, d));
+}
+
+// ---- the fine level's cycle kernels -----------------------------------------------------------
+// The scaled fine level has unit diagonal, held in every row's first slot and not read; the values
+// of the other slots are FP16.  A row is a chain of dependent loads -- slice offset, slots,
+// gathers of x -- and with one row per thread the chip waits on that chain at half its DRAM rate.
+// So the warps are persistent (a tile of 8 slices per block and turn) and pipelined: while the
+// gathers of a tile are under way, the slots and own-row entries of the next one and the slice
+// offset of the one after are too.
+// Rows outside the hierarchy are one bit each (a word per slice).
+// Measured (B200, us a kernel, one row per thread with the diagonal read -> this): 3.19M rows 39-42 ->
+// 29 (52 bytes a row at 5.7 TB/s), 10.95M rows 139-150 -> 107-122.  16-bit columns relative to
+// two bases per slot position (26 bytes a row's slots instead of 36) were no faster unpipelined
+// (37-39, 154-163) and lost the pipeline where decoding waits for the bases.
+struct FineView {
+    int64_t n_slices;
+    const int64_t *off;
+    const int32_t *col;
+    const __half *hval;
+    const uint32_t *outside;  // per slice: the rows outside the hierarchy
+};
+
+__global__ void k_outside_bits(int64_t n, const int32_t *__restrict__ agg, uint32_t *__restrict__ bits) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;  // n is a multiple of 32
+    if (i >= n) return;
+    const unsigned m = __ballot_sync(kFull, agg[i] < 0);
+    if ((threadIdx.x & 31) == 0) bits[i / kS] = m;
+}
+
+constexpr int kFn = 6;  // off-diagonal slots loaded together: all of a tetrahedron face's row
+enum FineOp : int { kOpFirst, kOpFirstW, kOpStep, kOpResid };
+
+// OP kOpFirst (kOpFirstW with smoother weights w): the first two Chebyshev steps from x = 0
+// (fine_first) on x = b; kOpStep: one step (fine_step); kOpResid: out = b - S^ x.
+// RD: the step continues a sequence (reads d); WD: a later step reads the d written here.
+template <int OP, bool RD, bool WD>
+__global__ void __launch_bounds__(256, 4) k_fine(Gate gate, FineView A, const float *__restrict__ b,
+                                                 const float *__restrict__ w, const float *__restrict__ x,
+                                                 float *__restrict__ out, float *__restrict__ d, float c0, float c1,
+                                                 float c2) {
+    constexpr bool first = OP == kOpFirst || OP == kOpFirstW;
+    const int lane = threadIdx.x & 31;
+    const int64_t step = (int64_t)gridDim.x * 8;
+    int64_t sl = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (sl >= A.n_slices) return;
+    struct Stage {
+        int64_t off;
+        int wd;
+        int32_t c[kFn];
+        __half v[kFn];
+        float xi, bi, wi, di;
+        uint32_t outside;
+    } st;
+    auto load = [&](int64_t s, int64_t o, int64_t o2) {
+        st.off = o;
+        st.wd = (int)((o2 - o) / kS);
+#pragma unroll
+        for (int k = 0; k < kFn; ++k) {
+            const int64_t slot = o + (int64_t)(k + 1) * kS + lane;
+            st.c[k] = k + 1 < st.wd ? __ldcs(A.col + slot) : 0;
+            st.v[k] = k + 1 < st.wd ? __ldcs(A.hval + slot) : __ushort_as_half(0);
+        }
+        const int64_t i = s * kS + lane;
+        st.xi = x[i];
+        st.bi = first ? st.xi : b[i];
+        st.wi = (OP == kOpFirstW || (OP == kOpStep && w)) ? w[i] : 1.f;
+        st.di = RD ? d[i] : 0.f;
+        st.outside = OP == kOpResid ? 0u : __ldg(A.outside + s);
+    };
+    load(sl, A.off[sl], A.off[sl + 1]);
+    int64_t s1 = sl + step, o1 = 0, o2 = 0;
+    if (s1 < A.n_slices) {
+        o1 = A.off[s1];
+        o2 = A.off[s1 + 1];
+    }
+    if (closed(gate)) return;
+    for (;;) {
+        float g[kFn];
+#pragma unroll
+        for (int k = 0; k < kFn; ++k) {
+            g[k] = k + 1 < st.wd ? x[st.c[k]] : 0.f;
+            if (OP == kOpFirstW) g[k] *= k + 1 < st.wd ? w[st.c[k]] : 0.f;
+        }
+        const Stage cur = st;
+        const int64_t i = sl * kS + lane;
+        sl = s1;
+        if (sl < A.n_slices) {
+            load(sl, o1, o2);
+            s1 = sl + step;
+            if (s1 < A.n_slices) {
+                o1 = A.off[s1];
+                o2 = A.off[s1 + 1];
+            }
+        }
+        float y = 0.f;
+#pragma unroll
+        for (int k = 0; k < kFn; ++k) y = __fmaf_rn(__half2float(cur.v[k]), g[k], y);
+        for (int j = kFn + 1; j < cur.wd; ++j) {
+            const int64_t slot = cur.off + (int64_t)j * kS + lane;
+            const int32_t c = __ldcs(A.col + slot);
+            y = __fmaf_rn(__half2float(__ldcs(A.hval + slot)), OP == kOpFirstW ? w[c] * x[c] : x[c], y);
+        }
+        y = __fadd_rn(y, OP == kOpFirstW ? __fmul_rn(cur.wi, cur.xi) : cur.xi);  // the diagonal
+        const bool outside = cur.outside >> lane & 1u;  // a row outside the hierarchy: exact
+        if (OP == kOpResid) {
+            out[i] = __fadd_rn(cur.bi, -y);
+        } else if (first) {
+            float x1;
+            const float dn = fine_first(cur.bi, cur.wi, y, c0, c1, c2, x1);
+            if (WD) d[i] = outside ? 0.f : dn;
+            out[i] = outside ? cur.bi : x1 + dn;
+        } else {
+            const float dn = fine_step(cur.bi, cur.wi, y, cur.di, RD ? c1 : 0.f, c2);
+            if (WD) d[i] = outside ? 0.f : dn;
+            out[i] = outside ? cur.wi * cur.bi : cur.xi + dn;
+        }
+        if (sl >= A.n_slices) return;
+    }
+}
+
 // ---- fine-level smoothing with the matrix streamed by TMA bulk copies ----------------------
 // The fine level's row kernels are one long stream of SELL slots (column index and FP16 value,
 // 6 bytes a slot) plus gathers of x[col] that mostly hit L2.  In the thread-per-row kernels each
@@ -1236,8 +1362,7 @@ __global__ void __launch_bounds__(256) k_coarse_dots(Gate gate, MatView A, const
 // (256 rows) through a ring of NST shared-memory stages with 1D bulk copies (cp.async.bulk,
 // completion counted on an mbarrier), so the DRAM stream runs NST - 1 tiles ahead of the warps,
 // which read their slots from shared memory and only wait on the gathers.  The row arithmetic
-// and its summation order are those of k_sm_first_step, k_sm_step<1> and k_residual<1>
-// (bit-identical results).  Measured, it is no faster: the gathers, not the slots, set the
+// and its summation order are those of k_fine (bit-identical results).  Measured, it is no faster: the gathers, not the slots, set the
 // latency, and the stages halve the threads per SM (fine_tma, off by default).  Every wait is
 // bounded: a stage that does not complete in kFineSpin polls sets *err, and the CTA waits
 // (bounded again) for its copies in flight before it returns.
@@ -1348,27 +1473,27 @@ __global__ void __launch_bounds__(256) k_fine_tma(Gate gate, FineTma F, const fl
 #pragma unroll
             for (int q = 0; q < kB; ++q) {
                 c[q] = q < w ? cs[q * kS] : 0;
-                v[q] = q < w ? __half2float(vs[q * kS]) : 0.f;
+                v[q] = q > 0 && q < w ? __half2float(vs[q * kS]) : 0.f;
             }
             float g[kB];
 #pragma unroll
             for (int q = 0; q < kB; ++q) g[q] = q < w ? xg[c[q]] : 0.f;
             float y = 0.f;
 #pragma unroll
-            for (int q = 0; q < kB; ++q) y += v[q] * g[q];
-            for (int j = kB; j < w; ++j) y += __half2float(vs[j * kS]) * xg[cs[j * kS]];
+            for (int q = 0; q < kB; ++q) y = __fmaf_rn(v[q], g[q], y);
+            for (int j = kB; j < w; ++j) y = __fmaf_rn(__half2float(vs[j * kS]), xg[cs[j * kS]], y);
             if (i < F.n) {
+                y = __fadd_rn(y, xg[i]);  // the unit diagonal last, as in k_fine
                 if (MODE == kFineResid) {
-                    x_out[i] = b[i] - y;
+                    x_out[i] = __fadd_rn(b[i], -y);
                 } else if (MODE == kFineFirst) {
                     const float bi = b[i];
                     if (agg && agg[i] < 0) {
                         d[i] = 0.f;
                         x_out[i] = bi;
                     } else {
-                        const float x1 = c0 * bi;
-                        const float r = bi - c0 * y;
-                        const float dn = c1 * x1 + c2 * r;
+                        float x1;
+                        const float dn = fine_first(bi, 1.f, y, c0, c1, c2, x1);
                         d[i] = dn;
                         x_out[i] = x1 + dn;
                     }
@@ -1378,8 +1503,7 @@ __global__ void __launch_bounds__(256) k_fine_tma(Gate gate, FineTma F, const fl
                         d[i] = 0.f;
                         x_out[i] = di * b[i];
                     } else {
-                        const float r = b[i] - y;
-                        const float dn = (c1 != 0.f ? c1 * d[i] : 0.f) + c2 * di * r;
+                        const float dn = fine_step(b[i], di, y, c1 != 0.f ? d[i] : 0.f, c1, c2);
                         d[i] = dn;
                         x_out[i] = x_in[i] + dn;
                     }
@@ -1812,6 +1936,7 @@ void Amg::release() {
     tickets_.release();
     w0_.release();
     fine_half_.release();
+    fine_out_.release();
     w0_used_ = nullptr;
     isd_.release();
     dense_inv_.release();
@@ -2272,6 +2397,15 @@ cudaError_t Amg::setup(const DevSystem &sys, const AmgOptions &o, cudaStream_t s
         AMG_CK(cudaGetLastError());
     }
     w0_used_ = w0;
+    if (opt_.half_fine && n_levels_ > 1) {
+        int dev = 0, sms = 0;
+        AMG_CK(cudaGetDevice(&dev));
+        AMG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        fine_grid_ = 4 * sms;  // k_fine: four blocks to an SM
+        AMG_CK(fine_out_.ensure(L0.A.n_slices));
+        k_outside_bits<<<nblk(L0.A.n, 256), 256, 0, s>>>(L0.A.n, L0.agg.p, fine_out_.p);
+        AMG_CK(cudaGetLastError());
+    }
     // partial sums of the coarse-correction scaling, one slice per level
     dots_off_.assign(n_levels_, 0);
     int64_t tot = 0;
@@ -2714,13 +2848,23 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
     const bool use_tail = tail_phases_ > 0 && tail_level_ > l0;
     // the fine level's kernels stream its FP16 matrix through shared memory (k_fine_tma)
     const bool tma0 = fine_tma_ && opt_.half_fine && l0 == 0;
+    const bool half0 = opt_.half_fine && !tma0 && nl > 1;
+    const FineView F{lv_[0].A.n_slices, lv_[0].A.slice_off, lv_[0].A.col,
+                     reinterpret_cast<const __half *>(fine_half_.p), fine_out_.p};
+    const unsigned gf = (unsigned)std::min<int64_t>((F.n_slices + 7) / 8, fine_grid_);
+    // a Chebyshev step of the fine level; more: a later step of the sequence reads d
+    auto fine_step0 = [&](const float *b, const float *w, const float *xi, float *xo, float *d, float c1, float c2,
+                          bool more) {
+        const auto f = c1 != 0.f ? (more ? k_fine<kOpStep, true, true> : k_fine<kOpStep, true, false>)
+                                 : (more ? k_fine<kOpStep, false, true> : k_fine<kOpStep, false, false>);
+        f<<<gf, 256, 0, s>>>(gate_, F, b, w, xi, xo, d, 0.f, c1, c2);
+    };
     for (int l = l0; l < (use_tail ? tail_level_ : nl - 1); ++l) {
         AmgLevel &L = lv_[l];
         const float *b = l == 0 ? r : L.b.p;
         // the scaled fine level has unit diagonal; with smoother weights Omega, D^-1 -> Omega
         const float *invd = l == 0 ? fw() : L.inv_diag.p;
-        MatView A = view(L.A);
-        if (l == 0 && opt_.half_fine) A.hval = reinterpret_cast<const __half *>(fine_half_.p);
+        const MatView A = view(L.A);
         const unsigned g = nblk(L.A.n, 256), gs = row_blocks(L);
         const auto sm_step = sm_step_kernel(L.g);
         cheb_coeffs(L, c1, c2);
@@ -2728,7 +2872,11 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
         int k0 = 1;
         if (l == 0 && pre >= 2) {  // first two steps in one pass
             rec_step(true);
-            if (fine_w_)
+            if (opt_.half_fine && (fine_w_ || !tma0)) {
+                const auto f = fine_w_ ? (pre > 2 ? k_fine<kOpFirstW, false, true> : k_fine<kOpFirstW, false, false>)
+                                       : (pre > 2 ? k_fine<kOpFirst, false, true> : k_fine<kOpFirst, false, false>);
+                f<<<gf, 256, 0, s>>>(gate_, F, b, fw(), b, xo, L.d.p, (float)c2[0], (float)c1[1], (float)c2[1]);
+            } else if (fine_w_)
                 k_sm_first_step_w<<<g, 256, 0, s>>>(gate_, A, b, fw(), xo, L.d.p, (float)c2[0], (float)c1[1],
                                                     (float)c2[1], L.agg.p);
             else if (tma0)
@@ -2748,6 +2896,8 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
             if (l == 0) rec_step(true);
             if (l == 0 && tma0)
                 launch_fine<kFineStep>(n_done, n_inst, b, invd, xi, xo, L.d.p, 0.f, (float)c1[k], (float)c2[k], s);
+            else if (l == 0 && half0)
+                fine_step0(b, invd, xi, xo, L.d.p, (float)c1[k], (float)c2[k], k + 1 < pre);
             else
                 sm_step<<<gs, 256, 0, s>>>(gate_, A, b, invd, xi, xo, L.d.p, (float)c1[k], (float)c2[k], L.agg.p);
             long_rows(L.A, 0, b, invd, xi, xo, L.d.p, (float)c1[k], (float)c2[k], nullptr);
@@ -2757,6 +2907,8 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
         xout[l] = xi;
         if (l == 0 && tma0)
             launch_fine<kFineResid>(n_done, n_inst, b, nullptr, xi, L.r.p, nullptr, 0.f, 0.f, 0.f, s);
+        else if (l == 0 && half0)
+            k_fine<kOpResid, false, false><<<gf, 256, 0, s>>>(gate_, F, b, nullptr, xi, L.r.p, nullptr, 0.f, 0.f, 0.f);
         else
             residual_kernel(L.g)<<<gs, 256, 0, s>>>(gate_, A, b, xi, L.r.p);
         long_rows(L.A, 1, b, nullptr, xi, L.r.p, nullptr, 0.f, 0.f, nullptr);
@@ -2807,8 +2959,7 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
         AmgLevel &L = lv_[l];
         const float *b = l == 0 ? r : L.b.p;
         const float *invd = l == 0 ? fw() : L.inv_diag.p;
-        MatView A = view(L.A);
-        if (l == 0 && opt_.half_fine) A.hval = reinterpret_cast<const __half *>(fine_half_.p);
+        const MatView A = view(L.A);
         const unsigned g = nblk(L.A.n, 256), gs = row_blocks(L);
         const auto sm_step = sm_step_kernel(L.g);
         cheb_coeffs(L, c1, c2);
@@ -2835,6 +2986,8 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
             if (l == 0 && tma0)
                 launch_fine<kFineStep>(n_done, n_inst, b, invd, xi, xo, L.d.p, 0.f, k == 0 ? 0.f : (float)c1[k],
                                        (float)c2[k], s);
+            else if (l == 0 && half0)
+                fine_step0(b, invd, xi, xo, L.d.p, k == 0 ? 0.f : (float)c1[k], (float)c2[k], k + 1 < deg);
             else
                 sm_step<<<gs, 256, 0, s>>>(gate_, A, b, invd, xi, xo, L.d.p, k == 0 ? 0.f : (float)c1[k],
                                            (float)c2[k], L.agg.p);
@@ -2872,8 +3025,7 @@ cudaError_t Amg::smooth_fine(const float *b, float *x, cudaStream_t s) {
     cheb_coeffs(L, c1, c2);
     const int pre = pre_degree();
     const float *invd = fw();
-    MatView A = view(L.A);
-    if (opt_.half_fine) A.hval = reinterpret_cast<const __half *>(fine_half_.p);
+    const MatView A = view(L.A);
     const int32_t *agg = n_levels_ > 1 ? L.agg.p : nullptr;
     const Gate g{nullptr, 0};
     float *xi = L.xa.p, *xo = L.xb.p;

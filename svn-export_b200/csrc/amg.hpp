@@ -214,6 +214,8 @@ private:
     DBuf<double> pw_part_, pw_sums_;  // its per-block partial norms and the two norms per level
     DBuf<float> w0_;                // sqrt(diag S) per fine row
     DBuf<uint16_t> fine_half_;      // FP16 bits of the fine matrix's values (half_fine)
+    DBuf<uint32_t> fine_out_;       // per fine slice, the rows outside the hierarchy
+    int64_t fine_grid_ = 1;         // blocks of the fine level's persistent kernels at most
     // the fine level's TMA-staged cycle kernels (k_fine_tma): ready, stage size, grid, the
     // widest tile read at setup and the stage-wait error flag
     bool fine_tma_ = false;

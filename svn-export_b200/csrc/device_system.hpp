@@ -43,7 +43,8 @@ struct DevPlan {
     int32_t *blk_inst = nullptr, *tile_begin = nullptr, *tile_end = nullptr, *inst_blk = nullptr;
 };
 
-// SELL-C-sigma matrix view in solver-row space (rows padded per instance to whole tiles).
+// SELL-C-sigma matrix view in solver-row space (rows padded per instance to whole tiles).  Every
+// row holds its diagonal in its first slot.
 template <typename T> struct SellView {
     int64_t n_rows;
     const int64_t *slice_off;  // [n_slices+1] first slot of each 32-row slice

@@ -2434,8 +2434,9 @@ int mh_get_schur_system(const mh_handle *hc, int32_t *row_ptr, int32_t *col, dou
         const int64_t sl = r / mh::kSliceRowsHost, lane = r % mh::kSliceRowsHost;
         const int64_t off = hs.slice_off[sl];
         for (int64_t j = 0; j < hs.row_ptr[r + 1] - hs.row_ptr[r]; ++j) {
-            if (col) col[k] = hs.row_edge[hs.row_col[hs.row_ptr[r] + j]];
-            if (val) val[k] = v[off + j * mh::kSliceRowsHost + lane];
+            const int32_t c = hs.row_col[hs.row_ptr[r] + j];
+            if (col) col[k] = hs.row_edge[c];
+            if (val) val[k] = v[off + mh::sell_pos(r, c, j) * mh::kSliceRowsHost + lane];
             ++k;
         }
         if (row_ptr) row_ptr[e + 1] = (int32_t)k;
@@ -2870,13 +2871,20 @@ int mh_amg_level(const mh_handle *hc, int32_t level, int64_t *n, int64_t *nnz, i
     for (int64_t i = 0; i < real; ++i) {
         const int64_t sl = i / mh::kSliceRowsHost, ln = i % mh::kSliceRowsHost;
         const int64_t w = (off[sl + 1] - off[sl]) / mh::kSliceRowsHost;
-        for (int64_t j = 0; j < w; ++j) {
+        auto put = [&](int64_t j) {
             const int64_t slot = off[sl] + j * mh::kSliceRowsHost + ln;
-            if (v[slot] == 0.f) continue;
+            if (v[slot] == 0.f) return;
             if (col) col[k] = c[slot];
             if (val) val[k] = v[slot];
             ++k;
+        };
+        // columns ascending: the fine level's rows hold their diagonal in front
+        int64_t j = 0;
+        if (level == 0) {
+            for (j = 1; j < w && c[off[sl] + j * mh::kSliceRowsHost + ln] < i; ++j) put(j);
+            put(0);
         }
+        for (; j < w; ++j) put(j);
         if (row_ptr) row_ptr[i + 1] = (int32_t)k;
     }
     if (n) *n = real;

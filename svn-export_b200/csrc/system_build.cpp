@@ -234,14 +234,14 @@ int build_host_system(const MeshData &m, const Topology &t, const std::vector<in
         int64_t off = hs.slice_off[s], w = (hs.slice_off[s + 1] - off) / kSliceRowsHost;
         for (int64_t j = 0; j < w; ++j) {
             int32_t c = (j < len[r]) ? hs.row_col[hs.row_ptr[r] + j] : (int32_t)r;
-            hs.sell_col[off + j * kSliceRowsHost + lane] = c;
-            if (j < len[r] && c == r) hs.diag_slot[r] = (int32_t)(off + j * kSliceRowsHost + lane);
+            hs.sell_col[off + (j < len[r] ? sell_pos(r, c, j) : j) * kSliceRowsHost + lane] = c;
         }
+        hs.diag_slot[r] = (int32_t)(off + lane);
     }
     auto slot_of = [&](int64_t r, int32_t c) -> int64_t {
         auto b = hs.row_col.begin() + hs.row_ptr[r], e = hs.row_col.begin() + hs.row_ptr[r + 1];
         int64_t j = std::lower_bound(b, e, c) - b;
-        return hs.slice_off[r / kSliceRowsHost] + j * kSliceRowsHost + r % kSliceRowsHost;
+        return hs.slice_off[r / kSliceRowsHost] + sell_pos(r, c, j) * kSliceRowsHost + r % kSliceRowsHost;
     };
 
     // the extra blocks' values summed per slot in group order (the host does it once)
@@ -414,12 +414,12 @@ int build_host_system_csr(int64_t n, const int32_t *row_ptr, const int32_t *col,
         const int64_t off = hs.slice_off[sl], w = (hs.slice_off[sl + 1] - off) / kSliceRowsHost;
         const int64_t len = hs.row_ptr[r + 1] - hs.row_ptr[r];
         for (int64_t j = 0; j < w; ++j) {
-            const int64_t slot = off + j * kSliceRowsHost + lane;
             const int32_t c = j < len ? hs.row_col[hs.row_ptr[r] + j] : (int32_t)r;
+            const int64_t slot = off + (j < len ? sell_pos(r, c, j) : j) * kSliceRowsHost + lane;
             hs.sell_col[slot] = c;
-            if (j < len && c == r) hs.diag_slot[r] = (int32_t)slot;
             if (j < len && r < n) hs.csr_slot[hs.row_ptr[r] + j] = (int32_t)slot;
         }
+        hs.diag_slot[r] = (int32_t)(off + lane);
     }
     hs.slot_cstart.assign(hs.n_slots + 1, 0);
     hs.row_cstart.assign(pad + 1, 0);

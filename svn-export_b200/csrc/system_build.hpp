@@ -11,6 +11,10 @@
 
 namespace mh {
 
+// Slot within its row of the j-th smallest column c of row r: the diagonal comes first (kernels
+// that know it skip its slot), the others follow in ascending order.
+inline int64_t sell_pos(int64_t r, int32_t c, int64_t j) { return c == r ? 0 : c < r ? j + 1 : j; }
+
 struct HostSystem {
     // instances: element ranges [inst_el[i], inst_el[i+1])
     std::vector<int64_t> inst_el;
