@@ -77,80 +77,154 @@ __device__ __forceinline__ void finish_inst(InstCtl *c, int status, int32_t *n_d
     atomicAdd(n_done, 1);
 }
 
-// a = (S^ h)[row] with float4 node states (FIRST: h = (r, 0, 0, 0) from a scalar vector)
-template <bool FIRST>
-__device__ __forceinline__ float4 aggregate(const SellView<float> &A, const float *__restrict__ r,
-                                            const float4 *__restrict__ h, int64_t sl, int lane) {
+// (S^ v)[row]
+__device__ __forceinline__ float sell_row_dot(const SellView<float> &A, const float *__restrict__ v, int64_t sl,
+                                              int lane) {
     const int64_t off = A.slice_off[sl];
     const int w = (int)((A.slice_off[sl + 1] - off) / kSliceRows);
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float acc = 0.f;
     for (int j = 0; j < w; ++j) {
         const int64_t slot = off + (int64_t)j * kSliceRows + lane;
-        const float v = __ldcs(A.val + slot);
-        const int32_t c = __ldcs(A.col + slot);
-        if (FIRST) {
-            acc.x += v * r[c];
-        } else {
-            const float4 hc = h[c];
-            acc.x += v * hc.x;
-            acc.y += v * hc.y;
-            acc.z += v * hc.z;
-            acc.w += v * hc.w;
-        }
+        acc += __ldcs(A.val + slot) * v[__ldcs(A.col + slot)];
     }
     return acc;
 }
 
-// One layer of the network for the rows of the block's tiles (R = 1 tiles of 256 rows).
-// FIRST: the input is the scalar residual; LAST: only channel 0 of the output is stored, as
-// z, and the partial dot z.q_old of flexible CG is reduced (beta = z.q_old / (p.q)_old).
 // ---- flexible CG ------------------------------------------------------------------------
-// p = z - beta p; partial p.r -> rho (alpha = p.r / p.q is then formed by the SpMV kernel).
-__global__ void __launch_bounds__(kBlockThreads)
-    k_fcg_direction(const float *__restrict__ z, const float *__restrict__ r, float *__restrict__ p,
-                    double *__restrict__ partial, InstCtl *__restrict__ ctl, Plan plan, int32_t *n_done) {
+// One iteration after z = M r is two kernels (beta, the direction, S^ p and the update as kernels of
+// their own were four, and each ends in a last-block reduction that the next one waits for):
+//   k_fcg_spmv:   s = S^ z with the sums z.q, z.r, p.r, z.s over the previous direction (p, q = S^ p);
+//                 the last block forms beta = z.q / p.q, the new direction's p.r = z.r - beta p.r and
+//                 p.q = z.s - beta z.q (S^ is symmetric and z.S^ p = z.q), alpha = p.r / p.q;
+//   k_fcg_update: p = z - beta p, q = s - beta q, x += alpha p, r -= alpha q, r.r, stopping test.
+// q follows the direction's recurrence instead of a product with the new p: the same to a rounding
+// in FP32, and the FP64 residual at the end of the run does not use it.
+// Both move the bytes that the four did (60 a row and the matrix); the row entries go four to a
+// load in the update and are loaded a tile ahead with the slots in the product.
+// The blocks of an instance take its tiles in turn (solver.cu, Tiles).
+// Measured (B200, us an iteration without the preconditioner, four kernels over neighbouring tiles
+// -> these): 52k rows 20 -> 11, 3.2M 96 -> 68, 10.9M 381 -> 233 (the update at 6.3 TB/s).
+struct FcgStage {
+    static constexpr int kJ = 6;
+    int64_t off;
+    int w;
+    int32_t c[kJ];
+    float v[kJ];
+    float dg, z, r, p, q;
+};
+
+__device__ __forceinline__ void fcg_stage_load(const SellView<float> &A, const float *__restrict__ z,
+                                               const float *__restrict__ r, const float *__restrict__ p,
+                                               const float *__restrict__ q, bool have, int tile, FcgStage &st) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t sl = (int64_t)tile * kWarpsPerBlock + warp, row = sl * kSliceRows + lane;
+    st.off = A.slice_off[sl];
+    st.w = (int)((A.slice_off[sl + 1] - st.off) / kSliceRows);
+    st.dg = __ldcs(A.val + st.off + lane);  // a row's first slot is its diagonal
+#pragma unroll
+    for (int j = 0; j < FcgStage::kJ; ++j) {
+        const bool in = j + 1 < st.w;
+        const int64_t slot = st.off + (int64_t)(j + 1) * kSliceRows + lane;
+        st.c[j] = in ? __ldcs(A.col + slot) : 0;
+        st.v[j] = in ? __ldcs(A.val + slot) : 0.f;
+    }
+    st.z = z[row];
+    st.r = r[row];
+    st.p = have ? p[row] : 0.f;
+    st.q = have ? q[row] : 0.f;
+}
+
+__global__ void __launch_bounds__(kBlockThreads, 4)
+    k_fcg_spmv(SellView<float> A, const float *__restrict__ z, const float *__restrict__ r,
+               const float *__restrict__ p, const float *__restrict__ q, float *__restrict__ s,
+               double *__restrict__ partial, InstCtl *__restrict__ ctl, Plan plan, int32_t *n_done) {
     const int inst = plan.inst[blockIdx.x];
     InstCtl *c = ctl + inst;
     if (c->done) return;
-    const double beta = c->beta;
-    double pr = 0.0;
-    for (int tile = plan.tile_begin[blockIdx.x]; tile < plan.tile_end[blockIdx.x]; ++tile) {
-        const int64_t row = (int64_t)tile * kBlockThreads + threadIdx.x;
-        // beta = 0 starts a new direction sequence: p is not read (it may hold a broken one)
-        const float pn = beta == 0.0 ? z[row] : (float)((double)z[row] - beta * (double)p[row]);
-        p[row] = pn;
-        pr += (double)pn * (double)r[row];
+    const double pq_old = c->aux[0];
+    const bool have = c->aux[1] != 0.0 && pq_old != 0.0;  // else (p, q) may hold a broken direction
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // the instance's blocks take its tiles in turn, so that all of them gather from one moving window
+    const int pb = plan.inst_blk[inst], nb = plan.inst_blk[inst + 1] - pb;
+    const int tb = plan.tile_begin[pb] + ((int)blockIdx.x - pb), te = plan.tile_end[pb + nb - 1];
+    constexpr int kJ = FcgStage::kJ;
+    Sums<4> t = {{0.0, 0.0, 0.0, 0.0}};
+    FcgStage st;
+    if (tb < te) fcg_stage_load(A, z, r, p, q, have, tb, st);
+    for (int tile = tb; tile < te; tile += nb) {
+        float g[kJ];
+#pragma unroll
+        for (int j = 0; j < kJ; ++j) g[j] = z[st.c[j]];
+        const FcgStage cur = st;
+        if (tile + nb < te) fcg_stage_load(A, z, r, p, q, have, tile + nb, st);
+        double y = (double)cur.dg * (double)cur.z;
+#pragma unroll
+        for (int j = 0; j < kJ; ++j) y += (double)cur.v[j] * (double)g[j];
+        for (int j = kJ + 1; j < cur.w; ++j) {
+            const int64_t slot = cur.off + (int64_t)j * kSliceRows + lane;
+            y += (double)__ldcs(A.val + slot) * (double)z[__ldcs(A.col + slot)];
+        }
+        s[((int64_t)tile * kWarpsPerBlock + warp) * kSliceRows + lane] = (float)y;
+        t.v[0] += (double)cur.z * (double)cur.q;
+        t.v[1] += (double)cur.z * (double)cur.r;
+        t.v[2] += (double)cur.p * (double)cur.r;
+        t.v[3] += (double)cur.z * y;
     }
-    Sums<1> s = {{pr}};
-    Sums<1> tot;
-    if (block_finish<1>(s, partial, c, plan, inst, tot) && threadIdx.x == 0) {
-        c->rho = tot.v[0];
-        if (!isfinite(tot.v[0])) finish_inst(c, -6, n_done);
+    Sums<4> tot;
+    if (block_finish<4>(t, partial, c, plan, inst, tot) && threadIdx.x == 0) {
+        const double beta = have ? tot.v[0] / pq_old : 0.0;
+        const double pr = tot.v[1] - beta * tot.v[2], pq = tot.v[3] - beta * tot.v[0];
+        c->rho = pr;
+        c->beta = beta;
+        c->alpha = 0.0;
+        c->aux[2] = pq;
+        if (!isfinite(pr)) finish_inst(c, -6, n_done);
+        else if (pr == 0.0) finish_inst(c, 0, n_done);
+        else if (!(pq > 0.0) || !isfinite(pq)) finish_inst(c, isfinite(pq) ? -8 : -6, n_done);
+        else c->alpha = pr / pq;
     }
 }
 
-// x += alpha p; r -= alpha q; r.r and the stopping test.  Also keeps (p.q) for the next beta.
 __global__ void __launch_bounds__(kBlockThreads)
-    k_fcg_update(float *__restrict__ x, float *__restrict__ r, const float *__restrict__ p,
-                 const float *__restrict__ q, double *__restrict__ partial, InstCtl *__restrict__ ctl, Plan plan,
-                 int32_t *n_done) {
+    k_fcg_update(float4 *__restrict__ x, float4 *__restrict__ r, float4 *__restrict__ p, float4 *__restrict__ q,
+                 const float4 *__restrict__ z, const float4 *__restrict__ s, double *__restrict__ partial,
+                 InstCtl *__restrict__ ctl, Plan plan, int32_t *n_done) {
     const int inst = plan.inst[blockIdx.x];
     InstCtl *c = ctl + inst;
     if (c->done) return;
-    const double alpha = c->alpha;
+    const double alpha = c->alpha, beta = c->beta;
     double rr = 0.0;
-    for (int tile = plan.tile_begin[blockIdx.x]; tile < plan.tile_end[blockIdx.x]; ++tile) {
-        const int64_t row = (int64_t)tile * kBlockThreads + threadIdx.x;
-        x[row] = (float)((double)x[row] + alpha * (double)p[row]);
-        const float rn = (float)((double)r[row] - alpha * (double)q[row]);
-        r[row] = rn;
-        rr += (double)rn * (double)rn;
+    // beta = 0 starts a new direction sequence: p and q are not used (they may hold a broken one)
+    auto dir = [&](float a, float b) { return beta == 0.0 ? a : (float)((double)a - beta * (double)b); };
+    auto one = [&](float zv, float sv, float &pv, float &qv, float &xv, float &rv) {
+        pv = dir(zv, pv);
+        qv = dir(sv, qv);
+        xv = (float)((double)xv + alpha * (double)pv);
+        rv = (float)((double)rv - alpha * (double)qv);
+        rr += (double)rv * (double)rv;
+    };
+    // four rows a thread and turn: four tiles at a time of the instance's run, the blocks in turn
+    const int pb = plan.inst_blk[inst], nb = plan.inst_blk[inst + 1] - pb;
+    constexpr int64_t kPer = kBlockThreads / 4;
+    const int64_t i0 = plan.tile_begin[pb] * kPer, end = plan.tile_end[pb + nb - 1] * kPer;
+    for (int64_t i = i0 + ((int64_t)blockIdx.x - pb) * kBlockThreads + threadIdx.x; i < end;
+         i += (int64_t)nb * kBlockThreads) {
+        const float4 zv = __ldcs(z + i), sv = __ldcs(s + i);
+        float4 pv = p[i], qv = q[i], xv = x[i], rv = r[i];
+        one(zv.x, sv.x, pv.x, qv.x, xv.x, rv.x);
+        one(zv.y, sv.y, pv.y, qv.y, xv.y, rv.y);
+        one(zv.z, sv.z, pv.z, qv.z, xv.z, rv.z);
+        one(zv.w, sv.w, pv.w, qv.w, xv.w, rv.w);
+        p[i] = pv;
+        q[i] = qv;
+        x[i] = xv;
+        r[i] = rv;
     }
-    Sums<1> s = {{rr}};
+    Sums<1> t = {{rr}};
     Sums<1> tot;
-    if (block_finish<1>(s, partial, c, plan, inst, tot) && threadIdx.x == 0) {
-        c->aux[0] = c->rho / c->alpha;  // p.q of this iteration (alpha = p.r / p.q)
-        c->aux[1] = 1.0;                // (p, q) hold a direction the next one is made conjugate to
+    if (block_finish<1>(t, partial, c, plan, inst, tot) && threadIdx.x == 0) {
+        c->aux[0] = c->aux[2];  // p.q of this iteration
+        c->aux[1] = 1.0;        // (p, q) hold a direction the next one is made conjugate to
         c->rr = tot.v[0];
         c->iter += 1;
         if (!isfinite(tot.v[0])) finish_inst(c, -6, n_done);
@@ -161,17 +235,12 @@ __global__ void __launch_bounds__(kBlockThreads)
 
 // ---- Chebyshev-Jacobi polynomial preconditioner z = P_d(S^) r on [lo, hi] ---------------
 // step 0: d = r / theta, z = d;  step k: d = c1 d + c2 (r - S^ z_prev), z = z_prev + d.
-// The last step also reduces z.q_old for the flexible-CG beta.
 __global__ void __launch_bounds__(kBlockThreads)
     k_cheb_step(SellView<float> A, const float *__restrict__ r, const float *__restrict__ z_prev,
                 float *__restrict__ z_next, float *__restrict__ d, double c1, double c2, int first,
-                const float *__restrict__ q_old, double *__restrict__ partial, InstCtl *__restrict__ ctl, Plan plan,
-                int32_t *n_done) {
-    const int inst = plan.inst[blockIdx.x];
-    InstCtl *c = ctl + inst;
-    if (c->done) return;
+                const InstCtl *__restrict__ ctl, Plan plan) {
+    if (ctl[plan.inst[blockIdx.x]].done) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double zq = 0.0;
     for (int tile = plan.tile_begin[blockIdx.x]; tile < plan.tile_end[blockIdx.x]; ++tile) {
         const int64_t sl = (int64_t)tile * kWarpsPerBlock + warp;
         const int64_t row = sl * kSliceRows + lane;
@@ -181,39 +250,13 @@ __global__ void __launch_bounds__(kBlockThreads)
             d[row] = dn;
             zn = dn;
         } else {
-            const float4 az = aggregate<true>(A, z_prev, nullptr, sl, lane);
-            const double res = (double)r[row] - (double)az.x;
+            const double res = (double)r[row] - (double)sell_row_dot(A, z_prev, sl, lane);
             const float dn = (float)(c1 * (double)d[row] + c2 * res);
             d[row] = dn;
             zn = z_prev[row] + dn;
         }
         z_next[row] = zn;
-        if (q_old) zq += (double)zn * (double)q_old[row];
     }
-    if (partial) {
-        Sums<1> s = {{zq}};
-        Sums<1> tot;
-        if (block_finish<1>(s, partial, c, plan, inst, tot) && threadIdx.x == 0)
-            c->beta = (c->aux[1] != 0.0 && c->aux[0] != 0.0) ? tot.v[0] / c->aux[0] : 0.0;
-    }
-}
-
-// beta = z.q_old / (p.q)_old for flexible CG after a preconditioner that writes z only
-__global__ void __launch_bounds__(kBlockThreads)
-    k_fcg_beta(const float *__restrict__ z, const float *__restrict__ q_old, double *__restrict__ partial,
-               InstCtl *__restrict__ ctl, Plan plan) {
-    const int inst = plan.inst[blockIdx.x];
-    InstCtl *c = ctl + inst;
-    if (c->done) return;
-    double zq = 0.0;
-    for (int tile = plan.tile_begin[blockIdx.x]; tile < plan.tile_end[blockIdx.x]; ++tile) {
-        const int64_t row = (int64_t)tile * kBlockThreads + threadIdx.x;
-        zq += (double)z[row] * (double)q_old[row];
-    }
-    Sums<1> s = {{zq}};
-    Sums<1> tot;
-    if (block_finish<1>(s, partial, c, plan, inst, tot) && threadIdx.x == 0)
-        c->beta = (c->aux[1] != 0.0 && c->aux[0] != 0.0) ? tot.v[0] / c->aux[0] : 0.0;
 }
 
 // Gershgorin bound max_i sum_j |S^_ij| (upper bound of the spectrum of S^)
@@ -268,9 +311,8 @@ inline unsigned blocks_for(int64_t n, int th) { return (unsigned)((n + th - 1) /
 
 }  // namespace
 
-// z = NN(r) on the FP32 inner vectors; with q_old the last layer reduces z.q_old -> beta.
 cudaError_t launch_cheb_apply(const DevSystem &sys, const float *r, float *z0, float *z1, float *d, float *z_final,
-                              const float *q_old, int degree, double lo, double hi, cudaStream_t s) {
+                              int degree, double lo, double hi, cudaStream_t s) {
     if (sys.rows_per_thread != 1) return cudaErrorInvalidValue;  // tiles of 256 rows
     const SellView<float> A = {sys.n_rows, sys.slice_off, sys.col, sys.val32};
     const unsigned g = (unsigned)sys.plan[1].n_blocks;
@@ -288,30 +330,22 @@ cudaError_t launch_cheb_apply(const DevSystem &sys, const float *r, float *z0, f
         }
         const bool last = k == degree - 1;
         float *zn = last ? z_final : ((k % 2 == 0) ? z0 : z1);
-        k_cheb_step<<<g, kBlockThreads, 0, s>>>(A, r, zp, zn, d, c1, c2, k == 0 ? 1 : 0, last ? q_old : nullptr,
-                                                last && q_old ? sys.partial : nullptr, sys.ctl, p, sys.n_done);
+        k_cheb_step<<<g, kBlockThreads, 0, s>>>(A, r, zp, zn, d, c1, c2, k == 0 ? 1 : 0, sys.ctl, p);
         zp = zn;
     }
     return cudaGetLastError();
 }
 
-cudaError_t launch_fcg_beta(const DevSystem &sys, const float *z, const float *q_old, cudaStream_t s) {
+cudaError_t launch_fcg_iteration(const DevSystem &sys, const float *z, cudaStream_t s) {
     if (sys.rows_per_thread != 1) return cudaErrorInvalidValue;  // tiles of 256 rows
-    k_fcg_beta<<<(unsigned)sys.plan[1].n_blocks, kBlockThreads, 0, s>>>(z, q_old, sys.partial, sys.ctl, plan32(sys));
-    return cudaGetLastError();
-}
-
-cudaError_t launch_fcg_direction(const DevSystem &sys, const float *z, cudaStream_t s) {
-    if (sys.rows_per_thread != 1) return cudaErrorInvalidValue;  // tiles of 256 rows
-    k_fcg_direction<<<(unsigned)sys.plan[1].n_blocks, kBlockThreads, 0, s>>>(z, sys.r32, sys.p32, sys.partial, sys.ctl,
-                                                                            plan32(sys), sys.n_done);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_fcg_update(const DevSystem &sys, cudaStream_t s) {
-    if (sys.rows_per_thread != 1) return cudaErrorInvalidValue;  // tiles of 256 rows
-    k_fcg_update<<<(unsigned)sys.plan[1].n_blocks, kBlockThreads, 0, s>>>(sys.x32, sys.r32, sys.p32, sys.q32,
-                                                                         sys.partial, sys.ctl, plan32(sys), sys.n_done);
+    const SellView<float> A = {sys.n_rows, sys.slice_off, sys.col, sys.val32};
+    const unsigned g = (unsigned)sys.plan[1].n_blocks;
+    auto v4 = [](float *v) { return reinterpret_cast<float4 *>(v); };  // rows start on cudaMalloc's boundary
+    k_fcg_spmv<<<g, kBlockThreads, 0, s>>>(A, z, sys.r32, sys.p32, sys.q32, sys.s32, sys.partial, sys.ctl, plan32(sys),
+                                           sys.n_done);
+    k_fcg_update<<<g, kBlockThreads, 0, s>>>(v4(sys.x32), v4(sys.r32), v4(sys.p32), v4(sys.q32),
+                                             reinterpret_cast<const float4 *>(z), v4(sys.s32), sys.partial, sys.ctl,
+                                             plan32(sys), sys.n_done);
     return cudaGetLastError();
 }
 

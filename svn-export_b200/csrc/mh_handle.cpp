@@ -293,7 +293,7 @@ int device_setup(mh_handle *h) {
     s.r = dalloc<double>(h, nr);
     s.p = dalloc<double>(h, nr);
     s.q = dalloc<double>(h, nr);
-    s.w = dalloc<double>(h, nr);
+    s.s32 = dalloc<float>(h, nr);
     s.x32 = dalloc<float>(h, nr);
     s.r32 = dalloc<float>(h, nr);
     s.p32 = dalloc<float>(h, nr);
@@ -304,7 +304,7 @@ int device_setup(mh_handle *h) {
     s.n_done = dalloc<int32_t>(h, 1);
     s.inst_sums = dalloc<double>(h, mh::kSumStride * (size_t)s.n_inst);
     s.sum_ticket = dalloc<uint32_t>(h, s.n_inst);
-    if (!s.val_raw || !s.val64 || !s.val32 || !s.dsq || !s.b || !s.bh || !s.x || !s.r || !s.p || !s.q || !s.w ||
+    if (!s.val_raw || !s.val64 || !s.val32 || !s.dsq || !s.b || !s.bh || !s.x || !s.r || !s.p || !s.q || !s.s32 ||
         !s.x32 || !s.r32 || !s.p32 || !s.q32 || !s.z32 || !s.partial || !s.ctl || !s.n_done || !s.inst_sums ||
         !s.sum_ticket)
         return MH_ERR_NOMEM;
@@ -932,24 +932,19 @@ cudaError_t fcg_iteration(mh_handle *h, Pc kind, int degree, double lo, double h
     cudaError_t e;
     switch (kind) {
         case Pc::Cheb:
-            e = mh::launch_cheb_apply(sys, sys.r32, h->cheb_z0, h->cheb_z1, h->cheb_d, sys.z32, sys.q32, degree, lo, hi,
-                                      s);
+            e = mh::launch_cheb_apply(sys, sys.r32, h->cheb_z0, h->cheb_z1, h->cheb_d, sys.z32, degree, lo, hi, s);
             break;
         default:
             e = h->amg.apply(sys.r32, sys.z32, sys.n_done, sys.n_inst, s, prof);
-            if (e == cudaSuccess) e = mh::launch_fcg_beta(sys, sys.z32, sys.q32, s);
             break;
     }
-    if (e == cudaSuccess) e = mh::launch_fcg_direction(sys, sys.z32, s);
-    if (e == cudaSuccess) e = mh::launch_cg_spmv(sys, 32, s);
-    if (e == cudaSuccess) e = mh::launch_fcg_update(sys, s);
-    return e;
+    return e == cudaSuccess ? mh::launch_fcg_iteration(sys, sys.z32, s) : e;
 }
 
 int fcg_kernels_per_iteration(mh_handle *h, Pc kind, int degree) {
     switch (kind) {
-        case Pc::Cheb: return degree + 3;
-        default: return h->amg.kernels_per_apply() + 4;
+        case Pc::Cheb: return degree + 2;
+        default: return h->amg.kernels_per_apply() + 2;
     }
 }
 

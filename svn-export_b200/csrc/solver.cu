@@ -54,6 +54,18 @@ struct Plan {
     const int32_t *inst, *tile_begin, *tile_end, *inst_blk;
 };
 
+// The tiles of a block: its instance's blocks take the instance's tiles in turn, so that all of them
+// work in one moving window (gathers that one block brings into L2 serve the others, and the
+// streams stay on few DRAM pages).  A run of neighbouring tiles per block was 1.24x (FP64) and 1.32x
+// (FP32) slower per CG iteration at 10.9M rows, 1.04x and 1.10x at 3.2M.
+struct Tiles {
+    int begin, end, step;
+};
+__device__ __forceinline__ Tiles tiles_of(const Plan &plan, int inst) {
+    const int pb = plan.inst_blk[inst], nb = plan.inst_blk[inst + 1] - pb;
+    return {plan.tile_begin[pb] + ((int)blockIdx.x - pb), plan.tile_end[pb + nb - 1], nb};
+}
+
 // Publishes this block's partial sums and returns true in every thread of the block that
 // arrived last for its instance; that block then holds the instance totals in `tot`
 // (thread 0 only).
@@ -203,18 +215,19 @@ __global__ void __launch_bounds__(kBlockThreads, sizeof(T) == 4 ? 4 : 3)
     InstCtl *c = ctl + inst;
     if (c->done) return;
     Sums<3> s = {{0.0, 0.0, 0.0}};
-    const int tb = plan.tile_begin[blockIdx.x], te = plan.tile_end[blockIdx.x];
+    const Tiles T_ = tiles_of(plan, inst);
+    const int tb = T_.begin, te = T_.end, nb = T_.step;
     if (R == 1) {
         constexpr int kJ = SpmvStage<T>::kJ;
         const int lane = threadIdx.x & 31;
         SpmvStage<T> st;
         if (tb < te) spmv_stage_load<T>(A, p, r, tb, st);
-        for (int tile = tb; tile < te; ++tile) {
+        for (int tile = tb; tile < te; tile += nb) {
             T g[kJ];
 #pragma unroll
             for (int j = 0; j < kJ; ++j) g[j] = p[st.c[j]];
             const SpmvStage<T> cur = st;
-            if (tile + 1 < te) spmv_stage_load<T>(A, p, r, tile + 1, st);
+            if (tile + nb < te) spmv_stage_load<T>(A, p, r, tile + nb, st);
             double y = 0.0;
 #pragma unroll
             for (int j = 0; j < kJ; ++j) y += (double)cur.v[j] * (double)g[j];
@@ -228,7 +241,7 @@ __global__ void __launch_bounds__(kBlockThreads, sizeof(T) == 4 ? 4 : 3)
             s.v[2] += y * y;
         }
     } else {
-        for (int tile = tb; tile < te; ++tile) {
+        for (int tile = tb; tile < te; tile += nb) {
             double y[R];
             sell_rows<T, T, R>(A, p, tile, y);
 #pragma unroll
@@ -275,7 +288,8 @@ __global__ void __launch_bounds__(kBlockThreads) k_cg_update(T *__restrict__ x, 
     const double alpha = c->alpha, beta = c->beta;
     Sums<1> s = {{0.0}};
     // software-pipelined: the four loads of tile t+1 are issued before tile t is computed
-    const int tb = plan.tile_begin[blockIdx.x], te = plan.tile_end[blockIdx.x];
+    const Tiles T_ = tiles_of(plan, inst);
+    const int tb = T_.begin, te = T_.end, nb = T_.step;
     T pv[R], xv[R], rv[R], qv[R];
     auto load = [&](int tile) {
 #pragma unroll
@@ -288,7 +302,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_cg_update(T *__restrict__ x, 
         }
     };
     if (tb < te) load(tb);
-    for (int tile = tb; tile < te; ++tile) {
+    for (int tile = tb; tile < te; tile += nb) {
         T cp[R], cx[R], cr[R], cq[R];
 #pragma unroll
         for (int k = 0; k < R; ++k) {
@@ -297,7 +311,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_cg_update(T *__restrict__ x, 
             cr[k] = rv[k];
             cq[k] = qv[k];
         }
-        if (tile + 1 < te) load(tile + 1);
+        if (tile + nb < te) load(tile + nb);
 #pragma unroll
         for (int k = 0; k < R; ++k) {
             const int64_t row = flat_row<R>(tile, k);
@@ -336,7 +350,8 @@ __global__ void __launch_bounds__(kBlockThreads) k_cg_init(SellView<double> A, c
     InstCtl *c = ctl + inst;
     const bool active = !use_active || inst_sums[kSumStride * inst + kSumActive] != 0.0;
     Sums<2> s = {{0.0, 0.0}};
-    for (int tile = plan.tile_begin[blockIdx.x]; tile < plan.tile_end[blockIdx.x]; ++tile) {
+    const Tiles T_ = tiles_of(plan, inst);
+    for (int tile = T_.begin; tile < T_.end; tile += T_.step) {
         double y[R];
         sell_rows<double, double, R>(A, x, tile, y);
 #pragma unroll
@@ -382,7 +397,8 @@ __global__ void __launch_bounds__(kBlockThreads) k_residual64(SellView<double> A
     const int inst = plan.inst[blockIdx.x];
     InstCtl *c = ctl + inst;
     Sums<4> s = {{0.0, 0.0, 0.0, 0.0}};
-    for (int tile = plan.tile_begin[blockIdx.x]; tile < plan.tile_end[blockIdx.x]; ++tile) {
+    const Tiles T_ = tiles_of(plan, inst);
+    for (int tile = T_.begin; tile < T_.end; tile += T_.step) {
         double y[R];
         sell_rows<double, double, R>(A, x, tile, y);
 #pragma unroll
