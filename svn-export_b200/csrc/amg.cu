@@ -772,68 +772,174 @@ __global__ void k_slice_width(int64_t n_slices, int64_t nc, const int32_t *rowle
 
 
 // ---- dense coarsest level ----------------------------------------------------------------
-// In-place Gauss-Jordan inversion in shared memory (FP64, no pivoting: the matrix is SPD), one
-// block of 1024 threads, n <= kDenseMax.  The first n rows of the SELL matrix are gathered
-// into shared memory, inverted, and written out as FP32.  flag = 1 on a non-positive or
-// non-finite pivot.
-constexpr int kDenseMax = 160;  // n^2 doubles + n factors fit in 227 KB of shared memory
+// The coarsest matrix (n <= kDenseMax rows) is inverted in FP64 by block Gauss-Jordan without
+// pivoting (it is SPD), blocks of 32, one launch per block step over 64 x 64 tiles of the padded
+// matrix, reading one copy and writing the other.  In step k, with D = A_kk^-1 and P = D A_k. (P_k
+// = D in block column k): row block k becomes P, the other rows A_i. - A_ik P (0 for A_ik in block
+// column k).  Every block inverts A_kk itself (32 pivots) and forms P for its columns, so a step
+// needs nothing from another block of the same launch.  flag = 1 on a non-positive or non-finite
+// pivot.  A step costs 6-12 us, most of it the 32 pivots.
+// Measured (B200): the inverse of 130 rows 360 us by one block with the matrix in shared memory;
+// here 0.05 ms for 130 rows, 0.13 for 477, 0.5 for 1120.
+// kDenseMax: the limit was 160, what one SM's shared memory held.  An exact solve this high up
+// replaces one to three levels of seven latency-bound kernels each, in every cycle and in the setup,
+// and converges faster: n = 21 (1120 rows) 57 iterations of 145 us -> 40 of 113, n = 64 (847 rows)
+// 104 of 591 -> 73 of 545, 24 uneven systems (437 rows) 43.7 -> 34.5 ms.  At 1280 rows the inverse
+// is 6.5 MB, 3.5 us a pass from L2; at 2048 its setup (n^3) would cost more than the levels it saves.
+constexpr int kDenseMax = 1280;
+constexpr int kCoarseMin = 160;  // pairing passes go on down to this many rows
+constexpr int kGjB = 32, kGjTile = 64;
 
-__global__ void __launch_bounds__(1024) k_dense_inverse(MatView A, int n, float *inv, int32_t *flag) {
-    extern __shared__ double sm[];
-    double *M = sm, *fac = sm + n * n;
-    __shared__ double pinv;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // launched with 1024 threads
-    for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) M[idx] = 0.0;
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        int64_t base;
-        int w, ln;
-        row_of(A, i, base, w, ln);
-        for (int j = 0; j < w; ++j) {
-            const int64_t slot = base + (int64_t)j * kS + ln;
-            const int32_t c = A.col[slot];
-            if (c < n) M[i * n + c] += (double)A.val[slot];
+// the n x n part of A in the np x np matrix M (zeroed before; identity in the padding)
+__global__ void k_dense_scatter(MatView A, int n, int np, double *__restrict__ M) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= np) return;
+    if (i >= n) {
+        M[(size_t)i * np + i] = 1.0;
+        return;
+    }
+    int64_t base;
+    int w, ln;
+    row_of(A, i, base, w, ln);
+    for (int j = 0; j < w; ++j) {
+        const int64_t slot = base + (int64_t)j * kS + ln;
+        const int32_t c = A.col[slot];
+        if (c < n) M[(size_t)i * np + c] += (double)A.val[slot];
+    }
+}
+
+__global__ void __launch_bounds__(256) k_gj_step(const double *__restrict__ src, double *__restrict__ dst, int np,
+                                                 int k, int32_t *flag) {
+    __shared__ double D[kGjB][kGjB + 1], rowb[2][kGjB], colb[2][kGjB];
+    __shared__ double Ai[kGjTile][kGjB + 1], P[kGjB][kGjTile];
+    const int t = threadIdx.x, kb = k * kGjB;
+    const int i0 = blockIdx.y * kGjTile, j0 = blockIdx.x * kGjTile;
+    auto at = [&](int r, int c) { return r < np && c < np ? src[(size_t)r * np + c] : 0.0; };
+    // A_ik and A_kj are on their way while A_kk is inverted
+    for (int q = t; q < kGjTile * kGjB; q += 256) {
+        Ai[q / kGjB][q % kGjB] = at(i0 + q / kGjB, kb + q % kGjB);
+        P[q / kGjTile][q % kGjTile] = at(kb + q / kGjTile, j0 + q % kGjTile);
+    }
+    // D: thread t holds four entries of row r
+    const int r = t >> 3, c4 = (t & 7) * 4;
+    double m[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) m[q] = src[(size_t)(kb + r) * np + kb + c4 + q];
+    bool bad = false;
+#pragma unroll 1
+    for (int p = 0; p < kGjB; ++p) {
+        double *rb = rowb[p & 1], *cb = colb[p & 1];
+        if (r == p)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) rb[c4 + q] = m[q];
+        if ((p & ~3) == c4)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (c4 + q == p) cb[r] = m[q];
+        __syncthreads();
+        const double piv = rb[p];
+        const bool ok = piv > 0.0 && isfinite(piv);
+        bad |= !ok;
+        const double pinv = ok ? 1.0 / piv : 0.0, f = cb[r];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const bool jp = c4 + q == p;
+            const double a = (jp ? 1.0 : rb[c4 + q]) * pinv;
+            m[q] = r == p ? a : (jp ? 0.0 : m[q]) - f * a;
         }
     }
+    if (bad && t == 0) *flag = 1;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) D[r][c4 + q] = m[q];
     __syncthreads();
-    for (int k = 0; k < n; ++k) {
-        if (threadIdx.x == 0) {
-            const double p = M[k * n + k];
-            const bool ok = p > 0.0 && isfinite(p);
-            if (!ok) *flag = 1;
-            pinv = ok ? 1.0 / p : 0.0;
-        }
-        for (int i = threadIdx.x; i < n; i += blockDim.x) fac[i] = M[i * n + k];
-        __syncthreads();
-        // row k: a_kj / p, with a_kk := 1 / p
-        for (int j = threadIdx.x; j < n; j += blockDim.x) M[k * n + j] = (j == k ? 1.0 : M[k * n + j]) * pinv;
-        __syncthreads();
-        // rows i != k: a_ij -= f_i a_kj, with a_ik := -f_i / p (32 x 32 threads: lanes take
-        // consecutive columns, warps rows; a_kj is loaded once per column, f_i is a broadcast)
-        for (int j = tx; j < n; j += 32) {
-            const double akj = M[k * n + j];
-            const bool jk = j == k;
-            for (int i = ty; i < n; i += 32) {
-                if (i == k) continue;
-                const double base = jk ? 0.0 : M[i * n + j];
-                M[i * n + j] = base - fac[i] * akj;
+    // P = D A_kj (D itself in block column k): thread t takes column j and 8 of the 32 rows
+    {
+        const int j = t & 63, rg = (t >> 6) * 8;
+        double acc[8];
+        const int cb = j0 + j - kb;
+        if (cb >= 0 && cb < kGjB) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) acc[q] = D[rg + q][cb];
+        } else {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) acc[q] = 0.0;
+            for (int l = 0; l < kGjB; ++l) {
+                const double a = P[l][j];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) acc[q] += D[rg + q][l] * a;
             }
         }
         __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 8; ++q) P[rg + q][j] = acc[q];
     }
-    for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) inv[idx] = (float)M[idx];
+    __syncthreads();
+    // the tile: thread t takes rows ty + 16 a and columns tx + 16 b
+    const int tx = t & 15, ty = t >> 4;
+    double acc[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
+#pragma unroll 4
+    for (int l = 0; l < kGjB; ++l) {
+        double x[4], y[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            x[a] = Ai[ty + 16 * a][l];
+            y[a] = P[l][tx + 16 * a];
+        }
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) acc[a][b] += x[a] * y[b];
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const int i = i0 + ty + 16 * a;
+        if (i >= np) continue;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int j = j0 + tx + 16 * b;
+            if (j >= np) continue;
+            const bool in_r = i >= kb && i < kb + kGjB, in_c = j >= kb && j < kb + kGjB;
+            dst[(size_t)i * np + j] =
+                in_r ? P[i - kb][j - j0] : (in_c ? 0.0 : src[(size_t)i * np + j]) - acc[a][b];
+        }
+    }
 }
 
-// x[i] = sum_j inv[i][j] b[j] for i < n (one warp per row); rows n..n_pad-1 get 0
-__global__ void k_dense_gemv(Gate gate, const float *__restrict__ inv, int64_t n, int64_t n_pad, const float *__restrict__ b,
-                             float *__restrict__ x) {
+// the inverse in FP32, rows of ld entries (a multiple of 4; zeros past n)
+__global__ void k_dense_store(int n, int np, int ld, const double *__restrict__ M, float *__restrict__ inv) {
+    const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= (int64_t)n * ld) return;
+    const int i = (int)(q / ld), j = (int)(q % ld);
+    inv[q] = j < n ? (float)M[(size_t)i * np + j] : 0.f;
+}
+
+__host__ __device__ inline int64_t dense_ld(int64_t n) { return (n + 3) / 4 * 4; }
+
+// x[i] = sum_j inv[i][j] b[j] for i < n (one warp per row, four entries to a load); rows
+// n..n_pad-1 get 0.  b has n_pad >= ld entries.
+__global__ void __launch_bounds__(256) k_dense_gemv(Gate gate, const float *__restrict__ inv, int64_t n, int64_t ld,
+                                                    int64_t n_pad, const float *__restrict__ b, float *__restrict__ x) {
     if (closed(gate)) return;
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= n_pad) return;
     float s = 0.f;
-    if (i < n)
-        for (int64_t j = lane; j < n; j += 32) s += inv[i * n + j] * b[j];
+    if (i < n) {
+        const float4 *row = reinterpret_cast<const float4 *>(inv + i * ld);
+        const float4 *b4 = reinterpret_cast<const float4 *>(b);
+#pragma unroll 4
+        for (int64_t j = lane; j < ld / 4; j += 32) {
+            const float4 a = row[j], v = b4[j];
+            s += a.x * v.x;
+            s += a.y * v.y;
+            s += a.z * v.z;
+            s += a.w * v.w;
+        }
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
     if (lane == 0) x[i] = s;
@@ -1819,12 +1925,19 @@ __global__ void __launch_bounds__(kTailThreads, 1)
                 }
                 break;
             case kTailDense: {
-                const int64_t n = p.dense_n, n_pad = L.A.n;
+                const int64_t n = p.dense_n, n_pad = L.A.n, ld = dense_ld(n);
                 const int lane = threadIdx.x & 31;
                 for (int64_t i = tid >> 5; i < n_pad; i += n_thr >> 5) {
                     float s = 0.f;
                     if (i < n)
-                        for (int64_t j = lane; j < n; j += 32) s += __ldg(p.dense + i * n + j) * __ldcg(p.b + j);
+                        for (int64_t j = lane; j < ld / 4; j += 32) {
+                            const float4 a = __ldg(reinterpret_cast<const float4 *>(p.dense + i * ld) + j);
+                            const float4 v = __ldcg(reinterpret_cast<const float4 *>(p.b) + j);
+                            s += a.x * v.x;
+                            s += a.y * v.y;
+                            s += a.z * v.z;
+                            s += a.w * v.w;
+                        }
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
                     if (lane == 0) p.x_out[i] = s;
@@ -1940,6 +2053,7 @@ void Amg::release() {
     w0_used_ = nullptr;
     isd_.release();
     dense_inv_.release();
+    for (auto &w : dense_work_) w.release();
     bound_.release();
     tail_prog_.release();
     tail_levels_.release();
@@ -2195,21 +2309,25 @@ cudaError_t Amg::galerkin(const AmgMatrix &A, const int32_t *agg, int64_t nc, co
     return cudaSuccess;
 }
 
-cudaError_t Amg::dense_coarse(const AmgMatrix &A, cudaStream_t s) {
-    const int64_t n = dense_n_;
-    AMG_CK(dense_inv_.ensure((size_t)n * n));
+// ok: the matrix was positive definite and its inverse is in place
+cudaError_t Amg::dense_coarse(const AmgMatrix &A, bool &ok, cudaStream_t s) {
+    const int n = (int)dense_n_, np = (int)round_up(n, kGjB);
+    const int64_t ld = dense_ld(n);
+    AMG_CK(dense_inv_.ensure((size_t)n * ld));
+    for (auto &w : dense_work_) AMG_CK(w.ensure((size_t)np * np));
     AMG_CK(flag_.ensure(1));
     AMG_CK(cudaMemsetAsync(flag_.p, 0, sizeof(int32_t), s));
-    const size_t smem = (size_t)(n * n + n) * sizeof(double);
-    AMG_CK(cudaFuncSetAttribute(k_dense_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_dense_inverse<<<1, 1024, smem, s>>>(view(A), (int)n, dense_inv_.p, flag_.p);
+    AMG_CK(cudaMemsetAsync(dense_work_[0].p, 0, (size_t)np * np * sizeof(double), s));
+    k_dense_scatter<<<nblk(np, 128), 128, 0, s>>>(view(A), n, np, dense_work_[0].p);
+    const unsigned tiles = nblk(np, kGjTile);
+    int from = 0;
+    for (int k = 0; k < np / kGjB; ++k, from ^= 1)
+        k_gj_step<<<dim3(tiles, tiles), 256, 0, s>>>(dense_work_[from].p, dense_work_[from ^ 1].p, np, k, flag_.p);
+    k_dense_store<<<nblk(n * ld, 256), 256, 0, s>>>(n, np, (int)ld, dense_work_[from].p, dense_inv_.p);
     AMG_CK(cudaGetLastError());
     AMG_CK(cudaMemcpyAsync(h_flag_, flag_.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
     AMG_CK(cudaStreamSynchronize(s));
-    if (*h_flag_) {
-        err = "coarsest matrix is not positive definite";
-        return cudaErrorInvalidValue;
-    }
+    ok = *h_flag_ == 0;
     return cudaSuccess;
 }
 
@@ -2272,7 +2390,9 @@ cudaError_t Amg::setup(const DevSystem &sys, const AmgOptions &o, cudaStream_t s
         L.nc = 0;
         n_levels_ = l + 1;
         const int64_t n_real = l == 0 ? sys.n_rows : (l > 0 ? lv_[l - 1].nc : 0);
-        if (n_real <= opt_.coarse_max || l + 1 >= opt_.max_levels) break;
+        // (a fine level of more than kCoarseMin rows always gets a coarser one)
+        if (n_real <= (l == 0 ? std::min(opt_.coarse_max, kCoarseMin) : opt_.coarse_max) || l + 1 >= opt_.max_levels)
+            break;
         // pairing passes: pass 1 on A_l, pass p on the Galerkin matrix of pass p-1's pairs;
         // the aggregation of the level is their composition
         const int passes = l == 0 ? opt_.pair_passes : opt_.pair_passes_coarse;
@@ -2283,7 +2403,7 @@ cudaError_t Amg::setup(const DevSystem &sys, const AmgOptions &o, cudaStream_t s
             cudaSuccess)
             return e;
         const int32_t *cagg = L.agg.p, *cms = L.mem_start.p, *cmr = L.mem_rows.p;
-        for (int p = 1; p < passes && nc > opt_.coarse_max; ++p) {
+        for (int p = 1; p < passes && nc > std::min(opt_.coarse_max, kCoarseMin); ++p) {
             AmgMatrix M;
             const int slot = p & 1;
             if ((e = galerkin(cur, cagg, nc, cms, cmr, mid_off_[slot], mid_col_[slot], mid_val_[slot], mid_rlen_[slot],
@@ -2389,8 +2509,18 @@ cudaError_t Amg::setup(const DevSystem &sys, const AmgOptions &o, cudaStream_t s
     }
     const AmgLevel &Lc = lv_[n_levels_ - 1];
     dense_n_ = n_levels_ == 1 ? Lc.A.n : lv_[n_levels_ - 2].nc;
-    if (dense_n_ > kDenseMax) {  // too large for the shared-memory inverse: smooth it instead
-        dense_n_ = 0;
+    if (!dense_planned()) dense_n_ = 0;
+    if (dense_n_ > 0) {
+        bool ok = false;
+        if ((e = dense_coarse(Lc.A, ok, s)) != cudaSuccess) return e;
+        if (!ok && dense_n_ <= kCoarseMin) {
+            err = "coarsest matrix is not positive definite";
+            return cudaErrorInvalidValue;
+        }
+        // (a larger matrix can lose definiteness to its FP32 rounding: smoothed instead)
+        if (!ok) dense_n_ = 0;
+    }
+    if (dense_n_ == 0) {  // too large for the dense inverse: a polynomial on the level instead
         AmgLevel &Lm = lv_[n_levels_ - 1];
         AMG_CK(Lm.agg.ensure(Lm.A.n));
         k_mark_isolated<<<nblk(Lm.A.n, 256), 256, 0, s>>>(view(Lm.A), Lm.agg.p);
@@ -2424,8 +2554,15 @@ cudaError_t Amg::setup(const DevSystem &sys, const AmgOptions &o, cudaStream_t s
     AMG_CK(alpha_.ensure(n_levels_ + 1));
     AMG_CK(tickets_.ensure(n_levels_ + 1));
     AMG_CK(cudaMemsetAsync(tickets_.p, 0, (n_levels_ + 1) * sizeof(unsigned int), s));
-    if (dense_n_ > 0) AMG_CK(dense_coarse(Lc.A, s));
     return build_tail(s);
+}
+
+// whether the coarsest level gets a dense inverse: small enough, and never the fine level of a
+// system without coarser ones unless that is tiny
+bool Amg::dense_planned() const {
+    const int64_t n = n_levels_ == 1 ? lv_[0].A.n : lv_[n_levels_ - 2].nc;
+    const int64_t most = std::min(kDenseMax, std::max(opt_.coarse_max, kCoarseMin));
+    return n <= (n_levels_ == 1 ? kCoarseMin : most);
 }
 
 cudaError_t Amg::power_estimates(cudaStream_t s, int only_level) {
@@ -2438,10 +2575,11 @@ cudaError_t Amg::power_estimates(cudaStream_t s, int only_level) {
     AMG_CK(pw_sums_.ensure(2 * (size_t)std::max(n_levels_, 1)));
     if (only_level < 0)
         AMG_CK(cudaMemsetAsync(pw_sums_.p, 0, 2 * (size_t)std::max(n_levels_, 1) * sizeof(double), s));
-    // the coarsest level is solved, not smoothed (unless coarsening stalled: it then gets a
-    // Chebyshev polynomial of its own and an estimate too)
+    // the coarsest level is solved, not smoothed (unless coarsening stalled above the dense limit:
+    // it then gets a Chebyshev polynomial of its own and an estimate too)
     for (int l = 0; l < n_levels_; ++l) {
         if (only_level >= 0 && l != only_level) continue;
+        if (l > 0 && l == n_levels_ - 1 && dense_planned()) continue;
         AmgLevel &L = lv_[l];
         const int64_t n = L.A.n;
         if (n <= 0) continue;
@@ -2934,7 +3072,8 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
         const float *b = nl == 1 ? r : Lc.b.p;
         if (dense_n_ > 0) {
             float *x = nl == 1 ? z : Lc.xa.p;
-            k_dense_gemv<<<nblk(Lc.A.n * 32, 256), 256, 0, s>>>(gate_, dense_inv_.p, dense_n_, Lc.A.n, b, x);
+            k_dense_gemv<<<nblk(Lc.A.n * 32, 256), 256, 0, s>>>(gate_, dense_inv_.p, dense_n_, dense_ld(dense_n_), Lc.A.n,
+                                                                 b, x);
             xout[nl - 1] = x;
         } else {
             const unsigned g = nblk(Lc.A.n, 256), gs = row_blocks(Lc);

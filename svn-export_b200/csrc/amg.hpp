@@ -11,7 +11,7 @@
 //   carry the weights sqrt(diag S): P_0 = W P, and A_1 = P^T S P in the unscaled space.
 //   Coarse matrices are stored as SELL-32 like the fine one; their rows are built by one warp each (gather,
 //   bitonic sort by column, deterministic segmented sum).  The coarsest level (<= coarse_max
-//   rows) is inverted densely in FP64 (in-place Gauss-Jordan in shared memory, one block); if
+//   rows) is inverted densely in FP64 (block Gauss-Jordan); if
 //   coarsening stalls above that size, the coarsest level gets a degree-12 Chebyshev polynomial.
 // Apply (one V-cycle, FP32): Chebyshev smoothing of degree d on [hi/ratio, hi] of D^-1 A
 // before and after the coarse correction (symmetric, so the cycle is an SPD operator).
@@ -29,7 +29,7 @@ namespace mh {
 
 struct AmgOptions {
     int max_levels = 20;
-    int coarse_max = 160;   // dense coarsest solve at or below this many rows (<= 160)
+    int coarse_max = 1280;  // dense coarsest solve at or below this many rows (<= 1280)
     int pair_rounds = 4;    // handshake rounds per pairing pass
     int pair_passes = 2;    // pairing passes from the fine level (2: aggregates of up to 4 rows)
     int pair_passes_coarse = 3;  // ... from the coarser levels (aggregates of up to 8)
@@ -49,7 +49,7 @@ struct AmgOptions {
     float power_safety = 1.1f;  // smoothing interval top = min(Gershgorin, safety * estimate)
     int coarse_degree = 12;     // Chebyshev degree of a smoothed (not inverted) coarsest level
     float coarse_ratio = 50.f;  // ... on [hi / coarse_ratio, hi]
-    int stall_rows = 32768; // after two coarsenings in a row that kept more than half of the rows, a
+    int stall_rows = 16384; // after two coarsenings in a row that kept more than half of the rows, a
                             // next level of at most this many rows is the coarsest (0: off)
     int fine_tma = 0;       // 1: the fine level's cycle kernels stream the matrix through shared
                             // memory with TMA bulk copies (with half_fine; amg.cu k_fine_tma)
@@ -161,7 +161,8 @@ private:
                          DBuf<int32_t> &c_rlen, DBuf<int32_t> &c_long, AmgMatrix &C, cudaStream_t s,
                          const float *wt);
     cudaError_t level_stats(AmgLevel &L, unsigned int *bound, cudaStream_t s);
-    cudaError_t dense_coarse(const AmgMatrix &A, cudaStream_t s);
+    cudaError_t dense_coarse(const AmgMatrix &A, bool &ok, cudaStream_t s);
+    bool dense_planned() const;
     // lambda_max estimates of D^-1 A on every level but the coarsest (power iteration from a
     // fixed pseudo-random start; deterministic sums), as |v_k|^2 and |v_{k-1}|^2 per level
     cudaError_t power_estimates(cudaStream_t s, int only_level = -1);
@@ -199,7 +200,8 @@ private:
     std::vector<int64_t> dots_long_off_;
     int last_long_launches_ = 0;
     DBuf<float> isd_;
-    DBuf<float> dense_inv_;
+    DBuf<float> dense_inv_;         // inverse of the coarsest matrix, and the two copies it is made in
+    DBuf<double> dense_work_[2];
     DBuf<int32_t> flag_;
     DBuf<unsigned int> bound_;
     DBuf<double> dots_, alpha_;     // coarse-correction scaling: partials, factor per level

@@ -1080,7 +1080,7 @@ mh::AmgOptions amg_options() {
     env_i("MH_AMG_PRE", o.pre_degree, 0, 8);
     env_i("MH_AMG_PASSES", o.pair_passes, 1, 4);
     env_i("MH_AMG_CPASSES", o.pair_passes_coarse, 1, 4);
-    env_i("MH_AMG_COARSE", o.coarse_max, 16, 160);
+    env_i("MH_AMG_COARSE", o.coarse_max, 16, 1280);
     env_i("MH_AMG_ROUNDS", o.pair_rounds, 1, 16);
     env_i("MH_AMG_KCYCLE", o.kcycle, 0, 1);
     env_i("MH_AMG_KLEVELS", o.kcycle_levels, 0, 64);
