@@ -132,7 +132,7 @@ typedef struct mh_solve_opts {
     int32_t inner_max_it;   /* FP32 iterations between two replacements at most (2000;
                                after the learned method fell back, at least 200)     */
     int32_t iters_per_graph;/* Krylov iterations per captured CUDA graph launch; 0:
-                               16, or 4 for the multigrid methods (long iterations)  */
+                               16, or 2 for the multigrid methods (long iterations)  */
     int32_t profile_kernels;/* 1: time every Krylov kernel with CUDA events in-graph */
     int32_t host_loop;      /* 0: each Krylov run is one graph launch whose iterations
                                repeat on the device (a conditional loop that ends when

@@ -62,7 +62,7 @@ MatView view(const AmgMatrix &A) { return {A.n, A.slice_off, A.col, A.val, A.rle
 
 // Rows longer than this (hub aggregates: a fracture intersection or a channel that couples to
 // every aggregate along it) are skipped by the thread-per-row kernels and handled by a block
-// each (k_long_rows), so that one row does not serialise its warp.
+// each (long_row), so that one row does not serialise its warp.
 constexpr int kLongRow = 96;
 __device__ __forceinline__ bool is_long(const MatView &A, int64_t i) { return A.rlen && A.rlen[i] > kLongRow; }
 
@@ -974,33 +974,16 @@ __device__ __forceinline__ float fine_dot(const MatView &A, int64_t base, int w,
     return y;
 }
 
-__device__ __forceinline__ float row_dot(const MatView &A, int64_t i, const float *__restrict__ x) {
-    int64_t base;
-    int w, ln;
-    row_of(A, i, base, w, ln);
-    if (A.rlen) {
-        float y = 0.f;
-        for (int j = 0; j < w; ++j) {
-            const int64_t slot = base + (int64_t)j * kS + ln;
-            y += __ldg(A.val + slot) * x[__ldg(A.col + slot)];
-        }
-        return y;
-    }
-    return fine_dot(A, base, w, ln, x);
-}
-
 // Coarse rows are long (tens of entries), so one thread walking a row issues a long chain of
 // dependent loads and the small coarse levels run at load latency.  The row kernels therefore
 // take G warps per 32-row slice (G = AmgLevel::g, chosen from the level's mean slice width):
 // warp g of a slice's group takes the slots g, g + G, g + 2G, ... of its 32 rows, eight loaded
 // together, and the G partial sums meet in shared memory in warp order (deterministic).  Blocks
-// hold 8 warps, i.e. 8 / G slices.  G = 1 is one thread per row (row_dot).
+// hold 8 warps, i.e. 8 / G slices.  G = 1 is one thread per row.
 template <int G>
-__device__ __forceinline__ float split_part(const MatView &A, int64_t i, int g, const float *__restrict__ x) {
-    if (G == 1) return row_dot(A, i, x);
-    int64_t base;
-    int w, ln;
-    row_of(A, i, base, w, ln);
+__device__ __forceinline__ float split_part(const MatView &A, int64_t base, int w, int ln, int g,
+                                            const float *__restrict__ x) {
+    if (G == 1 && !A.rlen) return fine_dot(A, base, w, ln, x);
     constexpr int kB = 8;
     float y = 0.f;
     for (int j0 = g; j0 < w; j0 += kB * G) {
@@ -1017,7 +1000,7 @@ __device__ __forceinline__ float split_part(const MatView &A, int64_t i, int g, 
 #pragma unroll
         for (int k = 0; k < kB; ++k) gx[k] = j0 + k * G < w ? x[c[k]] : 0.f;
 #pragma unroll
-        for (int k = 0; k < kB; ++k) y += v[k] * gx[k];
+        for (int k = 0; k < kB; ++k) y = __fmaf_rn(v[k], gx[k], y);
     }
     return y;
 }
@@ -1041,7 +1024,7 @@ template <int G> __device__ __forceinline__ float split_sum(float y) {
 }
 
 // first Chebyshev step from x = 0: d = c2 D^-1 b, x = d
-// (invd null: unit diagonal, the Jacobi-scaled fine level)
+// (invd null: unit diagonal, the Jacobi-scaled fine level; d null: not kept, it is x)
 __global__ void k_sm_first(Gate gate, int64_t n, const float *__restrict__ b, const float *__restrict__ invd, float c2,
                            float *__restrict__ x, float *__restrict__ d, const int32_t *__restrict__ agg) {
     if (closed(gate)) return;
@@ -1049,17 +1032,17 @@ __global__ void k_sm_first(Gate gate, int64_t n, const float *__restrict__ b, co
     if (i >= n) return;
     const float di = invd ? invd[i] : 1.f;
     if (agg && agg[i] < 0) {  // a row outside the hierarchy: exact
-        d[i] = 0.f;
+        if (d) d[i] = 0.f;
         x[i] = di * b[i];
         return;
     }
     const float v = c2 * di * b[i];
-    d[i] = v;
+    if (d) d[i] = v;
     x[i] = v;
 }
 
 // restriction fused with the first smoothing step of the coarse level:
-// b_c[I] = sum over the rows of I of w r, then x = d = c2 D_c^-1 b_c
+// b_c[I] = sum over the rows of I of w r, then x = d = c2 D_c^-1 b_c (d null: not kept)
 __global__ void k_restrict_first(Gate gate, int64_t nc, int64_t nc_pad, const int32_t *__restrict__ ms,
                                  const int32_t *__restrict__ mr, const float *__restrict__ r,
                                  const float *__restrict__ wt, const float *__restrict__ invd_c, float c2,
@@ -1074,35 +1057,8 @@ __global__ void k_restrict_first(Gate gate, int64_t nc, int64_t nc_pad, const in
     bc[I] = s;
     const bool exact = agg_c[I] < 0;
     const float v = (exact ? 1.f : c2) * invd_c[I] * s;
-    d[I] = exact ? 0.f : v;
+    if (d) d[I] = exact ? 0.f : v;
     x[I] = v;
-}
-
-// Chebyshev step: d = c1 d + c2 D^-1 (b - A x_in), x_out = x_in + d (c1 = 0: d is not read)
-template <int G>
-__global__ void __launch_bounds__(256) k_sm_step(Gate gate, MatView A, const float *__restrict__ b,
-                                                 const float *__restrict__ invd, const float *__restrict__ x_in,
-                                                 float *__restrict__ x_out, float *__restrict__ d, float c1, float c2,
-                                                 const int32_t *__restrict__ agg) {
-    if (closed(gate)) return;
-    int64_t i;
-    int g;
-    split_row<G>(i, g);
-    const bool outside = i < A.n && agg && agg[i] < 0;
-    const bool live = i < A.n && !outside && !is_long(A, i);  // long rows: k_long_rows
-    const float y = split_sum<G>(live ? split_part<G>(A, i, g, x_in) : 0.f);
-    if (g != 0 || i >= A.n) return;
-    const float di = invd ? invd[i] : 1.f;
-    if (outside) {  // a row outside the hierarchy: exact
-        d[i] = 0.f;
-        x_out[i] = di * b[i];
-        return;
-    }
-    if (!live) return;
-    const float r = b[i] - y;
-    const float dn = (c1 != 0.f ? c1 * d[i] : 0.f) + c2 * di * r;
-    d[i] = dn;
-    x_out[i] = x_in[i] + dn;
 }
 
 // The fine level's first two Chebyshev steps from x = 0 in one pass (unit diagonal), FP32 values
@@ -1120,7 +1076,10 @@ __global__ void k_sm_first_step(Gate gate, MatView A, const float *__restrict__ 
         return;
     }
     const float x1 = c0 * bi;
-    const float r = bi - c0 * row_dot(A, i, b);
+    int64_t base;
+    int w, ln;
+    row_of(A, i, base, w, ln);
+    const float r = bi - c0 * fine_dot(A, base, w, ln, b);
     const float dn = c1 * x1 + c2 * r;
     d[i] = dn;
     x_out[i] = x1 + dn;
@@ -1154,18 +1113,6 @@ __global__ void k_sm_first_step_w(Gate gate, MatView A, const float *__restrict_
     const float dn = c1 * x1 + c2 * wi * (bi - c0 * y);
     d[i] = dn;
     x_out[i] = x1 + dn;
-}
-
-template <int G>
-__global__ void __launch_bounds__(256) k_residual(Gate gate, MatView A, const float *__restrict__ b,
-                                                  const float *__restrict__ x, float *__restrict__ r) {
-    if (closed(gate)) return;
-    int64_t i;
-    int g;
-    split_row<G>(i, g);
-    const bool live = i < A.n && !is_long(A, i);  // long rows: k_long_rows
-    const float y = split_sum<G>(live ? split_part<G>(A, i, g, x) : 0.f);
-    if (g == 0 && live) r[i] = b[i] - y;
 }
 
 // b_c[I] = sum of r over the rows of coarse row I (in member order); padding rows get 0
@@ -1202,49 +1149,6 @@ __global__ void k_prolong(Gate gate, int64_t n, const int32_t *__restrict__ agg,
     if (a >= 0) x[i] += al * (wt ? wt[i] : 1.f) * xc[a];
 }
 
-// One block per long row (kLongRow): y = (A x)_i by a block reduction, then the epilogue of
-// the thread-per-row kernel it stands in for.  MODE 0: Chebyshev step (k_sm_step), 1: residual
-// (k_residual), 2: the row's terms x_i b_i and x_i (A x)_i of the coarse-correction scaling
-// (k_coarse_dots), written to long_part[2k], [2k+1], 3: power step D^-1 A x (k_power_step).
-template <int MODE>
-__global__ void __launch_bounds__(256) k_long_rows(Gate gate, MatView A, const int32_t *__restrict__ rows,
-                                                   const float *__restrict__ b, const float *__restrict__ invd,
-                                                   const float *__restrict__ x_in, float *__restrict__ out,
-                                                   float *__restrict__ d, float c1, float c2,
-                                                   double *__restrict__ long_part) {
-    if (closed(gate)) return;
-    const int64_t i = rows[blockIdx.x];
-    int64_t base;
-    int w, ln;
-    row_of(A, i, base, w, ln);
-    float y = 0.f;
-    for (int j = threadIdx.x; j < w; j += blockDim.x) {
-        const int64_t slot = base + (int64_t)j * kS + ln;
-        y += __ldg(A.val + slot) * x_in[__ldg(A.col + slot)];
-    }
-    __shared__ float red[8];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(kFull, y, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = y;
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    y = 0.f;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) y += red[k];
-    if (MODE == 0) {
-        const float di = invd ? invd[i] : 1.f;
-        const float dn = (c1 != 0.f ? c1 * d[i] : 0.f) + c2 * di * (b[i] - y);
-        d[i] = dn;
-        out[i] = x_in[i] + dn;
-    } else if (MODE == 1) {
-        out[i] = b[i] - y;
-    } else if (MODE == 3) {
-        out[i] = invd ? invd[i] * y : y;
-    } else {
-        long_part[2 * blockIdx.x] = (double)x_in[i] * (double)b[i];
-        long_part[2 * blockIdx.x + 1] = (double)x_in[i] * (double)y;
-    }
-}
-
 // long-row list: flags (1 where rlen > kLongRow) for a scan, then the compacted row indices
 __global__ void k_flag_long(int64_t n, const int32_t *rlen, int32_t *flag) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1256,25 +1160,85 @@ __global__ void k_compact_long(int64_t n, const int32_t *flag, const int32_t *po
     if (i < n && flag[i]) list[1 + pos[i]] = (int32_t)i;
 }
 
-// Energy-optimal scaling of a coarse correction: per block partials of x_c.b_c and
-// x_c.(A_c x_c) (the fine-level quantities e.r and e.Ae for e = P x_c).
-template <int G>
-__global__ void __launch_bounds__(256) k_coarse_dots(Gate gate, MatView A, const float *__restrict__ x,
-                                                     const float *__restrict__ b, double *__restrict__ part,
-                                                     unsigned int *ticket, double *alpha,
-                                                     const double *__restrict__ long_part, int32_t n_long) {
-    if (closed(gate)) return;
-    int64_t i;
-    int g;
-    split_row<G>(i, g);
-    const bool live = i < A.n && !is_long(A, i);  // long rows' terms come from k_long_rows in long_part
-    const float y = split_sum<G>(live ? split_part<G>(A, i, g, x) : 0.f);
-    double xb = 0.0, xax = 0.0;
-    if (g == 0 && live) {
-        const double xi = (double)x[i];
-        xb = xi * (double)b[i];
-        xax = xi * (double)y;
+// ---- row kernels ----------------------------------------------------------------------------
+// The cycle's (and the power iteration's) passes over a level's rows, y = (A x)_i with
+//   kRowStep   d = c1 d + c2 D^-1 (b - y), out = x + d: a Chebyshev step (c1 = 0: d is not read; dx:
+//              the sequence's second step, whose d is x itself; wd: a later step reads d)
+//   kRowResid  out = b - y
+//   kRowDots   alpha = x.b / x.y, the energy-optimal scaling of a coarse correction (the fine-level
+//              quantities e.r and e.Ae for e = P x), by the last block in block order
+//   kRowPower  out = D^-1 y
+// Rows of more than kLongRow entries get a block each, behind the blocks of the others in the same
+// launch (as launches of their own they cost 2.5-3 us each, 26 of them in a cycle of the n = 96 system).
+enum RowOp : int { kRowStep, kRowResid, kRowDots, kRowPower };
+struct RowArgs {
+    Gate gate;
+    MatView A;
+    const float *b, *invd, *x;
+    float *out, *d;
+    float c1, c2;
+    int dx, wd;
+    const int32_t *agg;       // kRowStep: rows outside the hierarchy (agg < 0) are solved exactly
+    const int32_t *longrows;
+    int32_t n_long;
+    unsigned int row_blocks;  // blocks of the other rows; block row_blocks + k takes long row k
+    double *part, *long_part, *alpha;
+    unsigned int *ticket;
+};
+
+// the step's arithmetic, rounding for rounding the same in every kernel that has it
+__device__ __forceinline__ float coarse_step(float b, float y, float di, float d, float c1, float c2) {
+    return __fmaf_rn(__fmul_rn(c2, di), __fadd_rn(b, -y), __fmul_rn(c1, d));
+}
+
+template <int OP>
+__device__ __forceinline__ void row_finish(const RowArgs &a, int64_t i, float y, float b, float x, float di, float d,
+                                           bool outside) {
+    if (OP == kRowStep) {
+        const float dn = coarse_step(b, y, di, d, a.c1, a.c2);
+        if (a.wd) a.d[i] = outside ? 0.f : dn;
+        a.out[i] = outside ? __fmul_rn(di, b) : __fadd_rn(x, dn);  // outside the hierarchy: exact
+    } else if (OP == kRowResid) {
+        a.out[i] = __fadd_rn(b, -y);
+    } else if (OP == kRowPower) {
+        a.out[i] = di * y;
     }
+}
+template <int OP> __device__ __forceinline__ float own_d(const RowArgs &a, int64_t i, float x) {
+    return OP == kRowStep && a.c1 != 0.f ? (a.dx ? x : a.d[i]) : 0.f;
+}
+
+// a long row by the whole block (256 threads)
+template <int OP> __device__ void long_row(const RowArgs &a, int k) {
+    const int64_t i = a.longrows[k];
+    int64_t base;
+    int w, ln;
+    row_of(a.A, i, base, w, ln);
+    float y = 0.f;
+    for (int j = threadIdx.x; j < w; j += 256) {
+        const int64_t slot = base + (int64_t)j * kS + ln;
+        y = __fmaf_rn(__ldg(a.A.val + slot), a.x[__ldg(a.A.col + slot)], y);
+    }
+    __shared__ float red[8];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(kFull, y, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = y;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    y = 0.f;
+    for (int q = 0; q < 8; ++q) y += red[q];
+    if (OP == kRowDots) {
+        a.long_part[2 * k] = (double)a.x[i] * (double)a.b[i];
+        a.long_part[2 * k + 1] = (double)a.x[i] * (double)y;
+    } else {
+        const float x = OP == kRowStep ? a.x[i] : 0.f;
+        row_finish<OP>(a, i, y, OP == kRowPower ? 0.f : a.b[i], x, a.invd ? a.invd[i] : 1.f, own_d<OP>(a, i, x), false);
+    }
+}
+
+// kRowDots: the block's terms (in thread 0), and in the last block to arrive the sums of all
+// blocks' and long rows' terms in order
+__device__ void dots_finish(const RowArgs &a, double xb, double xax, bool has_terms) {
     __shared__ double sh[2][8];
     __shared__ bool am_last;
 #pragma unroll
@@ -1289,31 +1253,32 @@ __global__ void __launch_bounds__(256) k_coarse_dots(Gate gate, MatView A, const
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        double a = 0.0, c = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-            a += sh[0][w];
-            c += sh[1][w];
+        if (has_terms) {
+            double s = 0.0, c = 0.0;
+            for (int w = 0; w < 8; ++w) {
+                s += sh[0][w];
+                c += sh[1][w];
+            }
+            a.part[2 * blockIdx.x] = s;
+            a.part[2 * blockIdx.x + 1] = c;
         }
-        part[2 * blockIdx.x] = a;
-        part[2 * blockIdx.x + 1] = c;
         __threadfence();
-        am_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        am_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (!am_last) return;
-    // the last block: alpha from the partials in block order (deterministic)
     __threadfence();
     __shared__ double red[2][256];
-    double a = 0.0, c = 0.0;
-    for (int64_t k = threadIdx.x; k < gridDim.x; k += blockDim.x) {
-        a += __ldcg(part + 2 * k);
-        c += __ldcg(part + 2 * k + 1);
+    double s = 0.0, c = 0.0;
+    for (int64_t k = threadIdx.x; k < a.row_blocks; k += 256) {
+        s += __ldcg(a.part + 2 * k);
+        c += __ldcg(a.part + 2 * k + 1);
     }
-    for (int k = threadIdx.x; k < n_long; k += blockDim.x) {
-        a += __ldcg(long_part + 2 * k);
-        c += __ldcg(long_part + 2 * k + 1);
+    for (int k = threadIdx.x; k < a.n_long; k += 256) {
+        s += __ldcg(a.long_part + 2 * k);
+        c += __ldcg(a.long_part + 2 * k + 1);
     }
-    red[0][threadIdx.x] = a;
+    red[0][threadIdx.x] = s;
     red[1][threadIdx.x] = c;
     __syncthreads();
     for (int st = 128; st > 0; st >>= 1) {
@@ -1325,9 +1290,139 @@ __global__ void __launch_bounds__(256) k_coarse_dots(Gate gate, MatView A, const
     }
     if (threadIdx.x == 0) {
         const double num = red[0][0], den = red[1][0];
-        *alpha = (den > 0.0 && num > 0.0 && isfinite(num / den)) ? num / den : 1.0;
-        *ticket = 0u;
+        *a.alpha = (den > 0.0 && num > 0.0 && isfinite(num / den)) ? num / den : 1.0;
+        *a.ticket = 0u;
     }
+}
+
+// G warps per slice (split_row).  The row's extent and its own entries are loaded before the gate
+// is looked at.
+template <int G, int OP> __global__ void __launch_bounds__(256, 8) k_rows(RowArgs a) {
+    if (blockIdx.x >= a.row_blocks) {
+        if (closed(a.gate)) return;
+        long_row<OP>(a, (int)(blockIdx.x - a.row_blocks));
+        if (OP == kRowDots) dots_finish(a, 0.0, 0.0, false);
+        return;
+    }
+    const MatView &A = a.A;
+    int64_t i, base = 0;
+    int g, w = 0, ln = 0;
+    split_row<G>(i, g);
+    const bool in = i < A.n;
+    bool outside = false, live = in;
+    float b = 0.f, x = 0.f, di = 1.f;
+    if (in) {
+        row_of(A, i, base, w, ln);
+        live = !A.rlen || A.rlen[i] <= kLongRow;
+        if (OP == kRowStep) outside = a.agg && a.agg[i] < 0;
+        if (g == 0) {
+            if (OP != kRowPower) b = a.b[i];
+            if (OP == kRowStep || OP == kRowDots) x = a.x[i];
+            if ((OP == kRowStep || OP == kRowPower) && a.invd) di = a.invd[i];
+        }
+    }
+    if (closed(a.gate)) return;
+    const float y = split_sum<G>(live && !outside ? split_part<G>(A, base, w, ln, g, a.x) : 0.f);
+    if (OP == kRowDots) {
+        const bool mine = g == 0 && live;
+        dots_finish(a, mine ? (double)x * (double)b : 0.0, mine ? (double)x * (double)y : 0.0, true);
+    } else if (g == 0 && live) {
+        row_finish<OP>(a, i, y, b, x, di, own_d<OP>(a, i, x), outside);
+    }
+}
+
+// The same on levels with many slices, one warp per slice: the blocks are persistent and each warp
+// runs through its slices' slots in chunks of eight, with the next chunk's slots (the next
+// slice's first, its rows' extents and own entries already there) under way while the current
+// chunk's gathers are.  One slice per group of warps and launch waits on the chain extent ->
+// slots -> gathers at 4.0-4.4 TB/s.  Measured, a step: 975k rows of 11 entries 28 -> 22 us, 1.0M of
+// 19 37 -> 37, 462k of 24 27 -> 25, 3.7M of 11 97 -> 92; the scaling's pass 31 -> 21 and 111 -> 81.
+template <int OP> __global__ void __launch_bounds__(256, 3) k_rows_pipe(RowArgs a) {
+    if (blockIdx.x >= a.row_blocks) {
+        if (closed(a.gate)) return;
+        long_row<OP>(a, (int)(blockIdx.x - a.row_blocks));
+        if (OP == kRowDots) dots_finish(a, 0.0, 0.0, false);
+        return;
+    }
+    const MatView &A = a.A;
+    const int lane = threadIdx.x & 31;
+    const int64_t n_sl = A.n / kS, step = (int64_t)a.row_blocks * 8;
+    constexpr int kB = 8;
+    struct Row {  // a slice's row of this lane
+        int64_t base, i;
+        int len, most;  // slots of the row (0: outside or long), of the slice's longest row
+        float b, x, di, d;
+        bool outside, live;
+    };
+    auto open = [&](int64_t sl, Row &r) {
+        r.i = sl * kS + lane;
+        r.base = A.off[sl];
+        const int rl = A.rlen[r.i];
+        r.live = rl <= kLongRow;
+        r.outside = OP == kRowStep && a.agg && a.agg[r.i] < 0;
+        r.len = r.live && !r.outside ? rl : 0;
+        r.b = OP != kRowPower ? a.b[r.i] : 0.f;
+        r.x = OP == kRowStep || OP == kRowDots ? a.x[r.i] : 0.f;
+        r.di = (OP == kRowStep || OP == kRowPower) && a.invd ? a.invd[r.i] : 1.f;
+        r.d = own_d<OP>(a, r.i, r.x);
+    };
+    int32_t c[kB];
+    float v[kB];
+    auto load = [&](const Row &r, int j0) {
+#pragma unroll
+        for (int k = 0; k < kB; ++k) {
+            const bool in = j0 + k < r.len;
+            const int64_t slot = r.base + (int64_t)(j0 + k) * kS + lane;
+            c[k] = in ? __ldcs(A.col + slot) : -1;
+            v[k] = in ? __ldcs(A.val + slot) : 0.f;
+        }
+    };
+    double xb = 0.0, xax = 0.0;
+    int64_t sl = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5), s1 = sl + step;
+    Row r, nx;
+    const bool any = sl < n_sl;
+    if (any) {
+        open(sl, r);
+        if (s1 < n_sl) open(s1, nx);
+    }
+    if (closed(a.gate)) return;
+    if (any) {
+        r.most = __reduce_max_sync(kFull, r.len);
+        load(r, 0);
+        int j0 = 0;
+        float y = 0.f;
+        for (;;) {
+            float gx[kB], vv[kB];
+#pragma unroll
+            for (int k = 0; k < kB; ++k) gx[k] = c[k] >= 0 ? a.x[c[k]] : 0.f;
+#pragma unroll
+            for (int k = 0; k < kB; ++k) vv[k] = v[k];
+            const bool last = j0 + kB >= r.most;
+            if (!last) load(r, j0 + kB);
+            else if (s1 < n_sl) load(nx, 0);
+#pragma unroll
+            for (int k = 0; k < kB; ++k) y = __fmaf_rn(vv[k], gx[k], y);
+            j0 += kB;
+            if (!last) continue;
+            if (OP == kRowDots) {
+                if (r.live) {
+                    xb += (double)r.x * (double)r.b;
+                    xax += (double)r.x * (double)y;
+                }
+            } else if (r.live) {
+                row_finish<OP>(a, r.i, y, r.b, r.x, r.di, r.d, r.outside);
+            }
+            if (s1 >= n_sl) break;
+            r = nx;
+            r.most = __reduce_max_sync(kFull, r.len);
+            sl = s1;
+            s1 += step;
+            if (s1 < n_sl) open(s1, nx);
+            j0 = 0;
+            y = 0.f;
+        }
+    }
+    if (OP == kRowDots) dots_finish(a, xb, xax, true);
 }
 
 // The fine level's update arithmetic, rounding for rounding the same in every kernel that has it
@@ -1654,13 +1749,13 @@ constexpr int kTailThreads = 1024, kTailWarps = kTailThreads / 32;
 constexpr int kTailGroups = kTailThreads / 256;  // 256-thread groups per CTA
 
 enum TailOp : int32_t {
-    kTailStep = 0,           // Chebyshev step (k_sm_step + k_long_rows<0>)
-    kTailResid = 1,          // residual (k_residual + k_long_rows<1>)
+    kTailStep = 0,           // Chebyshev step (kRowStep)
+    kTailResid = 1,          // residual (kRowResid)
     kTailRestrict = 2,       // restriction (k_restrict)
     kTailRestrictFirst = 3,  // restriction and the coarse level's first step (k_restrict_first)
     kTailFirst = 4,          // first step from zero (k_sm_first)
     kTailDense = 5,          // dense coarsest solve (k_dense_gemv)
-    kTailDots = 6,           // coarse-correction scaling (k_long_rows<2> + k_coarse_dots)
+    kTailDots = 6,           // coarse-correction scaling (kRowDots)
     kTailProlong = 7         // prolongation (k_prolong)
 };
 
@@ -1709,14 +1804,14 @@ __device__ __forceinline__ float tail_part(const MatView &A, int64_t i, int g, i
 #pragma unroll
         for (int k = 0; k < kB; ++k) gx[k] = j0 + k * G < w ? __ldcg(x + c[k]) : 0.f;
 #pragma unroll
-        for (int k = 0; k < kB; ++k) y += v[k] * gx[k];
+        for (int k = 0; k < kB; ++k) y = __fmaf_rn(v[k], gx[k], y);
     }
     return y;
 }
 
 // Step, Resid or Dots over the regular rows of a level: rounds of 32 warps per CTA, warp gw of
 // the cluster-wide virtual grid taking slice gw / G, part g = gw % G (split_row's mapping);
-// Dots leaves its per-256-thread-group partials (k_coarse_dots' blocks) in part.
+// Dots leaves its per-256-thread-group partials (kRowDots' blocks) in part.
 __device__ void tail_rows(const TailPhase &p, const TailLevel &L, int cta, int n_cta, double *__restrict__ part,
                           float (*sh)[32], double (*shd)[kTailWarps]) {
     const MatView &A = L.A;
@@ -1774,24 +1869,23 @@ __device__ void tail_rows(const TailPhase &p, const TailLevel &L, int cta, int n
         }
         if (g != 0 || i >= A.n) continue;
         if (p.op == kTailResid) {
-            if (live) p.x_out[i] = __ldcg(p.b + i) - y;
+            if (live) p.x_out[i] = __fadd_rn(__ldcg(p.b + i), -y);
             continue;
         }
         const float di = L.invd ? __ldg(L.invd + i) : 1.f;
         if (outside) {
             p.d[i] = 0.f;
-            p.x_out[i] = di * __ldcg(p.b + i);
+            p.x_out[i] = __fmul_rn(di, __ldcg(p.b + i));
             continue;
         }
         if (!live) continue;
-        const float rr = __ldcg(p.b + i) - y;
-        const float dn = (p.c1 != 0.f ? p.c1 * __ldcg(p.d + i) : 0.f) + p.c2 * di * rr;
+        const float dn = coarse_step(__ldcg(p.b + i), y, di, p.c1 != 0.f ? __ldcg(p.d + i) : 0.f, p.c1, p.c2);
         p.d[i] = dn;
-        p.x_out[i] = __ldcg(p.x_in + i) + dn;
+        p.x_out[i] = __fadd_rn(__ldcg(p.x_in + i), dn);
     }
 }
 
-// the long rows of a level: 256-thread groups, one row each (k_long_rows' block); Dots leaves
+// the long rows of a level: 256-thread groups, one row each (long_row); Dots leaves
 // the rows' terms in long_part
 __device__ void tail_long(const TailPhase &p, const TailLevel &L, int cta, int n_cta, double *__restrict__ long_part,
                           float (*red)[8]) {
@@ -1810,7 +1904,7 @@ __device__ void tail_long(const TailPhase &p, const TailLevel &L, int cta, int n
             row_of(A, i, base, w, ln);
             for (int j = t; j < w; j += 256) {
                 const int64_t slot = base + (int64_t)j * kS + ln;
-                y += __ldg(A.val + slot) * __ldcg(p.x_in + __ldg(A.col + slot));
+                y = __fmaf_rn(__ldg(A.val + slot), __ldcg(p.x_in + __ldg(A.col + slot)), y);
             }
         }
 #pragma unroll
@@ -1822,11 +1916,12 @@ __device__ void tail_long(const TailPhase &p, const TailLevel &L, int cta, int n
             for (int q = 0; q < 8; ++q) y += red[grp][q];
             if (p.op == kTailStep) {
                 const float di = L.invd ? __ldg(L.invd + i) : 1.f;
-                const float dn = (p.c1 != 0.f ? p.c1 * __ldcg(p.d + i) : 0.f) + p.c2 * di * (__ldcg(p.b + i) - y);
+                const float dn =
+                    coarse_step(__ldcg(p.b + i), y, di, p.c1 != 0.f ? __ldcg(p.d + i) : 0.f, p.c1, p.c2);
                 p.d[i] = dn;
-                p.x_out[i] = __ldcg(p.x_in + i) + dn;
+                p.x_out[i] = __fadd_rn(__ldcg(p.x_in + i), dn);
             } else if (p.op == kTailResid) {
-                p.x_out[i] = __ldcg(p.b + i) - y;
+                p.x_out[i] = __fadd_rn(__ldcg(p.b + i), -y);
             } else {
                 const double xi = (double)__ldcg(p.x_in + i);
                 __stcg(long_part + 2 * k, xi * (double)__ldcg(p.b + i));
@@ -1861,7 +1956,7 @@ __global__ void __launch_bounds__(kTailThreads, 1)
                 tail_rows(p, L, cta, n_cta, scratch, sh, shd);
                 tail_long(p, L, cta, n_cta, scratch + long_off, red);
                 cluster.sync();
-                // the factor from the partials in k_coarse_dots' order, by the first CTA
+                // the factor from the partials in dots_finish's order, by the first CTA
                 if (cta == 0) {
                     const int64_t n_vb = (L.A.n / kS * L.g + 7) / 8;
                     double a = 0.0, c = 0.0;
@@ -1959,15 +2054,9 @@ __global__ void __launch_bounds__(kTailThreads, 1)
     }
 }
 
-// the row kernels of a level with G warps per slice (G = 1, 2, 4 or 8)
-decltype(&k_sm_step<1>) sm_step_kernel(int g) {
-    return g >= 8 ? k_sm_step<8> : g >= 4 ? k_sm_step<4> : g >= 2 ? k_sm_step<2> : k_sm_step<1>;
-}
-decltype(&k_residual<1>) residual_kernel(int g) {
-    return g >= 8 ? k_residual<8> : g >= 4 ? k_residual<4> : g >= 2 ? k_residual<2> : k_residual<1>;
-}
-decltype(&k_coarse_dots<1>) coarse_dots_kernel(int g) {
-    return g >= 8 ? k_coarse_dots<8> : g >= 4 ? k_coarse_dots<4> : g >= 2 ? k_coarse_dots<2> : k_coarse_dots<1>;
+// the row kernel of a level with G warps per slice (G = 1, 2, 4 or 8)
+template <int OP> decltype(&k_rows<1, OP>) rows_kernel(int g) {
+    return g >= 8 ? k_rows<8, OP> : g >= 4 ? k_rows<4, OP> : g >= 2 ? k_rows<2, OP> : k_rows<1, OP>;
 }
 decltype(&k_level_diag<1>) level_diag_kernel(int g) {
     return g >= 8 ? k_level_diag<8> : g >= 4 ? k_level_diag<4> : g >= 2 ? k_level_diag<2> : k_level_diag<1>;
@@ -1977,7 +2066,16 @@ decltype(&k_pair_want<1>) pair_want_kernel(int g) {
 }
 // blocks of 8 warps covering n rows (a multiple of 32) with G warps per slice
 unsigned split_blocks(int64_t n, int g) { return nblk(n / kS * g, 8); }
-unsigned row_blocks(const AmgLevel &L) { return split_blocks(L.A.n, L.g); }
+unsigned row_blocks(const AmgLevel &L) { return L.pipe ? L.pipe : split_blocks(L.A.n, L.g); }
+template <int OP> void launch_rows(const AmgLevel &L, RowArgs a, cudaStream_t s) {
+    a.A = view(L.A);
+    a.longrows = L.A.longrows;
+    a.n_long = (int32_t)std::max<int64_t>(0, L.A.n_long);
+    a.row_blocks = row_blocks(L);
+    const unsigned grid = a.row_blocks + (unsigned)a.n_long;
+    if (L.pipe) k_rows_pipe<OP><<<grid, 256, 0, s>>>(a);
+    else rows_kernel<OP>(L.g)<<<grid, 256, 0, s>>>(a);
+}
 // warps per slice for a matrix: the fewest with at most `width` slots per warp and row (one on
 // the fine level, whose 7-8 entries per row are loaded together by each thread)
 int split_of(const AmgMatrix &A, int forced, int width) {
@@ -2106,8 +2204,7 @@ cudaError_t Amg::level_stats(AmgLevel &L, unsigned int *bound, cudaStream_t s) {
 }
 
 // ---- spectral estimates ---------------------------------------------------------------------
-// One power-iteration step y = D^-1 A x (thread per row over the whole row, long rows included:
-// setup only).  The start vector is a fixed pseudo-random sign pattern of amplitude in [0.5, 1)
+// The power iteration's steps y = D^-1 A x are the cycle's row kernels (kRowPower).  The start vector is a fixed pseudo-random sign pattern of amplitude in [0.5, 1)
 // (no scaling between steps: |D^-1 A| <= a few, so 12 steps stay far from FP32 overflow).
 __global__ void k_power_start(int64_t n, float *x) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -2117,20 +2214,6 @@ __global__ void k_power_start(int64_t n, float *x) {
     h *= 2246822519u;
     h ^= h >> 13;
     x[i] = ((h & 1u) ? 1.f : -1.f) * (0.5f + (float)((h >> 8) & 0xffffu) * (0.5f / 65536.f));
-}
-
-// y = D^-1 A x with the cycle's row kernels' split (G warps per slice, eight loads in flight);
-// the long rows are left to k_long_rows<3>
-template <int G>
-__global__ void __launch_bounds__(256) k_power_step(MatView A, const float *__restrict__ invd,
-                                                    const float *__restrict__ x, float *__restrict__ y) {
-    int64_t i;
-    int g;
-    split_row<G>(i, g);
-    const bool live = i < A.n && !is_long(A, i);
-    const float acc = split_sum<G>(live ? split_part<G>(A, i, g, x) : 0.f);
-    if (g != 0 || !live) return;
-    y[i] = invd ? invd[i] * acc : acc;
 }
 
 // per-block partial sums of x.x and y.y (fixed grid, fixed tree: deterministic)
@@ -2190,15 +2273,22 @@ __global__ void __launch_bounds__(256) k_fine_bound(MatView A, const float *__re
     }
 }
 
+// the totals of the partials, by one warp in a fixed order
 __global__ void k_power_total(const double *__restrict__ part, int nb, double *__restrict__ out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
     double a = 0.0, b = 0.0;
-    for (int k = 0; k < nb; ++k) {
+    for (int k = threadIdx.x; k < nb; k += 32) {
         a += part[2 * k];
         b += part[2 * k + 1];
     }
-    out[0] = a;
-    out[1] = b;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(kFull, a, o);
+        b += __shfl_xor_sync(kFull, b, o);
+    }
+    if (threadIdx.x == 0) {
+        out[0] = a;
+        out[1] = b;
+    }
 }
 
 // One pairing pass on A (rows excluded by row_edge < 0 or without coupling get agg = -1):
@@ -2334,6 +2424,11 @@ cudaError_t Amg::dense_coarse(const AmgMatrix &A, bool &ok, cudaStream_t s) {
 cudaError_t Amg::setup(const DevSystem &sys, const AmgOptions &o, cudaStream_t s) {
     opt_ = o;
     if (!h_flag_) AMG_CK(cudaHostAlloc((void **)&h_flag_, sizeof(int32_t), cudaHostAllocDefault));
+    if (sms_ == 0) {
+        int dev = 0;
+        AMG_CK(cudaGetDevice(&dev));
+        AMG_CK(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
+    }
     // device words the setup fills and the host reads once at its end: the Gershgorin bound of
     // each level, and the Galerkin overflow flag
     AMG_CK(bounds_.ensure(o.max_levels + 1));
@@ -2489,6 +2584,9 @@ cudaError_t Amg::setup(const DevSystem &sys, const AmgOptions &o, cudaStream_t s
             // warps per slice in the row kernels: at most split_width slots per warp and row
             // (the fine level, 7-8 entries per row, keeps one thread per row)
             lv_[l].g = split_of(lv_[l].A, opt_.split, opt_.split_width);
+            // levels with at least two slices for every warp of the chip (three blocks of eight to
+            // an SM): the persistent row kernels
+            lv_[l].pipe = lv_[l].A.rlen && lv_[l].A.n_slices >= 2 * 8 * 3 * (int64_t)sms_ ? 3u * (unsigned)sms_ : 0u;
         }
         if ((e2 = power_estimates(s)) != cudaSuccess) return e2;
         if (opt_.power_steps > 0) {
@@ -2528,10 +2626,7 @@ cudaError_t Amg::setup(const DevSystem &sys, const AmgOptions &o, cudaStream_t s
     }
     w0_used_ = w0;
     if (opt_.half_fine && n_levels_ > 1) {
-        int dev = 0, sms = 0;
-        AMG_CK(cudaGetDevice(&dev));
-        AMG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        fine_grid_ = 4 * sms;  // k_fine: four blocks to an SM
+        fine_grid_ = 4 * sms_;  // k_fine: four blocks to an SM
         AMG_CK(fine_out_.ensure(L0.A.n_slices));
         k_outside_bits<<<nblk(L0.A.n, 256), 256, 0, s>>>(L0.A.n, L0.agg.p, fine_out_.p);
         AMG_CK(cudaGetLastError());
@@ -2586,20 +2681,14 @@ cudaError_t Amg::power_estimates(cudaStream_t s, int only_level) {
         // the fine level is the Jacobi-scaled system (unit diagonal): no D^-1, or the
         // smoother's row weights
         const float *invd = l == 0 ? fw() : L.inv_diag.p;
-        const MatView V = view(L.A);
         float *x = pw_a_.p, *y = pw_b_.p;
         k_power_start<<<nblk(n, 256), 256, 0, s>>>(n, x);
         for (int k = 0; k < opt_.power_steps; ++k) {
-            const unsigned gs = row_blocks(L);
-            switch (L.g >= 8 ? 8 : L.g >= 4 ? 4 : L.g >= 2 ? 2 : 1) {
-                case 8: k_power_step<8><<<gs, 256, 0, s>>>(V, invd, x, y); break;
-                case 4: k_power_step<4><<<gs, 256, 0, s>>>(V, invd, x, y); break;
-                case 2: k_power_step<2><<<gs, 256, 0, s>>>(V, invd, x, y); break;
-                default: k_power_step<1><<<gs, 256, 0, s>>>(V, invd, x, y); break;
-            }
-            if (L.A.n_long > 0)
-                k_long_rows<3><<<(unsigned)L.A.n_long, 256, 0, s>>>(Gate{nullptr, 0}, V, L.A.longrows, nullptr, invd,
-                                                                    x, y, nullptr, 0.f, 0.f, nullptr);
+            RowArgs a = {};
+            a.x = x;
+            a.out = y;
+            a.invd = invd;
+            launch_rows<kRowPower>(L, a, s);
             if (k + 1 < opt_.power_steps) std::swap(x, y);
         }
         k_power_norms<<<kPowerBlocks, 256, 0, s>>>(n, x, y, pw_part_.p);
@@ -2669,7 +2758,7 @@ void Amg::cheb_coeffs(const AmgLevel &L, std::vector<double> &c1, std::vector<do
 int Amg::kernels_per_apply() const {
     const int deg = std::max(1, opt_.cheb_degree), pre = pre_degree();
     const int coarse = dense_n_ > 0 ? 1 : std::max(1, opt_.coarse_degree);
-    return last_long_launches_ + (n_levels_ - 1) * (pre + deg + 3) + coarse - std::max(0, n_levels_ - 2) -
+    return (n_levels_ - 1) * (pre + deg + 3) + coarse - std::max(0, n_levels_ - 2) -
            (n_levels_ > 1 && pre >= 2 ? 1 : 0) +
            (opt_.kcycle ? std::min(opt_.kcycle_levels, std::max(0, n_levels_ - (dense_n_ > 0 ? 2 : 1))) : 0) -
            (tail_phases_ > 0 ? tail_regular_ - 1 : 0);
@@ -2953,19 +3042,22 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
                        AmgProf *prof, float **x_l0) {
     const Gate gate_{n_done, n_inst};
     const int pre = pre_degree();
-    int launches = 0;  // kernels of one cycle, for the launch count
-    auto long_rows = [&](const AmgMatrix &M, int mode, const float *b, const float *invd, const float *x_in,
-                         float *out, float *d, float c1, float c2, double *part) {
-        if (M.n_long <= 0) return;
-        const unsigned gl = (unsigned)M.n_long;
-        const MatView V = view(M);
-        if (mode == 0)
-            k_long_rows<0><<<gl, 256, 0, s>>>(gate_, V, M.longrows, b, invd, x_in, out, d, c1, c2, part);
-        else if (mode == 1)
-            k_long_rows<1><<<gl, 256, 0, s>>>(gate_, V, M.longrows, b, invd, x_in, out, d, c1, c2, part);
-        else
-            k_long_rows<2><<<gl, 256, 0, s>>>(gate_, V, M.longrows, b, invd, x_in, out, d, c1, c2, part);
-        ++launches;
+    // a Chebyshev step of a level; dx: d is x_in (the second step), more: a later step reads d
+    auto step = [&](const AmgLevel &L, const float *b, const float *invd, const float *xi, float *xo, float c1,
+                    float c2, bool dx, bool more, const int32_t *agg) {
+        RowArgs a = {};
+        a.gate = gate_;
+        a.b = b;
+        a.invd = invd;
+        a.x = xi;
+        a.out = xo;
+        a.d = L.d.p;
+        a.c1 = c1;
+        a.c2 = c2;
+        a.dx = dx;
+        a.wd = more;
+        a.agg = agg;
+        launch_rows<kRowStep>(L, a, s);
     };
     // inside a capture only cudaEventRecordExternal turns a record into a graph node
     auto rec = [&](cudaEvent_t ev) {
@@ -3002,9 +3094,7 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
         const float *b = l == 0 ? r : L.b.p;
         // the scaled fine level has unit diagonal; with smoother weights Omega, D^-1 -> Omega
         const float *invd = l == 0 ? fw() : L.inv_diag.p;
-        const MatView A = view(L.A);
-        const unsigned g = nblk(L.A.n, 256), gs = row_blocks(L);
-        const auto sm_step = sm_step_kernel(L.g);
+        const unsigned g = nblk(L.A.n, 256);
         cheb_coeffs(L, c1, c2);
         float *xi = L.xa.p, *xo = L.xb.p;
         int k0 = 1;
@@ -3015,19 +3105,19 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
                                        : (pre > 2 ? k_fine<kOpFirst, false, true> : k_fine<kOpFirst, false, false>);
                 f<<<gf, 256, 0, s>>>(gate_, F, b, fw(), b, xo, L.d.p, (float)c2[0], (float)c1[1], (float)c2[1]);
             } else if (fine_w_)
-                k_sm_first_step_w<<<g, 256, 0, s>>>(gate_, A, b, fw(), xo, L.d.p, (float)c2[0], (float)c1[1],
+                k_sm_first_step_w<<<g, 256, 0, s>>>(gate_, view(L.A), b, fw(), xo, L.d.p, (float)c2[0], (float)c1[1],
                                                     (float)c2[1], L.agg.p);
             else if (tma0)
                 launch_fine<kFineFirst>(n_done, n_inst, b, nullptr, nullptr, xo, L.d.p, (float)c2[0], (float)c1[1],
                                         (float)c2[1], s);
             else
-                k_sm_first_step<<<g, 256, 0, s>>>(gate_, A, b, xo, L.d.p, (float)c2[0], (float)c1[1], (float)c2[1],
+                k_sm_first_step<<<g, 256, 0, s>>>(gate_, view(L.A), b, xo, L.d.p, (float)c2[0], (float)c1[1], (float)c2[1],
                                                   L.agg.p);
             rec_step(false);
             std::swap(xi, xo);
             k0 = 2;
         } else if (l == 0 || l == l0) {  // (a cycle started below the fine level: its first step)
-            k_sm_first<<<g, 256, 0, s>>>(gate_, L.A.n, b, invd, (float)c2[0], xi, L.d.p, L.agg.p);
+            k_sm_first<<<g, 256, 0, s>>>(gate_, L.A.n, b, invd, (float)c2[0], xi, nullptr, L.agg.p);
         }
         // (coarser levels: the first step was fused into the restriction from the level above)
         for (int k = k0; k < pre; ++k) {
@@ -3037,8 +3127,7 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
             else if (l == 0 && half0)
                 fine_step0(b, invd, xi, xo, L.d.p, (float)c1[k], (float)c2[k], k + 1 < pre);
             else
-                sm_step<<<gs, 256, 0, s>>>(gate_, A, b, invd, xi, xo, L.d.p, (float)c1[k], (float)c2[k], L.agg.p);
-            long_rows(L.A, 0, b, invd, xi, xo, L.d.p, (float)c1[k], (float)c2[k], nullptr);
+                step(L, b, invd, xi, xo, (float)c1[k], (float)c2[k], k == 1, k + 1 < pre, L.agg.p);
             if (l == 0) rec_step(false);
             std::swap(xi, xo);
         }
@@ -3047,16 +3136,22 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
             launch_fine<kFineResid>(n_done, n_inst, b, nullptr, xi, L.r.p, nullptr, 0.f, 0.f, 0.f, s);
         else if (l == 0 && half0)
             k_fine<kOpResid, false, false><<<gf, 256, 0, s>>>(gate_, F, b, nullptr, xi, L.r.p, nullptr, 0.f, 0.f, 0.f);
-        else
-            residual_kernel(L.g)<<<gs, 256, 0, s>>>(gate_, A, b, xi, L.r.p);
-        long_rows(L.A, 1, b, nullptr, xi, L.r.p, nullptr, 0.f, 0.f, nullptr);
+        else {
+            RowArgs a = {};
+            a.gate = gate_;
+            a.b = b;
+            a.x = xi;
+            a.out = L.r.p;
+            launch_rows<kRowResid>(L, a, s);
+        }
         AmgLevel &C = lv_[l + 1];
         const float *wt = l == 0 ? w0_used_ : nullptr;
         if (l + 2 < nl) {
             std::vector<double> cc1, cc2;
             cheb_coeffs(C, cc1, cc2);
             k_restrict_first<<<nblk(C.A.n, 256), 256, 0, s>>>(gate_, L.nc, C.A.n, L.mem_start.p, L.mem_rows.p, L.r.p, wt,
-                                                              C.inv_diag.p, (float)cc2[0], C.b.p, C.xa.p, C.d.p,
+                                                              C.inv_diag.p, (float)cc2[0], C.b.p, C.xa.p,
+                                                              use_tail && l + 1 == tail_level_ ? C.d.p : nullptr,
                                                               C.agg.p);
         } else {
             k_restrict<<<nblk(C.A.n, 256), 256, 0, s>>>(gate_, L.nc, C.A.n, L.mem_start.p, L.mem_rows.p, L.r.p, C.b.p, wt);
@@ -3076,17 +3171,14 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
                                                                  b, x);
             xout[nl - 1] = x;
         } else {
-            const unsigned g = nblk(Lc.A.n, 256), gs = row_blocks(Lc);
-            const auto sm_step = sm_step_kernel(Lc.g);
+            const unsigned g = nblk(Lc.A.n, 256);
             cheb_coeffs(Lc, c1, c2, std::max(1, opt_.coarse_degree), opt_.coarse_ratio);
             float *xi = Lc.xa.p, *xo = Lc.xb.p;
-            k_sm_first<<<g, 256, 0, s>>>(gate_, Lc.A.n, b, Lc.inv_diag.p, (float)c2[0], xi, Lc.d.p, Lc.agg.p);
+            k_sm_first<<<g, 256, 0, s>>>(gate_, Lc.A.n, b, Lc.inv_diag.p, (float)c2[0], xi, nullptr, Lc.agg.p);
             const int cdeg = std::max(1, opt_.coarse_degree);
             for (int k = 1; k < cdeg; ++k) {
                 float *xk = (nl == 1 && k == cdeg - 1) ? z : xo;
-                sm_step<<<gs, 256, 0, s>>>(gate_, view(Lc.A), b, Lc.inv_diag.p, xi, xk, Lc.d.p, (float)c1[k],
-                                           (float)c2[k], Lc.agg.p);
-                long_rows(Lc.A, 0, b, Lc.inv_diag.p, xi, xk, Lc.d.p, (float)c1[k], (float)c2[k], nullptr);
+                step(Lc, b, Lc.inv_diag.p, xi, xk, (float)c1[k], (float)c2[k], k == 1, k + 1 < cdeg, Lc.agg.p);
                 xo = xi;
                 xi = xk;
             }
@@ -3098,9 +3190,7 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
         AmgLevel &L = lv_[l];
         const float *b = l == 0 ? r : L.b.p;
         const float *invd = l == 0 ? fw() : L.inv_diag.p;
-        const MatView A = view(L.A);
-        const unsigned g = nblk(L.A.n, 256), gs = row_blocks(L);
-        const auto sm_step = sm_step_kernel(L.g);
+        const unsigned g = nblk(L.A.n, 256);
         cheb_coeffs(L, c1, c2);
         float *xi = xout[l];
         const double *al = nullptr;
@@ -3111,10 +3201,15 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
         } else if (opt_.kcycle && l < opt_.kcycle_levels && (l + 2 < nl || dense_n_ == 0)) {
             AmgLevel &C = lv_[l + 1];
             double *lp = dots_long_.p + dots_long_off_[l];
-            long_rows(C.A, 2, C.b.p, nullptr, xout[l + 1], nullptr, nullptr, 0.f, 0.f, lp);
-            coarse_dots_kernel(C.g)<<<row_blocks(C), 256, 0, s>>>(gate_, view(C.A), xout[l + 1], C.b.p,
-                                                                  dots_.p + dots_off_[l], tickets_.p + l,
-                                                                  alpha_.p + l, lp, (int32_t)C.A.n_long);
+            RowArgs a = {};
+            a.gate = gate_;
+            a.b = C.b.p;
+            a.x = xout[l + 1];
+            a.part = dots_.p + dots_off_[l];
+            a.long_part = lp;
+            a.alpha = alpha_.p + l;
+            a.ticket = tickets_.p + l;
+            launch_rows<kRowDots>(C, a, s);
             al = alpha_.p + l;
         }
         k_prolong<<<g, 256, 0, s>>>(gate_, L.A.n, L.agg.p, xout[l + 1], xi, al, opt_.alpha, l == 0 ? w0_used_ : nullptr);
@@ -3128,9 +3223,7 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
             else if (l == 0 && half0)
                 fine_step0(b, invd, xi, xo, L.d.p, k == 0 ? 0.f : (float)c1[k], (float)c2[k], k + 1 < deg);
             else
-                sm_step<<<gs, 256, 0, s>>>(gate_, A, b, invd, xi, xo, L.d.p, k == 0 ? 0.f : (float)c1[k],
-                                           (float)c2[k], L.agg.p);
-            long_rows(L.A, 0, b, invd, xi, xo, L.d.p, k == 0 ? 0.f : (float)c1[k], (float)c2[k], nullptr);
+                step(L, b, invd, xi, xo, k == 0 ? 0.f : (float)c1[k], (float)c2[k], false, k + 1 < deg, L.agg.p);
             if (l == 0) rec_step(false);
             other = xi;
             xi = xo;
@@ -3138,7 +3231,6 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
         xout[l] = xi;
     }
     if (prof) rec(prof->cycle[1]);
-    if (l0 == 0) last_long_launches_ = launches;
     if (x_l0) *x_l0 = xout[l0];
     return cudaGetLastError();
 }
@@ -3164,14 +3256,24 @@ cudaError_t Amg::smooth_fine(const float *b, float *x, cudaStream_t s) {
     cheb_coeffs(L, c1, c2);
     const int pre = pre_degree();
     const float *invd = fw();
-    const MatView A = view(L.A);
     const int32_t *agg = n_levels_ > 1 ? L.agg.p : nullptr;
     const Gate g{nullptr, 0};
     float *xi = L.xa.p, *xo = L.xb.p;
-    k_sm_first<<<nblk(L.A.n, 256), 256, 0, s>>>(g, L.A.n, b, invd, (float)c2[0], xi, L.d.p, agg);
-    const auto sm_step = sm_step_kernel(L.g);
+    k_sm_first<<<nblk(L.A.n, 256), 256, 0, s>>>(g, L.A.n, b, invd, (float)c2[0], xi, nullptr, agg);
     for (int k = 1; k < pre; ++k) {
-        sm_step<<<row_blocks(L), 256, 0, s>>>(g, A, b, invd, xi, xo, L.d.p, (float)c1[k], (float)c2[k], agg);
+        RowArgs a = {};
+        a.gate = g;
+        a.b = b;
+        a.invd = invd;
+        a.x = xi;
+        a.out = xo;
+        a.d = L.d.p;
+        a.c1 = (float)c1[k];
+        a.c2 = (float)c2[k];
+        a.dx = k == 1;
+        a.wd = k + 1 < pre;
+        a.agg = agg;
+        launch_rows<kRowStep>(L, a, s);
         std::swap(xi, xo);
     }
     AMG_CK(cudaGetLastError());

@@ -92,6 +92,7 @@ struct AmgLevel {
                                                // factor, at most the Gershgorin bound
     float gershgorin = 2.f;                    // Gershgorin bound of D^-1 A
     int g = 1;                                 // warps per slice in the row kernels (amg.cu)
+    unsigned pipe = 0;                         // blocks of the persistent row kernels (0: not for this level)
 };
 
 // Events recorded inside a captured V-cycle (as external event nodes) to time it: the whole
@@ -198,7 +199,6 @@ private:
     DBuf<float> tval_;
     DBuf<double> dots_long_;        // long rows' terms of the coarse-correction scaling
     std::vector<int64_t> dots_long_off_;
-    int last_long_launches_ = 0;
     DBuf<float> isd_;
     DBuf<float> dense_inv_;         // inverse of the coarsest matrix, and the two copies it is made in
     DBuf<double> dense_work_[2];
@@ -217,6 +217,7 @@ private:
     DBuf<float> w0_;                // sqrt(diag S) per fine row
     DBuf<uint16_t> fine_half_;      // FP16 bits of the fine matrix's values (half_fine)
     DBuf<uint32_t> fine_out_;       // per fine slice, the rows outside the hierarchy
+    int sms_ = 0;
     int64_t fine_grid_ = 1;         // blocks of the fine level's persistent kernels at most
     // the fine level's TMA-staged cycle kernels (k_fine_tma): ready, stage size, grid, the
     // widest tile read at setup and the stage-wait error flag

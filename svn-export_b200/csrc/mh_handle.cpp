@@ -1522,7 +1522,7 @@ int solve_impl(mh_handle *h, const mh_solve_opts *opts_in, mh_solve_stats *stats
     // the multigrid methods (plain or with the learned smoother) take long iterations and few
     // FP64 replacements
     const bool multigrid = o.method == MH_SOLVER_AMG || o.method == MH_SOLVER_FCG_LEARNED;
-    if (o.iters_per_graph <= 0) o.iters_per_graph = multigrid ? 4 : 16;
+    if (o.iters_per_graph <= 0) o.iters_per_graph = multigrid ? 2 : 16;
     if (o.inner_max_it <= 0) o.inner_max_it = 2000;
     if (!(o.inner_rtol > 0.0)) o.inner_rtol = multigrid ? 1e-3 : 0.1;
     // MH_HOST_LOOP=1 makes the host-polled loop the default (profilers cannot see the kernels
