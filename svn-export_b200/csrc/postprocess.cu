@@ -72,77 +72,197 @@ __global__ void __launch_bounds__(128) k_element_flux(ElemData d, const int32_t 
 // ---- node pressures (make_node_scalar_param, darcy_flow_mh_output.cc:424-546) ---------------
 // A node's pressure is the mean of the pressures of the elements and element sides that
 // contain it, weighted by (1 - d / D) / (n - 1): d the distance from the node to that element's
-// or side's centre, D the sum of those distances at the node, n their number.  One thread per
-// node gathers over the node's elements (ascending, from a CSR incidence list built once per
-// mesh): first every element centre, then every side of those elements that contains the node,
-// the order in which the reference's two element loops reach the node.  No atomics: repeated
-// calls give identical bits, and with the operation order of the reference (this file is
-// compiled without FMA contraction) the result equals the FP64 restatement bit for bit.
+// or side's centre, D the sum of those distances at the node, n their number.  The sums run over
+// the node's elements (ascending, from a CSR incidence list built once per mesh): first every
+// element centre, then every side of those elements that contains the node, the order in which
+// the reference's two element loops reach the node.  No atomics: repeated calls give identical
+// bits, and with the operation order of the reference (this file is compiled without FMA
+// contraction) the result equals the FP64 restatement bit for bit.
+//
+// A thread per node is bound by the FP64 divisions and square roots of its 4 x 24 terms, twice over,
+// in one chain.  A block takes 16 nodes instead: all its threads compute the distances (a thread
+// per node and element: the centre and up to three sides) into shared memory, one lane per node adds
+// them in order, all threads turn them into weighted pressures, one lane per node adds those in
+// order.  Divisions by 3, by D and by n - 1 are products with the divisor's reciprocal and two
+// corrections, which give the correctly rounded quotient (div_known).
+// Measured (B200, 274,625 nodes of a cube with 1.57M tetrahedra): 848 -> 354 us, now bound by the instructions of
+// the distances (about 300 a term) and the latency of their loads.
 __device__ __forceinline__ double node_dist(V3 a, V3 b) {
     const V3 d = v3sub(a, b);
     return sqrt(d.x * d.x + d.y * d.y + d.z * d.z);
 }
 
-__global__ void __launch_bounds__(128) k_node_pressure(ElemData d, const int32_t *__restrict__ inc_start,
-                                                       const int32_t *__restrict__ inc_el, int64_t n_nodes,
-                                                       const double *__restrict__ sol, int64_t n_sides, int64_t n_el,
-                                                       double *__restrict__ out) {
-    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= n_nodes) return;
-    const V3 Xv = {d.xyz[3 * v], d.xyz[3 * v + 1], d.xyz[3 * v + 2]};
-    const int32_t p0 = inc_start[v], p1 = inc_start[v + 1];
-    double D = 0.0, acc = 0.0;
-    int cnt = 0;
-    // pass 0: distance sum and count; pass 1: weighted pressures (same visiting order)
-    for (int pass = 0; pass < 2; ++pass) {
-        for (int32_t q = p0; q < p1; ++q) {  // element centres
-            const int e = inc_el[q];
-            const int N = d.el_side_start[e + 1] - d.el_side_start[e];
-            V3 c = {0.0, 0.0, 0.0};
-            for (int i = 0; i < N; ++i) {
-                const int nd = d.el_nodes[4 * e + i];
-                c = {c.x + d.xyz[3 * nd], c.y + d.xyz[3 * nd + 1], c.z + d.xyz[3 * nd + 2]};
-            }
-            c = v3div(c, (double)N);
-            const double dist = node_dist(Xv, c);
-            if (pass == 0) {
-                D += dist;
-                ++cnt;
-            } else {
-                acc += sol[n_sides + e] * (1.0 - dist / D) / (cnt - 1);
-            }
-        }
-        for (int32_t q = p0; q < p1; ++q) {  // sides containing the node
-            const int e = inc_el[q];
-            const int s0 = d.el_side_start[e];
-            const int N = d.el_side_start[e + 1] - s0, dim = N - 1;
-            int nd[4];
-            int kv = 0;
-            for (int i = 0; i < N; ++i) {
-                nd[i] = d.el_nodes[4 * e + i];
-                if (nd[i] == v) kv = i;
-            }
-            for (int s = 0; s < N; ++s) {
-                bool has = false;
-                for (int k = 0; k < dim; ++k) has |= dev_side_node(dim, s, k) == kv;
-                if (!has) continue;
-                V3 cs = {0.0, 0.0, 0.0};
-                for (int k = 0; k < dim; ++k) {
-                    const int m = nd[dev_side_node(dim, s, k)];
-                    cs = {cs.x + d.xyz[3 * m], cs.y + d.xyz[3 * m + 1], cs.z + d.xyz[3 * m + 2]};
-                }
-                cs = v3div(cs, (double)dim);
-                const double dist = node_dist(Xv, cs);
-                if (pass == 0) {
-                    D += dist;
-                    ++cnt;
-                } else {
-                    acc += sol[n_sides + n_el + d.side_edge[s0 + s]] * (1.0 - dist / D) / (cnt - 1);
-                }
-            }
-        }
+// a / b, correctly rounded, with y = 1 / b correctly rounded: two corrections of a y by fma.  The
+// first leaves a quotient within one unit in the last place, the second rounds it correctly
+// (P. Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, IBM J.
+// Res. Dev. 34, 1990, theorem 8).  Operands whose products could leave the normal range are divided.
+__device__ __forceinline__ double div_known(double a, double b, double y) {
+    const double m = fabs(a), n = fabs(b);
+    if (!((m > 1e-140 && m < 1e140) && (n > 1e-140 && n < 1e140))) return a / b;
+    double q = a * y;
+    q = fma(fma(-b, q, a), y, q);
+    return fma(fma(-b, q, a), y, q);
+}
+
+// the sum of N points divided by N
+template <int N> __device__ __forceinline__ V3 mean_of(V3 c) {
+    if (N == 3) {
+        const double y = 1.0 / 3.0;
+        return {div_known(c.x, 3.0, y), div_known(c.y, 3.0, y), div_known(c.z, 3.0, y)};
     }
-    out[v] = acc;
+    return v3scale(c, N == 4 ? 0.25 : N == 2 ? 0.5 : 1.0);  // exact
+}
+
+// whether side q of an element of dimension dim contains its node kv
+__device__ __forceinline__ bool side_has(int dim, int q, int kv) {
+    if (dim == 3) return q != kv;
+    if (dim == 2) return dev_side_node(2, q, 0) == kv || dev_side_node(2, q, 1) == kv;
+    return q == kv;
+}
+
+// one node and one of its elements: f(term, distance, index into sol) for the element's centre
+// (term 0) and its sides that contain the node (terms 1, 2, ...); kv: the node's place in the element
+template <int DIM, class F>
+__device__ __forceinline__ void node_terms(const ElemData &d, int64_t v, int e, int s0, V3 Xv, int64_t n_sides,
+                                           int64_t n_el, int &kv, F f) {
+    constexpr int N = DIM + 1;
+    const int4 nd4 = reinterpret_cast<const int4 *>(d.el_nodes)[e];
+    const int nd[4] = {nd4.x, nd4.y, nd4.z, nd4.w};
+    V3 X[N], c = {0.0, 0.0, 0.0};
+    kv = 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        if (nd[i] == v) kv = i;
+        const double *x = d.xyz + 3 * (int64_t)nd[i];
+        X[i] = {x[0], x[1], x[2]};
+        c = {c.x + X[i].x, c.y + X[i].y, c.z + X[i].z};
+    }
+    f(0, node_dist(Xv, mean_of<N>(c)), n_sides + e);
+    int t = 0;
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+        bool has = false;
+        V3 cs = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int k = 0; k < DIM; ++k) {
+            const int m = dev_side_node(DIM, q, k);
+            has |= m == kv;
+            cs = {cs.x + X[m].x, cs.y + X[m].y, cs.z + X[m].z};
+        }
+        if (has) f(++t, node_dist(Xv, mean_of<DIM>(cs)), n_sides + n_el + d.side_edge[s0 + q]);
+    }
+}
+// ... of any dimension; returns the element's dimension, which is also its number of such sides
+template <class F>
+__device__ __forceinline__ int node_terms_any(const ElemData &d, int64_t v, int e, V3 Xv, int64_t n_sides, int64_t n_el,
+                                              int &kv, F f) {
+    const int s0 = d.el_side_start[e], dim = d.el_side_start[e + 1] - s0 - 1;
+    if (dim == 3) node_terms<3>(d, v, e, s0, Xv, n_sides, n_el, kv, f);
+    else if (dim == 2) node_terms<2>(d, v, e, s0, Xv, n_sides, n_el, kv, f);
+    else node_terms<1>(d, v, e, s0, Xv, n_sides, n_el, kv, f);
+    return dim;
+}
+
+// the same by one thread (nodes of so many elements that a block's terms do not fit)
+__device__ double node_pressure_serial(const ElemData &d, int64_t v, const int32_t *inc_el, int32_t p0, int32_t p1,
+                                       const double *sol, int64_t n_sides, int64_t n_el) {
+    const V3 Xv = {d.xyz[3 * v], d.xyz[3 * v + 1], d.xyz[3 * v + 2]};
+    double D = 0.0, acc = 0.0;
+    int cnt = 0, kv;
+    for (int pass = 0; pass < 2; ++pass)
+        for (int kind = 0; kind < 2; ++kind)
+            for (int32_t q = p0; q < p1; ++q)
+                node_terms_any(d, v, inc_el[q], Xv, n_sides, n_el, kv, [&](int t, double dist, int64_t at) {
+                    if ((t > 0) != (kind > 0)) return;
+                    if (pass == 0) {
+                        D += dist;
+                        ++cnt;
+                    } else {
+                        acc += sol[at] * (1.0 - dist / D) / (cnt - 1);
+                    }
+                });
+    return acc;
+}
+
+// s plus the n side terms behind a pair's first, in order
+__device__ __forceinline__ double add_sides(double s, const double *pair, int n) {
+    const double a = pair[1], b = pair[2], c = pair[3];
+    s += a;
+    if (n > 1) s += b;
+    if (n > 2) s += c;
+    return s;
+}
+
+constexpr int kNpNodes = 16, kNpThreads = 128;
+constexpr int kNpCap = 640;  // (node, element) pairs of a block: 16 nodes of 24 elements are 384
+constexpr size_t kNpSmem = (4 * kNpCap + kNpNodes) * sizeof(double) + kNpCap;
+
+__global__ void __launch_bounds__(kNpThreads, 8) k_node_pressure(ElemData d, const int32_t *__restrict__ inc_start,
+                                                              const int32_t *__restrict__ inc_el, int64_t n_nodes,
+                                                              const double *__restrict__ sol, int64_t n_sides,
+                                                              int64_t n_el, double *__restrict__ out) {
+    extern __shared__ double npm[];  // four terms per pair; one entry of padding per node (banks)
+    unsigned char *terms = reinterpret_cast<unsigned char *>(npm + 4 * kNpCap + kNpNodes);
+    __shared__ int32_t start[kNpNodes + 1];
+    __shared__ double D[kNpNodes], yD[kNpNodes], n1[kNpNodes], yn1[kNpNodes];
+    const int64_t v0 = (int64_t)blockIdx.x * kNpNodes;
+    const int nn = (int)min((int64_t)kNpNodes, n_nodes - v0), t = threadIdx.x;
+    if (t <= nn) start[t] = inc_start[v0 + t];
+    __syncthreads();
+    const int32_t first = start[0], pairs = start[nn] - first;
+    if (pairs > kNpCap) {
+        if (t < nn) out[v0 + t] = node_pressure_serial(d, v0 + t, inc_el, start[t], start[t + 1], sol, n_sides, n_el);
+        return;
+    }
+    // eight threads to a node
+    constexpr int kPer = kNpThreads / kNpNodes;
+    const int k = t / kPer;
+    const int64_t v = v0 + k;
+    const int pa = k < nn ? start[k] - first + t % kPer : 0, pb = k < nn ? start[k + 1] - first : 0;
+    for (int p = pa; p < pb; p += kPer) {
+        const V3 Xv = {d.xyz[3 * v], d.xyz[3 * v + 1], d.xyz[3 * v + 2]};
+        double *to = npm + 4 * p + k;
+        int kv;
+        const int dim = node_terms_any(d, v, inc_el[first + p], Xv, n_sides, n_el, kv,
+                                       [&](int q, double dist, int64_t) { to[q] = dist; });
+        terms[p] = (unsigned char)(dim | kv << 4);
+    }
+    __syncthreads();
+    if (t < nn) {
+        const int a = start[t] - first, b = start[t + 1] - first;
+        double s = 0.0;
+        int cnt = 0;
+        for (int p = a; p < b; ++p) s += npm[4 * p + t];
+        for (int p = a; p < b; ++p) {
+            const int q = terms[p] & 15;
+            cnt += 1 + q;
+            s = add_sides(s, npm + 4 * p + t, q);
+        }
+        D[t] = s;
+        yD[t] = 1.0 / s;
+        n1[t] = (double)(cnt - 1);
+        yn1[t] = 1.0 / n1[t];
+    }
+    __syncthreads();
+    for (int p = pa; p < pb; p += kPer) {
+        const int e = inc_el[first + p];
+        const int dim = terms[p] & 15, kv = terms[p] >> 4, s0 = d.el_side_start[e];
+        double *to = npm + 4 * p + k;
+        auto weigh = [&](int q, int64_t at) {
+            to[q] = div_known(sol[at] * (1.0 - div_known(to[q], D[k], yD[k])), n1[k], yn1[k]);
+        };
+        weigh(0, n_sides + e);
+        for (int s = 0, q = 0; s <= dim; ++s)
+            if (side_has(dim, s, kv)) weigh(++q, n_sides + n_el + d.side_edge[s0 + s]);
+    }
+    __syncthreads();
+    if (t < nn) {
+        const int a = start[t] - first, b = start[t + 1] - first;
+        double s = 0.0;
+        for (int p = a; p < b; ++p) s += npm[4 * p + t];
+        for (int p = a; p < b; ++p) s = add_sides(s, npm + 4 * p + t, terms[p] & 15);
+        out[v0 + t] = s;
+    }
 }
 
 // ---- water balance (water_balance, darcy_flow_mh_output.cc:671-790) ----------------------------
@@ -233,9 +353,10 @@ __global__ void k_balance_regions(const int64_t *__restrict__ region_chunk, int3
 
 cudaError_t launch_node_pressure(const ElemData &d, const int32_t *inc_start, const int32_t *inc_el, int64_t n_nodes,
                                  const double *sol, int64_t n_sides, int64_t n_el, double *out, cudaStream_t s) {
-    if (n_nodes > 0)
-        k_node_pressure<<<(unsigned)((n_nodes + 127) / 128), 128, 0, s>>>(d, inc_start, inc_el, n_nodes, sol, n_sides,
-                                                                          n_el, out);
+    if (n_nodes <= 0) return cudaSuccess;
+    static_assert(kNpSmem <= 48 * 1024, "default limit of dynamic shared memory");
+    k_node_pressure<<<(unsigned)((n_nodes + kNpNodes - 1) / kNpNodes), kNpThreads, kNpSmem, s>>>(
+        d, inc_start, inc_el, n_nodes, sol, n_sides, n_el, out);
     return cudaGetLastError();
 }
 
