@@ -778,9 +778,9 @@ __global__ void k_slice_width(int64_t n_slices, int64_t nc, const int32_t *rowle
 // = D in block column k): row block k becomes P, the other rows A_i. - A_ik P (0 for A_ik in block
 // column k).  Every block inverts A_kk itself (32 pivots) and forms P for its columns, so a step
 // needs nothing from another block of the same launch.  flag = 1 on a non-positive or non-finite
-// pivot.  A step costs 6-12 us, most of it the 32 pivots.
+// pivot.
 // Measured (B200): the inverse of 130 rows 360 us by one block with the matrix in shared memory;
-// here 0.05 ms for 130 rows, 0.13 for 477, 0.5 for 1120.
+// here 15 us a step at 477 rows (0.23 ms), 27 at 1120 (0.95 ms).
 // kDenseMax: the limit was 160, what one SM's shared memory held.  An exact solve this high up
 // replaces one to three levels of seven latency-bound kernels each, in every cycle and in the setup,
 // and converges faster: n = 21 (1120 rows) 57 iterations of 145 us -> 40 of 113, n = 64 (847 rows)
@@ -808,6 +808,15 @@ __global__ void k_dense_scatter(MatView A, int n, int np, double *__restrict__ M
     }
 }
 
+// 1 / x to the last bit or so: the hardware's 20-bit approximation and two Newton steps (a quarter of
+// the latency of the full division, which is the pivots' critical path)
+__device__ __forceinline__ double quick_rcp(double x) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    r = fma(r, fma(-x, r, 1.0), r);
+    return fma(r, fma(-x, r, 1.0), r);
+}
+
 __global__ void __launch_bounds__(256) k_gj_step(const double *__restrict__ src, double *__restrict__ dst, int np,
                                                  int k, int32_t *flag) {
     __shared__ double D[kGjB][kGjB + 1], rowb[2][kGjB], colb[2][kGjB];
@@ -825,27 +834,32 @@ __global__ void __launch_bounds__(256) k_gj_step(const double *__restrict__ src,
     double m[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) m[q] = src[(size_t)(kb + r) * np + kb + c4 + q];
+    // pivot p: with a 1 in the pivot's place of row p, zeros left behind in row p and column p, and
+    // the factor -1 for row p, every entry is m -= f / pivot * row_p
     bool bad = false;
 #pragma unroll 1
-    for (int p = 0; p < kGjB; ++p) {
-        double *rb = rowb[p & 1], *cb = colb[p & 1];
-        if (r == p)
+    for (int p0 = 0; p0 < kGjB; p0 += 4) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) rb[c4 + q] = m[q];
-        if ((p & ~3) == c4)
+        for (int u = 0; u < 4; ++u) {
+            const int p = p0 + u;
+            double *rb = rowb[u & 1], *cb = colb[u & 1];
+            if (c4 == p0) {
+                cb[r] = m[u];
+                m[u] = r == p ? 1.0 : 0.0;
+            }
+            if (r == p) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (c4 + q == p) cb[r] = m[q];
-        __syncthreads();
-        const double piv = rb[p];
-        const bool ok = piv > 0.0 && isfinite(piv);
-        bad |= !ok;
-        const double pinv = ok ? 1.0 / piv : 0.0, f = cb[r];
+                for (int q = 0; q < 4; ++q) {
+                    rb[c4 + q] = m[q];
+                    m[q] = 0.0;
+                }
+            }
+            __syncthreads();
+            const double piv = cb[p];
+            bad |= !(piv > 0.0 && piv < 1e300);
+            const double g = (r == p ? -1.0 : cb[r]) * quick_rcp(piv);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const bool jp = c4 + q == p;
-            const double a = (jp ? 1.0 : rb[c4 + q]) * pinv;
-            m[q] = r == p ? a : (jp ? 0.0 : m[q]) - f * a;
+            for (int q = 0; q < 4; ++q) m[q] = fma(-g, rb[c4 + q], m[q]);
         }
     }
     if (bad && t == 0) *flag = 1;
