@@ -787,6 +787,7 @@ __global__ void k_slice_width(int64_t n_slices, int64_t nc, const int32_t *rowle
 // 104 of 591 -> 73 of 545, 24 uneven systems (437 rows) 43.7 -> 34.5 ms.  At 1280 rows the inverse
 // is 6.5 MB, 3.5 us a pass from L2; at 2048 its setup (n^3) would cost more than the levels it saves.
 constexpr int kDenseMax = 1280;
+constexpr int kHostWords = 256;  // pinned words of Amg's read-backs
 constexpr int kCoarseMin = 160;  // pairing passes go on down to this many rows
 constexpr int kGjB = 32, kGjTile = 64;
 
@@ -1168,9 +1169,9 @@ __global__ void k_flag_long(int64_t n, const int32_t *rlen, int32_t *flag) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) flag[i] = rlen[i] > kLongRow ? 1 : 0;
 }
-__global__ void k_compact_long(int64_t n, const int32_t *flag, const int32_t *pos, int32_t *list) {
+__global__ void k_compact_long(int64_t n, const int32_t *flag, const int32_t *pos, int32_t *list, int32_t *count) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) list[0] = pos[n];
+    if (i == 0) list[0] = *count = pos[n];
     if (i < n && flag[i]) list[1 + pos[i]] = (int32_t)i;
 }
 
@@ -2191,17 +2192,17 @@ cudaError_t Amg::scan_i64_dev(const int64_t *in, int64_t *out, int64_t n, cudaSt
 
 cudaError_t Amg::scan_i32(const int32_t *in, int32_t *out, int64_t n, int64_t &total, cudaStream_t s) {
     AMG_CK(launch_scan<int32_t>(in, out, n, scan32_blk_, s));
-    int32_t t = 0;
-    AMG_CK(cudaMemcpyAsync(&t, out + n, sizeof(t), cudaMemcpyDeviceToHost, s));
+    AMG_CK(cudaMemcpyAsync(h_flag_, out + n, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
     AMG_CK(cudaStreamSynchronize(s));
-    total = t;
+    total = *h_flag_;
     return cudaSuccess;
 }
 
 cudaError_t Amg::scan_i64(const int64_t *in, int64_t *out, int64_t n, int64_t &total, cudaStream_t s) {
     AMG_CK(launch_scan<int64_t>(in, out, n, scan64_blk_, s));
-    AMG_CK(cudaMemcpyAsync(&total, out + n, sizeof(total), cudaMemcpyDeviceToHost, s));
+    AMG_CK(cudaMemcpyAsync(h_flag_, out + n, sizeof(total), cudaMemcpyDeviceToHost, s));
     AMG_CK(cudaStreamSynchronize(s));
+    std::memcpy(&total, h_flag_, sizeof(total));
     return cudaSuccess;
 }
 
@@ -2342,7 +2343,7 @@ cudaError_t Amg::pair_pass(const AmgMatrix &A, const float *isd, const int32_t *
 cudaError_t Amg::galerkin(const AmgMatrix &A, const int32_t *agg, int64_t nc, const int32_t *mstart,
                           const int32_t *mrows, DBuf<int64_t> &c_off, DBuf<int32_t> &c_col, DBuf<float> &c_val,
                           DBuf<int32_t> &c_rlen, DBuf<int32_t> &c_long, AmgMatrix &C, cudaStream_t s,
-                          const float *wt) {
+                          const float *wt, int level) {
     const int64_t n_pad = round_up(nc, kS), n_sl = n_pad / kS;
     AMG_CK(rowlen_.ensure(n_pad));
     AMG_CK(cudaMemsetAsync(rowlen_.p, 0, n_pad * sizeof(int32_t), s));  // padding rows: no entries
@@ -2371,11 +2372,11 @@ cudaError_t Amg::galerkin(const AmgMatrix &A, const int32_t *agg, int64_t nc, co
     AMG_CK(cudaFuncSetAttribute(k_galerkin<kGalCapBig, kGalWarpsBig, true>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)big_smem));
     k_galerkin<kGalCap0, kGalWarps0, false><<<g0, kGalWarps0 * 32, 0, s>>>(
-        V, agg, mstart, mrows, nc, rowlen_.p, toff_.p, tcol_.p, tval_.p, flag_.p, wt, big_list_.p, big_count_.p);
+        V, agg, mstart, mrows, nc, rowlen_.p, toff_.p, tcol_.p, tval_.p, overflow_, wt, big_list_.p, big_count_.p);
     // the list pass reads its row count on the device (usually none: the blocks return at once);
     // an overflow there is reported at the end of the setup
     k_galerkin<kGalCapBig, kGalWarpsBig, true><<<148 * 2, kGalWarpsBig * 32, big_smem, s>>>(
-        V, agg, mstart, mrows, nc, rowlen_.p, toff_.p, tcol_.p, tval_.p, flag_.p, wt, big_list_.p, big_count_.p);
+        V, agg, mstart, mrows, nc, rowlen_.p, toff_.p, tcol_.p, tval_.p, overflow_, wt, big_list_.p, big_count_.p);
     AMG_CK(cudaGetLastError());
     k_slice_width<<<nblk(n_sl, 256), 256, 0, s>>>(n_sl, nc, rowlen_.p, width_.p);
     AMG_CK(cudaGetLastError());
@@ -2405,7 +2406,7 @@ cudaError_t Amg::galerkin(const AmgMatrix &A, const int32_t *agg, int64_t nc, co
     // the list holds its count in front: [count, rows...]; the host reads the counts of all
     // levels at the end of the setup
     AMG_CK(c_long.ensure(n_pad + 1));
-    k_compact_long<<<nblk(n_pad, 256), 256, 0, s>>>(n_pad, lflag_.p, lpos_.p, c_long.p);
+    k_compact_long<<<nblk(n_pad, 256), 256, 0, s>>>(n_pad, lflag_.p, lpos_.p, c_long.p, long_words_ + level);
     AMG_CK(cudaGetLastError());
     C.longrows = c_long.p + 1;
     C.long_count = c_long.p;
@@ -2413,42 +2414,41 @@ cudaError_t Amg::galerkin(const AmgMatrix &A, const int32_t *agg, int64_t nc, co
     return cudaSuccess;
 }
 
-// ok: the matrix was positive definite and its inverse is in place
-cudaError_t Amg::dense_coarse(const AmgMatrix &A, bool &ok, cudaStream_t s) {
+// *dense_flag_ != 0 afterwards: the matrix was not positive definite
+cudaError_t Amg::dense_coarse(const AmgMatrix &A, cudaStream_t s) {
     const int n = (int)dense_n_, np = (int)round_up(n, kGjB);
     const int64_t ld = dense_ld(n);
     AMG_CK(dense_inv_.ensure((size_t)n * ld));
     for (auto &w : dense_work_) AMG_CK(w.ensure((size_t)np * np));
-    AMG_CK(flag_.ensure(1));
-    AMG_CK(cudaMemsetAsync(flag_.p, 0, sizeof(int32_t), s));
     AMG_CK(cudaMemsetAsync(dense_work_[0].p, 0, (size_t)np * np * sizeof(double), s));
     k_dense_scatter<<<nblk(np, 128), 128, 0, s>>>(view(A), n, np, dense_work_[0].p);
     const unsigned tiles = nblk(np, kGjTile);
     int from = 0;
     for (int k = 0; k < np / kGjB; ++k, from ^= 1)
-        k_gj_step<<<dim3(tiles, tiles), 256, 0, s>>>(dense_work_[from].p, dense_work_[from ^ 1].p, np, k, flag_.p);
+        k_gj_step<<<dim3(tiles, tiles), 256, 0, s>>>(dense_work_[from].p, dense_work_[from ^ 1].p, np, k, dense_flag_);
     k_dense_store<<<nblk(n * ld, 256), 256, 0, s>>>(n, np, (int)ld, dense_work_[from].p, dense_inv_.p);
     AMG_CK(cudaGetLastError());
-    AMG_CK(cudaMemcpyAsync(h_flag_, flag_.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    AMG_CK(cudaStreamSynchronize(s));
-    ok = *h_flag_ == 0;
     return cudaSuccess;
 }
 
 cudaError_t Amg::setup(const DevSystem &sys, const AmgOptions &o, cudaStream_t s) {
     opt_ = o;
-    if (!h_flag_) AMG_CK(cudaHostAlloc((void **)&h_flag_, sizeof(int32_t), cudaHostAllocDefault));
+    if (!h_flag_) AMG_CK(cudaHostAlloc((void **)&h_flag_, kHostWords * sizeof(int32_t), cudaHostAllocDefault));
     if (sms_ == 0) {
         int dev = 0;
         AMG_CK(cudaGetDevice(&dev));
         AMG_CK(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
     }
-    // device words the setup fills and the host reads once at its end: the Gershgorin bound of
-    // each level, and the Galerkin overflow flag
-    AMG_CK(bounds_.ensure(o.max_levels + 1));
-    AMG_CK(cudaMemsetAsync(bounds_.p, 0, (o.max_levels + 1) * sizeof(unsigned int), s));
-    AMG_CK(flag_.ensure(1));
-    AMG_CK(cudaMemsetAsync(flag_.p, 0, sizeof(int32_t), s));
+    // device words the setup fills and the host reads at its end in one copy: the Gershgorin bound of
+    // each level (and a spare one), the count of long rows of each level, the Galerkin overflow
+    // flag and the dense inverse's flag
+    const int words = 2 * (o.max_levels + 1) + 2;
+    if (words > kHostWords) return cudaErrorInvalidValue;
+    AMG_CK(bounds_.ensure(words));
+    AMG_CK(cudaMemsetAsync(bounds_.p, 0, words * sizeof(unsigned int), s));
+    long_words_ = reinterpret_cast<int32_t *>(bounds_.p) + o.max_levels + 1;
+    overflow_ = long_words_ + o.max_levels + 1;
+    dense_flag_ = overflow_ + 1;
     if ((int)lv_.size() < o.max_levels) lv_.resize(o.max_levels);
     n_levels_ = 0;
     // level 0: the solver's FP32 scaled matrix
@@ -2516,7 +2516,7 @@ cudaError_t Amg::setup(const DevSystem &sys, const AmgOptions &o, cudaStream_t s
             AmgMatrix M;
             const int slot = p & 1;
             if ((e = galerkin(cur, cagg, nc, cms, cmr, mid_off_[slot], mid_col_[slot], mid_val_[slot], mid_rlen_[slot],
-                              mid_long_[slot], M, s, curw)) != cudaSuccess)
+                              mid_long_[slot], M, s, curw, l + 1)) != cudaSuccess)
                 return e;
             AMG_CK(isd_.ensure(M.n));
             AMG_CK(mid_invd_.ensure(M.n));
@@ -2551,7 +2551,8 @@ cudaError_t Amg::setup(const DevSystem &sys, const AmgOptions &o, cudaStream_t s
             nc = np;
         }
         // the coarse matrix from the last pass's pairs
-        if ((e = galerkin(cur, cagg, nc, cms, cmr, C.slice_off, C.col, C.val, C.rlen, C.longrows, C.A, s, curw)) !=
+        if ((e = galerkin(cur, cagg, nc, cms, cmr, C.slice_off, C.col, C.val, C.rlen, C.longrows, C.A, s, curw,
+                          l + 1)) !=
             cudaSuccess)
             return e;
         L.nc = nc;
@@ -2573,24 +2574,32 @@ cudaError_t Amg::setup(const DevSystem &sys, const AmgOptions &o, cudaStream_t s
         if (e2 != cudaSuccess || (e2 = fine_interval(s)) != cudaSuccess) return e2;
         // the bounds, the long-row counts and the overflow flag first: the power iteration's
         // row kernels need each level's split and long rows
+        const AmgLevel &Lc = lv_[n_levels_ - 1];
+        dense_n_ = !dense_planned() ? 0 : n_levels_ == 1 ? Lc.A.n : lv_[n_levels_ - 2].nc;
+        if (dense_n_ > 0 && (e2 = dense_coarse(Lc.A, s)) != cudaSuccess) return e2;
         std::vector<unsigned int> bits(n_levels_);
         std::vector<int32_t> nlong(n_levels_, 0);
         std::vector<double> pw(2 * n_levels_, 0.0);
-        AMG_CK(cudaMemcpyAsync(bits.data(), bounds_.p, n_levels_ * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
-        if (fine_w_)  // the fine level is smoothed on Omega S^: its own bound
-            AMG_CK(cudaMemcpyAsync(bits.data(), bounds_.p + opt_.max_levels, sizeof(unsigned int),
-                                   cudaMemcpyDeviceToHost, s));
-        for (int l = 1; l < n_levels_; ++l)
-            if (lv_[l].A.long_count)
-                AMG_CK(cudaMemcpyAsync(&nlong[l], lv_[l].A.long_count, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-        AMG_CK(cudaMemcpyAsync(h_flag_, flag_.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
         unsigned int widest = 0;
+        AMG_CK(cudaMemcpyAsync(h_flag_, bounds_.p, words * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
         if (opt_.fine_tma && opt_.half_fine && fine_tiles > 0)
             AMG_CK(cudaMemcpyAsync(&widest, tile_max_.p, sizeof(widest), cudaMemcpyDeviceToHost, s));
         AMG_CK(cudaStreamSynchronize(s));
-        if (*h_flag_) {
+        std::memcpy(bits.data(), h_flag_, n_levels_ * sizeof(unsigned int));
+        if (fine_w_) bits[0] = (unsigned int)h_flag_[opt_.max_levels];  // smoothed on Omega S^: its own bound
+        for (int l = 1; l < n_levels_; ++l) nlong[l] = h_flag_[o.max_levels + 1 + l];
+        if (h_flag_[words - 2]) {
             err = "Galerkin row wider than the gather buffer";
             return cudaErrorInvalidValue;
+        }
+        if (h_flag_[words - 1]) {
+            if (dense_n_ <= kCoarseMin) {
+                err = "coarsest matrix is not positive definite";
+                return cudaErrorInvalidValue;
+            }
+            // (a larger matrix can lose definiteness to its FP32 rounding: smoothed instead, on its
+            // Gershgorin interval)
+            dense_n_ = 0;
         }
         if (widest > 0) AMG_CK(prepare_fine_tma(widest, s));
         for (int l = 0; l < n_levels_; ++l) {
@@ -2604,8 +2613,9 @@ cudaError_t Amg::setup(const DevSystem &sys, const AmgOptions &o, cudaStream_t s
         }
         if ((e2 = power_estimates(s)) != cudaSuccess) return e2;
         if (opt_.power_steps > 0) {
-            AMG_CK(cudaMemcpyAsync(pw.data(), pw_sums_.p, 2 * n_levels_ * sizeof(double), cudaMemcpyDeviceToHost, s));
+            AMG_CK(cudaMemcpyAsync(h_flag_, pw_sums_.p, 2 * n_levels_ * sizeof(double), cudaMemcpyDeviceToHost, s));
             AMG_CK(cudaStreamSynchronize(s));
+            std::memcpy(pw.data(), h_flag_, 2 * n_levels_ * sizeof(double));
         }
         for (int l = 0; l < n_levels_; ++l) {
             float hi;
@@ -2618,19 +2628,6 @@ cudaError_t Amg::setup(const DevSystem &sys, const AmgOptions &o, cudaStream_t s
                 lv_[l].hi = (float)std::min((double)lv_[l].gershgorin, opt_.power_safety * est);
             }
         }
-    }
-    const AmgLevel &Lc = lv_[n_levels_ - 1];
-    dense_n_ = n_levels_ == 1 ? Lc.A.n : lv_[n_levels_ - 2].nc;
-    if (!dense_planned()) dense_n_ = 0;
-    if (dense_n_ > 0) {
-        bool ok = false;
-        if ((e = dense_coarse(Lc.A, ok, s)) != cudaSuccess) return e;
-        if (!ok && dense_n_ <= kCoarseMin) {
-            err = "coarsest matrix is not positive definite";
-            return cudaErrorInvalidValue;
-        }
-        // (a larger matrix can lose definiteness to its FP32 rounding: smoothed instead)
-        if (!ok) dense_n_ = 0;
     }
     if (dense_n_ == 0) {  // too large for the dense inverse: a polynomial on the level instead
         AmgLevel &Lm = lv_[n_levels_ - 1];

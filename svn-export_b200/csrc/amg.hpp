@@ -160,9 +160,9 @@ private:
     cudaError_t galerkin(const AmgMatrix &A, const int32_t *agg, int64_t nc, const int32_t *mstart,
                          const int32_t *mrows, DBuf<int64_t> &c_off, DBuf<int32_t> &c_col, DBuf<float> &c_val,
                          DBuf<int32_t> &c_rlen, DBuf<int32_t> &c_long, AmgMatrix &C, cudaStream_t s,
-                         const float *wt);
+                         const float *wt, int level);
     cudaError_t level_stats(AmgLevel &L, unsigned int *bound, cudaStream_t s);
-    cudaError_t dense_coarse(const AmgMatrix &A, bool &ok, cudaStream_t s);
+    cudaError_t dense_coarse(const AmgMatrix &A, cudaStream_t s);
     bool dense_planned() const;
     // lambda_max estimates of D^-1 A on every level but the coarsest (power iteration from a
     // fixed pseudo-random start; deterministic sums), as |v_k|^2 and |v_{k-1}|^2 per level
@@ -183,7 +183,8 @@ private:
     // pairing and Galerkin scratch
     DBuf<int32_t> mate_, want_, cid_, tmp_agg_, tmp_ms_, tmp_mr_, cnt_;
     DBuf<int64_t> packed_, pscan_;  // pairing: packed (leader, member count) and its scan
-    DBuf<unsigned int> bounds_;     // Gershgorin bound of each level (float bits)
+    DBuf<unsigned int> bounds_;     // the setup's result words: Gershgorin bound of each level (float bits), ...
+    int32_t *long_words_ = nullptr, *overflow_ = nullptr, *dense_flag_ = nullptr;  // ... and these (setup)
     DBuf<int64_t> width_, scan64_;
     DBuf<int32_t> rowlen_, scan32_blk_;
     DBuf<int64_t> scan64_blk_;

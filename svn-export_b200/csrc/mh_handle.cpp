@@ -73,8 +73,8 @@ struct mh_handle {
     double *d_aniso = nullptr;
     bool coeffs_set = false, bc_set = false, assembled = false, solved = false;
     bool general = false;               // a general SPD system given in CSR form (no mesh)
-    std::vector<double> gen_slot_val;   // its values in SELL slot order (host staging)
-    std::vector<double> gen_rhs;
+    double *d_csr_val = nullptr;        // its values in the caller's order, and their SELL slots
+    int32_t *d_csr_slot = nullptr;
     bool rhs_stale = false;             // boundary values changed since the last assembly
     int time_mode = 0;
     double dt = 0.0;
@@ -97,6 +97,7 @@ struct mh_handle {
     bool loop_unavailable = false;  // the device-side loop could not be built: poll from the host
     std::vector<cudaEvent_t> prof_ev[2];
     int32_t *h_done = nullptr;
+    void *h_small = nullptr;            // pinned staging of small read-backs (read_back)
     cudaEvent_t ev[8] = {};
     float ms_assembly = 0.f;
     int64_t n_launch = 0;               // kernels launched so far
@@ -155,6 +156,17 @@ using mh::HostSystem;
         }                                                                               \
     } while (0)
 
+// A read-back that the caller waits for.  Small ones go through pinned memory: a copy into
+// pageable memory is staged by the driver and holds the caller several microseconds longer.
+constexpr size_t kSmallBytes = 64 * 1024;
+int read_back(mh_handle *h, void *dst, const void *src, size_t bytes) {
+    const bool small = bytes <= kSmallBytes && h->h_small;
+    CK(cudaMemcpyAsync(small ? h->h_small : dst, src, bytes, cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    if (small) std::memcpy(dst, h->h_small, bytes);
+    return MH_OK;
+}
+
 template <class T> T *dalloc(mh_handle *h, size_t n) {
     void *p = nullptr;
     if (n == 0) n = 1;
@@ -200,6 +212,7 @@ int device_setup(mh_handle *h) {
     h->stream = h->own_stream;
     for (auto &e : h->ev) CK(cudaEventCreate(&e));
     CK(cudaHostAlloc((void **)&h->h_done, sizeof(int32_t) * 4, cudaHostAllocDefault));
+    CK(cudaHostAlloc(&h->h_small, kSmallBytes, cudaHostAllocDefault));
     const mh::MeshData &m = h->mesh;
     const mh::Topology &t = h->topo;
     const HostSystem &hs = h->hs;
@@ -318,6 +331,18 @@ int device_setup(mh_handle *h) {
     CK(cudaMemset(s.x32, 0, nr * sizeof(float)));
     CK(cudaMemset(s.sum_ticket, 0, s.n_inst * sizeof(uint32_t)));
     CK(cudaMemset(s.inst_sums, 0, mh::kSumStride * s.n_inst * sizeof(double)));
+    if (h->general) {
+        // the slots outside the caller's pattern hold a unit diagonal (padding rows) or 0 for good
+        if ((rc = upload(h, h->d_csr_slot, hs.csr_slot))) return rc;
+        h->d_csr_val = dalloc<double>(h, hs.nnz);
+        if (!h->d_csr_val) return MH_ERR_NOMEM;
+        CK(cudaMemset(s.val_raw, 0, hs.n_slots * sizeof(double)));
+        CK(cudaMemset(s.b, 0, nr * sizeof(double)));
+        std::vector<double> one(nr - t.n_edges(), 1.0);
+        std::vector<int32_t> at(hs.diag_slot.begin() + t.n_edges(), hs.diag_slot.end());
+        for (size_t k = 0; k < at.size(); ++k)  // fewer than kPadRows
+            CK(cudaMemcpy(s.val_raw + at[k], &one[k], sizeof(double), cudaMemcpyHostToDevice));
+    }
     const int64_t msize = t.n_sides() + m.n_el + t.n_edges();
     h->sol = dalloc<double>(h, msize);
     h->sol_prev = dalloc<double>(h, msize);
@@ -402,6 +427,12 @@ __global__ void k_fill(double *dst, int64_t n, double v) {
     if (i < n) dst[i] = v;
 }
 
+__global__ void k_scatter(int64_t n, const int32_t *__restrict__ to, const double *__restrict__ v,
+                          double *__restrict__ dst) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) dst[to[i]] = v[i];
+}
+
 // a field from the caller's host array, or its default value filled on the device
 int fill_or_default(mh_handle *h, double *dst, const double *src, int64_t n, double dflt) {
     if (n <= 0) return MH_OK;
@@ -427,8 +458,7 @@ int assemble_impl(mh_handle *h, int mode) {
     for (int d = 1; d <= 3; ++d) h->n_launch += h->as.dim_count[d] > 0;
     h->n_launch += 1 + ((mode & 1) ? 3 : 1);
     int32_t st = 0;
-    CK(cudaMemcpyAsync(&st, h->as.status, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
+    if (int rc = read_back(h, &st, h->as.status, sizeof(st))) return rc;
     CK(cudaEventElapsedTime(&h->ms_assembly, h->ev[0], h->ev[1]));
     if (st & 1) {
         h->err = "singular local MH matrix (|det| < DBL_MIN/DBL_EPSILON)";
@@ -448,9 +478,7 @@ int assemble_impl(mh_handle *h, int mode) {
 
 int read_ctl(mh_handle *h, std::vector<mh::InstCtl> &ctl) {
     ctl.resize(h->sys.n_inst);
-    CK(cudaMemcpyAsync(ctl.data(), h->sys.ctl, sizeof(mh::InstCtl) * ctl.size(), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    return MH_OK;
+    return read_back(h, ctl.data(), h->sys.ctl, sizeof(mh::InstCtl) * ctl.size());
 }
 
 // Captures `ipg` CG iterations (two kernels each) into a graph on the handle's own stream;
@@ -686,10 +714,7 @@ int true_residual(mh_handle *h, std::vector<double> &sums) {
     CK(mh::launch_residual64(h->sys, h->stream));
     h->n_launch += 1;
     sums.resize(mh::kSumStride * (size_t)h->sys.n_inst);
-    CK(cudaMemcpyAsync(sums.data(), h->sys.inst_sums, sizeof(double) * sums.size(), cudaMemcpyDeviceToHost,
-                       h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    return MH_OK;
+    return read_back(h, sums.data(), h->sys.inst_sums, sizeof(double) * sums.size());
 }
 
 struct SolveResult {
@@ -916,8 +941,7 @@ int nn_weights(mh_handle *h) {
 int spectrum_bound(mh_handle *h, double &hi) {
     CK(mh::launch_spectrum_bound(h->sys, h->spec_bound, h->stream));
     unsigned int bits = 0;
-    CK(cudaMemcpyAsync(&bits, h->spec_bound, sizeof(bits), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
+    if (int rc = read_back(h, &bits, h->spec_bound, sizeof(bits))) return rc;
     float f;
     std::memcpy(&f, &bits, sizeof(f));
     hi = f > 0.f ? (double)f : 2.0;
@@ -1192,9 +1216,7 @@ int solve_fcg(mh_handle *h, const mh_solve_opts &o, SolveResult &res, Pc kind) {
         const int t[2] = {mh::krylov_target_blocks(1, 64), mh::krylov_target_blocks(1, 32)};
         if ((rc = apply_launch_shape(h, 1, t))) return rc;
     }
-    double hi = 2.0;
-    if ((rc = spectrum_bound(h, hi))) return rc;
-    const double lo = hi / 30.0;
+    double hi = 0.0;  // spectrum bound of the Chebyshev-Jacobi polynomial, once that is used
     const int degree = std::max(1, std::min(o.cheb_degree, 16));
     if (kind == Pc::Amg || kind == Pc::Nn) {
         if ((rc = prepare_multigrid(h, kind, res.ms_setup))) {
@@ -1254,7 +1276,8 @@ int solve_fcg(mh_handle *h, const mh_solve_opts &o, SolveResult &res, Pc kind) {
             CK(mh::launch_ir_continue(h->sys, o.inner_rtol * o.inner_rtol, seg_max, h->stream));
         restart = false;
         const Pc cur = learned ? (use_nn ? Pc::Nn : Pc::Cheb) : kind;
-        if ((rc = run_fcg(h, cur, degree, lo, hi, o.iters_per_graph, seg_max, o.profile_kernels != 0))) return rc;
+        if (cur == Pc::Cheb && hi == 0.0 && (rc = spectrum_bound(h, hi))) return rc;
+        if ((rc = run_fcg(h, cur, degree, hi / 30.0, hi, o.iters_per_graph, seg_max, o.profile_kernels != 0))) return rc;
         CK(mh::launch_ir_correct(h->sys, h->stream));
         h->n_launch += 2;
         if ((rc = read_ctl(h, ctl))) return rc;
@@ -1882,25 +1905,22 @@ int mh_csr_set_values(mh_handle *h, const double *val, const double *rhs) {
         h->err = "non-finite matrix or right-hand side value";
         return MH_ERR_NONFINITE;
     }
-    h->gen_slot_val.assign(hs.n_slots, 0.0);
-    for (int64_t k = 0; k < nnz; ++k) h->gen_slot_val[hs.csr_slot[k]] = val[k];
-    for (int64_t r = 0; r < hs.n_rows; ++r) {
-        const double d = r < n ? h->gen_slot_val[hs.diag_slot[r]] : 1.0;
-        if (!(d > 0.0)) {
-            h->err = "row " + std::to_string(r) + " has a diagonal entry <= 0: not a positive definite system";
-            return MH_ERR_INVALID;
-        }
-        if (r >= n) h->gen_slot_val[hs.diag_slot[r]] = 1.0;  // padding rows: unit diagonal
+    int64_t bad = n;  // the first row whose diagonal is not positive
+#pragma omp parallel for schedule(static) reduction(min : bad) if (n > (1 << 16))
+    for (int64_t r = 0; r < n; ++r)
+        if (!(val[hs.csr_diag[r]] > 0.0)) bad = std::min(bad, r);
+    if (bad < n) {
+        h->err = "row " + std::to_string(bad) + " has a diagonal entry <= 0: not a positive definite system";
+        return MH_ERR_INVALID;
     }
-    h->gen_rhs.assign(hs.n_rows, 0.0);
-    std::copy(rhs, rhs + n, h->gen_rhs.begin());
     int rc = need_device(h);
     if (rc) return rc;
-    CK(cudaMemcpyAsync(h->sys.val_raw, h->gen_slot_val.data(), hs.n_slots * sizeof(double), cudaMemcpyHostToDevice,
-                       h->stream));
-    CK(cudaMemcpyAsync(h->sys.b, h->gen_rhs.data(), hs.n_rows * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemcpyAsync(h->d_csr_val, val, nnz * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemcpyAsync(h->sys.b, rhs, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    k_scatter<<<(unsigned)((nnz + 255) / 256), 256, 0, h->stream>>>(nnz, h->d_csr_slot, h->d_csr_val, h->sys.val_raw);
+    CK(cudaGetLastError());
     CK(mh::launch_scale(h->sys, 1, h->stream));
-    h->n_launch += 3;
+    h->n_launch += 4;
     CK(cudaStreamSynchronize(h->stream));
     h->assembled = true;
     h->rhs_stale = false;
@@ -1944,6 +1964,7 @@ void mh_destroy(mh_handle *h) {
     for (auto &e : h->ev)
         if (e) cudaEventDestroy(e);
     if (h->h_done) cudaFreeHost(h->h_done);
+    if (h->h_small) cudaFreeHost(h->h_small);
     if (h->own_stream) cudaStreamDestroy(h->own_stream);
     delete h;
 }
@@ -2365,8 +2386,7 @@ static int transport_values(mh_handle *h, const double *dev_porosity, double *de
     }
     CK(mh::launch_transport_matrix(h->ed, h->conv, dev_porosity, h->sol, dev_val, h->stream));
     unsigned long long bits = 0;
-    CK(cudaMemcpyAsync(&bits, h->conv.diag_max, sizeof(bits), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
+    if (int rc = read_back(h, &bits, h->conv.diag_max, sizeof(bits))) return rc;
     if (cfl) {
         double mx;
         std::memcpy(&mx, &bits, sizeof(mx));
@@ -2447,21 +2467,23 @@ int mh_unsteady_init(mh_handle *h, int32_t lumped, double dt, const double *init
     if (!h->coeffs_set || !h->bc_set) return MH_ERR_STATE;
     const int64_t n_el = h->mesh.n_el, ns = h->topo.n_sides(), ne = h->topo.n_edges();
     if (init_pressure && !check_finite(init_pressure, n_el)) return MH_ERR_NONFINITE;
-    std::vector<double> s0(ns + n_el + ne, 0.0);
-    if (init_pressure) {
-        if (!lumped) {
-            for (int64_t e = 0; e < n_el; ++e) s0[ns + e] = init_pressure[e];
-        } else {
-            // DarcyFlowLMH_Unsteady::setup_time_term: edge value += init / n_sides per side
-            for (int64_t e = 0; e < n_el; ++e) {
-                const int n = h->mesh.dim[e] + 1;
-                for (int i = 0; i < n; ++i)
-                    s0[ns + n_el + h->topo.side_edge[h->topo.el_side_start[e] + i]] += init_pressure[e] / n;
-            }
+    // the previous step's solution: zero but for the initial element pressures (MH) or the edge
+    // pressures they give (LMH)
+    const size_t bytes = (size_t)(ns + n_el + ne) * sizeof(double);
+    CK(cudaMemsetAsync(h->sol_prev, 0, bytes, h->stream));
+    std::vector<double> edge;
+    if (init_pressure && !lumped) {
+        CK(cudaMemcpyAsync(h->sol_prev + ns, init_pressure, n_el * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    } else if (init_pressure) {
+        // DarcyFlowLMH_Unsteady::setup_time_term: edge value += init / n_sides per side
+        edge.assign(ne, 0.0);
+        for (int64_t e = 0; e < n_el; ++e) {
+            const int n = h->mesh.dim[e] + 1;
+            for (int i = 0; i < n; ++i) edge[h->topo.side_edge[h->topo.el_side_start[e] + i]] += init_pressure[e] / n;
         }
+        CK(cudaMemcpyAsync(h->sol_prev + ns + n_el, edge.data(), ne * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     }
-    CK(cudaMemcpyAsync(h->sol_prev, s0.data(), s0.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->sol, s0.data(), s0.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemcpyAsync(h->sol, h->sol_prev, bytes, cudaMemcpyDeviceToDevice, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     h->time_mode = lumped ? 2 : 1;
     h->ed.time_mode = h->time_mode;

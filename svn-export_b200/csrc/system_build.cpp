@@ -409,6 +409,7 @@ int build_host_system_csr(int64_t n, const int32_t *row_ptr, const int32_t *col,
     hs.sell_col.resize(hs.n_slots);
     hs.diag_slot.resize(pad);
     hs.csr_slot.resize(hs.nnz);
+    hs.csr_diag.resize(n);
     for (int64_t r = 0; r < pad; ++r) {
         const int64_t sl = r / kSliceRowsHost, lane = r % kSliceRowsHost;
         const int64_t off = hs.slice_off[sl], w = (hs.slice_off[sl + 1] - off) / kSliceRowsHost;
@@ -418,6 +419,7 @@ int build_host_system_csr(int64_t n, const int32_t *row_ptr, const int32_t *col,
             const int64_t slot = off + (j < len ? sell_pos(r, c, j) : j) * kSliceRowsHost + lane;
             hs.sell_col[slot] = c;
             if (j < len && r < n) hs.csr_slot[hs.row_ptr[r] + j] = (int32_t)slot;
+            if (j < len && r < n && c == r) hs.csr_diag[r] = (int32_t)(hs.row_ptr[r] + j);
         }
         hs.diag_slot[r] = (int32_t)(off + lane);
     }

@@ -43,6 +43,7 @@ struct HostSystem {
     std::vector<int32_t> row_cstart, row_cidx;
     std::vector<int32_t> dim_list[4];
     std::vector<int32_t> csr_slot;       // general systems: SELL slot of every CSR entry
+    std::vector<int32_t> csr_diag;       // ... and the CSR entry of every row's diagonal
     // constant additions to the edge system (mortar coupling): slots and summed values
     std::vector<int32_t> add_slot;
     std::vector<double> add_val;
