@@ -14,8 +14,14 @@ namespace mh {
 // with 148; 22k edges: 2.84 with 88 blocks (256 rows), 3.00 with 48, 3.14 with 148.
 constexpr int64_t kResidentRows = 256;
 
+// Systems of at most this many rows run in one thread-block cluster: 2.70 us an iteration against
+// 2.97 on 49 blocks with 13k rows, 3.43 against 2.79 (FP32 4.01 against 3.36) with 22k.
+constexpr int64_t kClusterRows = 14336;
+
 struct ResidentPlan {
     int prec = 64;
+    bool cluster = false;             // one cluster of n_blocks blocks instead of a cooperative launch
+    int32_t rows_cap = 0;             // rows of the largest block
     int n_blocks = 0, threads = 0;
     int kr = 1;                       // rows per thread
     size_t smem = 0;                  // dynamic shared memory of the largest block
