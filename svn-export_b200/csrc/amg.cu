@@ -9,6 +9,7 @@
 #include <cuda_fp16.h>
 
 #include "amg.hpp"
+#include "pdl.hpp"
 
 namespace cg = cooperative_groups;
 
@@ -937,22 +938,30 @@ __host__ __device__ inline int64_t dense_ld(int64_t n) { return (n + 3) / 4 * 4;
 // x[i] = sum_j inv[i][j] b[j] for i < n (one warp per row, four entries to a load); rows
 // n..n_pad-1 get 0.  b has n_pad >= ld entries.
 __global__ void __launch_bounds__(256) k_dense_gemv(Gate gate, const float *__restrict__ inv, int64_t n, int64_t ld,
-                                                    int64_t n_pad, const float *__restrict__ b, float *__restrict__ x) {
-    if (closed(gate)) return;
+                                                    int64_t n_pad, const float *b, float *x) {
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
-    if (i >= n_pad) return;
+    const int nq = i < n ? (int)(ld / 4) : 0;
+    const float4 *row = reinterpret_cast<const float4 *>(inv + (i < n ? i : 0) * ld);
+    const float4 *b4 = reinterpret_cast<const float4 *>(b);
+    constexpr int kA = 5;  // loads of a lane ahead
+    float4 a[kA], v[kA];
+#pragma unroll
+    for (int k = 0; k < kA; ++k) a[k] = lane + 32 * k < nq ? __ldg(row + lane + 32 * k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    pdl_wait();
+    if (closed(gate) || i >= n_pad) return;
     float s = 0.f;
-    if (i < n) {
-        const float4 *row = reinterpret_cast<const float4 *>(inv + i * ld);
-        const float4 *b4 = reinterpret_cast<const float4 *>(b);
-#pragma unroll 4
-        for (int64_t j = lane; j < ld / 4; j += 32) {
-            const float4 a = row[j], v = b4[j];
-            s += a.x * v.x;
-            s += a.y * v.y;
-            s += a.z * v.z;
-            s += a.w * v.w;
+    for (int j0 = lane; j0 < nq; j0 += 32 * kA) {
+#pragma unroll
+        for (int k = 0; k < kA; ++k) v[k] = j0 + 32 * k < nq ? b4[j0 + 32 * k] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < kA; ++k) {
+            s += a[k].x * v[k].x;
+            s += a[k].y * v[k].y;
+            s += a[k].z * v[k].z;
+            s += a[k].w * v[k].w;
+            const int jn = j0 + 32 * (kA + k);
+            a[k] = jn < nq ? __ldg(row + jn) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     }
 #pragma unroll
@@ -995,27 +1004,34 @@ __device__ __forceinline__ float fine_dot(const MatView &A, int64_t base, int w,
 // warp g of a slice's group takes the slots g, g + G, g + 2G, ... of its 32 rows, eight loaded
 // together, and the G partial sums meet in shared memory in warp order (deterministic).  Blocks
 // hold 8 warps, i.e. 8 / G slices.  G = 1 is one thread per row.
+constexpr int kPart = 8;  // slots of a thread in flight
 template <int G>
-__device__ __forceinline__ float split_part(const MatView &A, int64_t base, int w, int ln, int g,
-                                            const float *__restrict__ x) {
+__device__ __forceinline__ void split_cols(const MatView &A, int64_t base, int w, int ln, int j0, int32_t (&c)[kPart]) {
+#pragma unroll
+    for (int k = 0; k < kPart; ++k) {
+        const int j = j0 + k * G;
+        c[k] = j < w ? __ldg(A.col + base + (int64_t)j * kS + ln) : 0;
+    }
+}
+// part g's sum; c: the columns of its first slots (split_cols from g)
+template <int G, bool AHEAD>
+__device__ __forceinline__ float split_part(const MatView &A, int64_t base, int w, int ln, int g, const float *x,
+                                            int32_t (&c)[kPart]) {
     if (G == 1 && !A.rlen) return fine_dot(A, base, w, ln, x);
-    constexpr int kB = 8;
     float y = 0.f;
-    for (int j0 = g; j0 < w; j0 += kB * G) {
-        int32_t c[kB];
-        float v[kB];
+    for (int j0 = g; j0 < w; j0 += kPart * G) {
+        if (!AHEAD) split_cols<G>(A, base, w, ln, j0, c);
+        float v[kPart], gx[kPart];
 #pragma unroll
-        for (int k = 0; k < kB; ++k) {
+        for (int k = 0; k < kPart; ++k) {
             const int j = j0 + k * G;
-            const int64_t slot = base + (int64_t)j * kS + ln;
-            c[k] = j < w ? __ldg(A.col + slot) : 0;
-            v[k] = j < w ? __ldg(A.val + slot) : 0.f;
+            v[k] = j < w ? __ldg(A.val + base + (int64_t)j * kS + ln) : 0.f;
         }
-        float gx[kB];
 #pragma unroll
-        for (int k = 0; k < kB; ++k) gx[k] = j0 + k * G < w ? x[c[k]] : 0.f;
+        for (int k = 0; k < kPart; ++k) gx[k] = j0 + k * G < w ? x[c[k]] : 0.f;
+        if (AHEAD) split_cols<G>(A, base, w, ln, j0 + kPart * G, c);
 #pragma unroll
-        for (int k = 0; k < kB; ++k) y = __fmaf_rn(v[k], gx[k], y);
+        for (int k = 0; k < kPart; ++k) y = __fmaf_rn(v[k], gx[k], y);
     }
     return y;
 }
@@ -1056,22 +1072,54 @@ __global__ void k_sm_first(Gate gate, int64_t n, const float *__restrict__ b, co
     x[i] = v;
 }
 
+// The members of a coarse row: its first ones' rows are looked up ahead.
+struct Members {
+    static constexpr int kAhead = 4;
+    int32_t k0 = 0, k1 = 0, row[kAhead];
+    __device__ __forceinline__ void open(int64_t I, int64_t nc, const int32_t *__restrict__ ms,
+                                         const int32_t *__restrict__ mr) {
+        if (I < nc) {
+            k0 = ms[I];
+            k1 = ms[I + 1];
+        }
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) row[k] = k0 + k < k1 ? mr[k0 + k] : -1;
+    }
+    // sum of w r over them, in member order
+    __device__ __forceinline__ float sum(const int32_t *__restrict__ mr, const float *r, const float *wt) const {
+        float u[kAhead], v[kAhead], s = 0.f;
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+            u[k] = wt && row[k] >= 0 ? wt[row[k]] : 1.f;
+            v[k] = row[k] >= 0 ? r[row[k]] : 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) s = __fmaf_rn(u[k], v[k], s);
+        for (int32_t k = k0 + kAhead; k < k1; ++k) s = __fmaf_rn(wt ? wt[mr[k]] : 1.f, r[mr[k]], s);
+        return s;
+    }
+};
+
 // restriction fused with the first smoothing step of the coarse level:
 // b_c[I] = sum over the rows of I of w r, then x = d = c2 D_c^-1 b_c (d null: not kept)
 __global__ void k_restrict_first(Gate gate, int64_t nc, int64_t nc_pad, const int32_t *__restrict__ ms,
-                                 const int32_t *__restrict__ mr, const float *__restrict__ r,
-                                 const float *__restrict__ wt, const float *__restrict__ invd_c, float c2,
-                                 float *__restrict__ bc, float *__restrict__ x, float *__restrict__ d,
+                                 const int32_t *__restrict__ mr, const float *r, const float *wt,
+                                 const float *__restrict__ invd_c, float c2, float *bc, float *x, float *d,
                                  const int32_t *__restrict__ agg_c) {
-    if (closed(gate)) return;
     const int64_t I = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (I >= nc_pad) return;
-    float s = 0.f;
-    if (I < nc)
-        for (int32_t k = ms[I]; k < ms[I + 1]; ++k) s += (wt ? wt[mr[k]] : 1.f) * r[mr[k]];
+    Members m;
+    bool exact = false;
+    float di = 0.f;
+    if (I < nc_pad) {
+        m.open(I, nc, ms, mr);
+        exact = agg_c[I] < 0;
+        di = invd_c[I];
+    }
+    pdl_wait();
+    if (closed(gate) || I >= nc_pad) return;
+    const float s = m.sum(mr, r, wt);
     bc[I] = s;
-    const bool exact = agg_c[I] < 0;
-    const float v = (exact ? 1.f : c2) * invd_c[I] * s;
+    const float v = (exact ? 1.f : c2) * di * s;
     if (d) d[I] = exact ? 0.f : v;
     x[I] = v;
 }
@@ -1131,15 +1179,14 @@ __global__ void k_sm_first_step_w(Gate gate, MatView A, const float *__restrict_
 }
 
 // b_c[I] = sum of r over the rows of coarse row I (in member order); padding rows get 0
-__global__ void k_restrict(Gate gate, int64_t nc, int64_t nc_pad, const int32_t *__restrict__ ms, const int32_t *__restrict__ mr,
-                           const float *__restrict__ r, float *__restrict__ bc, const float *__restrict__ wt) {
-    if (closed(gate)) return;
+__global__ void k_restrict(Gate gate, int64_t nc, int64_t nc_pad, const int32_t *__restrict__ ms,
+                           const int32_t *__restrict__ mr, const float *r, float *bc, const float *wt) {
     const int64_t I = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (I >= nc_pad) return;
-    float s = 0.f;
-    if (I < nc)
-        for (int32_t k = ms[I]; k < ms[I + 1]; ++k) s += (wt ? wt[mr[k]] : 1.f) * r[mr[k]];
-    bc[I] = s;
+    Members m;
+    if (I < nc_pad) m.open(I, nc, ms, mr);
+    pdl_wait();
+    if (closed(gate) || I >= nc_pad) return;
+    bc[I] = m.sum(mr, r, wt);
 }
 
 __global__ void k_to_half(int64_t n, const float *__restrict__ a, uint16_t *__restrict__ h) {
@@ -1153,15 +1200,14 @@ __global__ void k_to_float(int64_t n, const double *__restrict__ a, float *__res
 }
 
 // x += alpha P x_c (alpha from the device scalar when given, else the constant)
-__global__ void k_prolong(Gate gate, int64_t n, const int32_t *__restrict__ agg, const float *__restrict__ xc,
-                          float *__restrict__ x, const double *__restrict__ alpha_dev, float alpha,
-                          const float *__restrict__ wt) {
-    if (closed(gate)) return;
+__global__ void k_prolong(Gate gate, int64_t n, const int32_t *__restrict__ agg, const float *xc, float *x,
+                          const double *alpha_dev, float alpha, const float *wt) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int32_t a = agg[i];
+    const int32_t a = i < n ? agg[i] : -1;
+    pdl_wait();
+    if (closed(gate) || a < 0) return;
     const float al = alpha_dev ? (float)*alpha_dev : alpha;
-    if (a >= 0) x[i] += al * (wt ? wt[i] : 1.f) * xc[a];
+    x[i] += al * (wt ? wt[i] : 1.f) * xc[a];
 }
 
 // long-row list: flags (1 where rlen > kLongRow) for a scan, then the compacted row indices
@@ -1310,10 +1356,13 @@ __device__ void dots_finish(const RowArgs &a, double xb, double xax, bool has_te
     }
 }
 
-// G warps per slice (split_row).  The row's extent and its own entries are loaded before the gate
-// is looked at.
-template <int G, int OP> __global__ void __launch_bounds__(256, 8) k_rows(RowArgs a) {
+// G warps per slice (split_row).  What the matrix says is loaded before the wait for the kernel
+// before: the row's extent and, AHEAD, its first columns.  Those cost registers, so AHEAD is for grids
+// that run in one wave at four blocks an SM; larger ones need eight (149k rows in 1164 blocks: 8.5 us a
+// pass at 40 registers, 5.4 at 32).
+template <int G, int OP, bool AHEAD> __global__ void __launch_bounds__(256, AHEAD ? 4 : 8) k_rows(RowArgs a) {
     if (blockIdx.x >= a.row_blocks) {
+        pdl_wait();
         if (closed(a.gate)) return;
         long_row<OP>(a, (int)(blockIdx.x - a.row_blocks));
         if (OP == kRowDots) dots_finish(a, 0.0, 0.0, false);
@@ -1330,14 +1379,17 @@ template <int G, int OP> __global__ void __launch_bounds__(256, 8) k_rows(RowArg
         row_of(A, i, base, w, ln);
         live = !A.rlen || A.rlen[i] <= kLongRow;
         if (OP == kRowStep) outside = a.agg && a.agg[i] < 0;
-        if (g == 0) {
-            if (OP != kRowPower) b = a.b[i];
-            if (OP == kRowStep || OP == kRowDots) x = a.x[i];
-            if ((OP == kRowStep || OP == kRowPower) && a.invd) di = a.invd[i];
-        }
+        if (g == 0 && (OP == kRowStep || OP == kRowPower) && a.invd) di = a.invd[i];
+    }
+    int32_t c[kPart];
+    if (AHEAD) split_cols<G>(A, base, live && !outside ? w : 0, ln, g, c);
+    pdl_wait();
+    if (in && g == 0) {
+        if (OP != kRowPower) b = a.b[i];
+        if (OP == kRowStep || OP == kRowDots) x = a.x[i];
     }
     if (closed(a.gate)) return;
-    const float y = split_sum<G>(live && !outside ? split_part<G>(A, base, w, ln, g, a.x) : 0.f);
+    const float y = split_sum<G>(live && !outside ? split_part<G, AHEAD>(A, base, w, ln, g, a.x, c) : 0.f);
     if (OP == kRowDots) {
         const bool mine = g == 0 && live;
         dots_finish(a, mine ? (double)x * (double)b : 0.0, mine ? (double)x * (double)y : 0.0, true);
@@ -1354,6 +1406,7 @@ template <int G, int OP> __global__ void __launch_bounds__(256, 8) k_rows(RowArg
 // 19 37 -> 37, 462k of 24 27 -> 25, 3.7M of 11 97 -> 92; the scaling's pass 31 -> 21 and 111 -> 81.
 template <int OP> __global__ void __launch_bounds__(256, 3) k_rows_pipe(RowArgs a) {
     if (blockIdx.x >= a.row_blocks) {
+        pdl_wait();
         if (closed(a.gate)) return;
         long_row<OP>(a, (int)(blockIdx.x - a.row_blocks));
         if (OP == kRowDots) dots_finish(a, 0.0, 0.0, false);
@@ -1376,9 +1429,11 @@ template <int OP> __global__ void __launch_bounds__(256, 3) k_rows_pipe(RowArgs 
         r.live = rl <= kLongRow;
         r.outside = OP == kRowStep && a.agg && a.agg[r.i] < 0;
         r.len = r.live && !r.outside ? rl : 0;
+        r.di = (OP == kRowStep || OP == kRowPower) && a.invd ? a.invd[r.i] : 1.f;
+    };
+    auto open_vec = [&](Row &r) {
         r.b = OP != kRowPower ? a.b[r.i] : 0.f;
         r.x = OP == kRowStep || OP == kRowDots ? a.x[r.i] : 0.f;
-        r.di = (OP == kRowStep || OP == kRowPower) && a.invd ? a.invd[r.i] : 1.f;
         r.d = own_d<OP>(a, r.i, r.x);
     };
     int32_t c[kB];
@@ -1399,11 +1454,16 @@ template <int OP> __global__ void __launch_bounds__(256, 3) k_rows_pipe(RowArgs 
     if (any) {
         open(sl, r);
         if (s1 < n_sl) open(s1, nx);
+        r.most = __reduce_max_sync(kFull, r.len);
+        load(r, 0);
+    }
+    pdl_wait();
+    if (any) {
+        open_vec(r);
+        if (s1 < n_sl) open_vec(nx);
     }
     if (closed(a.gate)) return;
     if (any) {
-        r.most = __reduce_max_sync(kFull, r.len);
-        load(r, 0);
         int j0 = 0;
         float y = 0.f;
         for (;;) {
@@ -1432,7 +1492,10 @@ template <int OP> __global__ void __launch_bounds__(256, 3) k_rows_pipe(RowArgs 
             r.most = __reduce_max_sync(kFull, r.len);
             sl = s1;
             s1 += step;
-            if (s1 < n_sl) open(s1, nx);
+            if (s1 < n_sl) {
+                open(s1, nx);
+                open_vec(nx);
+            }
             j0 = 0;
             y = 0.f;
         }
@@ -1486,15 +1549,16 @@ enum FineOp : int { kOpFirst, kOpFirstW, kOpStep, kOpResid };
 // (fine_first) on x = b; kOpStep: one step (fine_step); kOpResid: out = b - S^ x.
 // RD: the step continues a sequence (reads d); WD: a later step reads the d written here.
 template <int OP, bool RD, bool WD>
-__global__ void __launch_bounds__(256, 4) k_fine(Gate gate, FineView A, const float *__restrict__ b,
-                                                 const float *__restrict__ w, const float *__restrict__ x,
-                                                 float *__restrict__ out, float *__restrict__ d, float c0, float c1,
-                                                 float c2) {
+__global__ void __launch_bounds__(256, 4) k_fine(Gate gate, FineView A, const float *b, const float *w, const float *x,
+                                                 float *out, float *d, float c0, float c1, float c2) {
     constexpr bool first = OP == kOpFirst || OP == kOpFirstW;
     const int lane = threadIdx.x & 31;
     const int64_t step = (int64_t)gridDim.x * 8;
     int64_t sl = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (sl >= A.n_slices) return;
+    if (sl >= A.n_slices) {
+        pdl_wait();
+        return;
+    }
     struct Stage {
         int64_t off;
         int wd;
@@ -1512,12 +1576,14 @@ __global__ void __launch_bounds__(256, 4) k_fine(Gate gate, FineView A, const fl
             st.c[k] = k + 1 < st.wd ? __ldcs(A.col + slot) : 0;
             st.v[k] = k + 1 < st.wd ? __ldcs(A.hval + slot) : __ushort_as_half(0);
         }
+        st.outside = OP == kOpResid ? 0u : __ldg(A.outside + s);
+    };
+    auto load_vec = [&](int64_t s) {
         const int64_t i = s * kS + lane;
         st.xi = x[i];
         st.bi = first ? st.xi : b[i];
         st.wi = (OP == kOpFirstW || (OP == kOpStep && w)) ? w[i] : 1.f;
         st.di = RD ? d[i] : 0.f;
-        st.outside = OP == kOpResid ? 0u : __ldg(A.outside + s);
     };
     load(sl, A.off[sl], A.off[sl + 1]);
     int64_t s1 = sl + step, o1 = 0, o2 = 0;
@@ -1525,6 +1591,8 @@ __global__ void __launch_bounds__(256, 4) k_fine(Gate gate, FineView A, const fl
         o1 = A.off[s1];
         o2 = A.off[s1 + 1];
     }
+    pdl_wait();
+    load_vec(sl);
     if (closed(gate)) return;
     for (;;) {
         float g[kFn];
@@ -1538,6 +1606,7 @@ __global__ void __launch_bounds__(256, 4) k_fine(Gate gate, FineView A, const fl
         sl = s1;
         if (sl < A.n_slices) {
             load(sl, o1, o2);
+            load_vec(sl);
             s1 = sl + step;
             if (s1 < A.n_slices) {
                 o1 = A.off[s1];
@@ -2070,8 +2139,11 @@ __global__ void __launch_bounds__(kTailThreads, 1)
 }
 
 // the row kernel of a level with G warps per slice (G = 1, 2, 4 or 8)
-template <int OP> decltype(&k_rows<1, OP>) rows_kernel(int g) {
-    return g >= 8 ? k_rows<8, OP> : g >= 4 ? k_rows<4, OP> : g >= 2 ? k_rows<2, OP> : k_rows<1, OP>;
+template <int OP, bool AHEAD> decltype(&k_rows<1, OP, AHEAD>) rows_kernel(int g) {
+    return g >= 8   ? k_rows<8, OP, AHEAD>
+           : g >= 4 ? k_rows<4, OP, AHEAD>
+           : g >= 2 ? k_rows<2, OP, AHEAD>
+                    : k_rows<1, OP, AHEAD>;
 }
 decltype(&k_level_diag<1>) level_diag_kernel(int g) {
     return g >= 8 ? k_level_diag<8> : g >= 4 ? k_level_diag<4> : g >= 2 ? k_level_diag<2> : k_level_diag<1>;
@@ -2082,14 +2154,15 @@ decltype(&k_pair_want<1>) pair_want_kernel(int g) {
 // blocks of 8 warps covering n rows (a multiple of 32) with G warps per slice
 unsigned split_blocks(int64_t n, int g) { return nblk(n / kS * g, 8); }
 unsigned row_blocks(const AmgLevel &L) { return L.pipe ? L.pipe : split_blocks(L.A.n, L.g); }
-template <int OP> void launch_rows(const AmgLevel &L, RowArgs a, cudaStream_t s) {
+constexpr unsigned kAheadBlocks = 4 * 148;
+template <int OP> void launch_rows(const AmgLevel &L, RowArgs a, cudaStream_t s, bool chained) {
     a.A = view(L.A);
     a.longrows = L.A.longrows;
     a.n_long = (int32_t)std::max<int64_t>(0, L.A.n_long);
     a.row_blocks = row_blocks(L);
     const unsigned grid = a.row_blocks + (unsigned)a.n_long;
-    if (L.pipe) k_rows_pipe<OP><<<grid, 256, 0, s>>>(a);
-    else rows_kernel<OP>(L.g)<<<grid, 256, 0, s>>>(a);
+    const auto k = L.pipe ? k_rows_pipe<OP> : grid <= kAheadBlocks ? rows_kernel<OP, true>(L.g) : rows_kernel<OP, false>(L.g);
+    launch_chained(chained, k, grid, 256, s, a);
 }
 // warps per slice for a matrix: the fewest with at most `width` slots per warp and row (one on
 // the fine level, whose 7-8 entries per row are loaded together by each thread)
@@ -2699,7 +2772,7 @@ cudaError_t Amg::power_estimates(cudaStream_t s, int only_level) {
             a.x = x;
             a.out = y;
             a.invd = invd;
-            launch_rows<kRowPower>(L, a, s);
+            launch_rows<kRowPower>(L, a, s, false);
             if (k + 1 < opt_.power_steps) std::swap(x, y);
         }
         k_power_norms<<<kPowerBlocks, 256, 0, s>>>(n, x, y, pw_part_.p);
@@ -3042,17 +3115,24 @@ bool Amg::fine_tma_failed(cudaStream_t s) {
 }
 
 cudaError_t Amg::apply(const float *r, float *z, const int32_t *n_done, int32_t n_inst, cudaStream_t s,
-                       AmgProf *prof) {
-    return cycle(0, r, z, n_done, n_inst, s, prof, nullptr);
+                       AmgProf *prof, bool follows) {
+    return cycle(0, r, z, n_done, n_inst, s, prof, nullptr, follows);
 }
 
 // The V-cycle from level l0: l0 = 0 is the preconditioner (rhs r, result z); l0 > 0 runs the
 // cycle of the coarser levels on the rhs already in lv_[l0].b and leaves its result in
 // *x_l0 (a level buffer), with no fine-level work.
 cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, int32_t n_inst, cudaStream_t s,
-                       AmgProf *prof, float **x_l0) {
+                       AmgProf *prof, float **x_l0, bool follows) {
     const Gate gate_{n_done, n_inst};
     const int pre = pre_degree();
+    // whether the next kernel's launch may overlap the one before (not beside recorded events)
+    bool chained = follows;
+    auto chain = [&] {
+        const bool c = chained && !prof;
+        chained = true;
+        return c;
+    };
     // a Chebyshev step of a level; dx: d is x_in (the second step), more: a later step reads d
     auto step = [&](const AmgLevel &L, const float *b, const float *invd, const float *xi, float *xo, float c1,
                     float c2, bool dx, bool more, const int32_t *agg) {
@@ -3068,7 +3148,7 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
         a.dx = dx;
         a.wd = more;
         a.agg = agg;
-        launch_rows<kRowStep>(L, a, s);
+        launch_rows<kRowStep>(L, a, s, chain());
     };
     // inside a capture only cudaEventRecordExternal turns a record into a graph node
     auto rec = [&](cudaEvent_t ev) {
@@ -3098,7 +3178,7 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
                           bool more) {
         const auto f = c1 != 0.f ? (more ? k_fine<kOpStep, true, true> : k_fine<kOpStep, true, false>)
                                  : (more ? k_fine<kOpStep, false, true> : k_fine<kOpStep, false, false>);
-        f<<<gf, 256, 0, s>>>(gate_, F, b, w, xi, xo, d, 0.f, c1, c2);
+        launch_chained(chain(), f, gf, 256, s, gate_, F, b, w, xi, xo, d, 0.f, c1, c2);
     };
     for (int l = l0; l < (use_tail ? tail_level_ : nl - 1); ++l) {
         AmgLevel &L = lv_[l];
@@ -3114,7 +3194,8 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
             if (opt_.half_fine && (fine_w_ || !tma0)) {
                 const auto f = fine_w_ ? (pre > 2 ? k_fine<kOpFirstW, false, true> : k_fine<kOpFirstW, false, false>)
                                        : (pre > 2 ? k_fine<kOpFirst, false, true> : k_fine<kOpFirst, false, false>);
-                f<<<gf, 256, 0, s>>>(gate_, F, b, fw(), b, xo, L.d.p, (float)c2[0], (float)c1[1], (float)c2[1]);
+                launch_chained(chain(), f, gf, 256, s, gate_, F, b, fw(), b, xo, L.d.p, (float)c2[0], (float)c1[1],
+                               (float)c2[1]);
             } else if (fine_w_)
                 k_sm_first_step_w<<<g, 256, 0, s>>>(gate_, view(L.A), b, fw(), xo, L.d.p, (float)c2[0], (float)c1[1],
                                                     (float)c2[1], L.agg.p);
@@ -3146,26 +3227,27 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
         if (l == 0 && tma0)
             launch_fine<kFineResid>(n_done, n_inst, b, nullptr, xi, L.r.p, nullptr, 0.f, 0.f, 0.f, s);
         else if (l == 0 && half0)
-            k_fine<kOpResid, false, false><<<gf, 256, 0, s>>>(gate_, F, b, nullptr, xi, L.r.p, nullptr, 0.f, 0.f, 0.f);
+            launch_chained(chain(), k_fine<kOpResid, false, false>, gf, 256, s, gate_, F, b, nullptr, xi, L.r.p, nullptr,
+                           0.f, 0.f, 0.f);
         else {
             RowArgs a = {};
             a.gate = gate_;
             a.b = b;
             a.x = xi;
             a.out = L.r.p;
-            launch_rows<kRowResid>(L, a, s);
+            launch_rows<kRowResid>(L, a, s, chain());
         }
         AmgLevel &C = lv_[l + 1];
         const float *wt = l == 0 ? w0_used_ : nullptr;
         if (l + 2 < nl) {
             std::vector<double> cc1, cc2;
             cheb_coeffs(C, cc1, cc2);
-            k_restrict_first<<<nblk(C.A.n, 256), 256, 0, s>>>(gate_, L.nc, C.A.n, L.mem_start.p, L.mem_rows.p, L.r.p, wt,
-                                                              C.inv_diag.p, (float)cc2[0], C.b.p, C.xa.p,
-                                                              use_tail && l + 1 == tail_level_ ? C.d.p : nullptr,
-                                                              C.agg.p);
+            launch_chained(chain(), k_restrict_first, nblk(C.A.n, 256), 256, s, gate_, L.nc, C.A.n, L.mem_start.p,
+                           L.mem_rows.p, L.r.p, wt, C.inv_diag.p, (float)cc2[0], C.b.p, C.xa.p,
+                           use_tail && l + 1 == tail_level_ ? C.d.p : nullptr, C.agg.p);
         } else {
-            k_restrict<<<nblk(C.A.n, 256), 256, 0, s>>>(gate_, L.nc, C.A.n, L.mem_start.p, L.mem_rows.p, L.r.p, C.b.p, wt);
+            launch_chained(chain(), k_restrict, nblk(C.A.n, 256), 256, s, gate_, L.nc, C.A.n, L.mem_start.p, L.mem_rows.p,
+                           L.r.p, C.b.p, wt);
         }
     }
     // coarsest: dense inverse, or (when coarsening stalled above the dense limit) a Chebyshev
@@ -3178,8 +3260,8 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
         const float *b = nl == 1 ? r : Lc.b.p;
         if (dense_n_ > 0) {
             float *x = nl == 1 ? z : Lc.xa.p;
-            k_dense_gemv<<<nblk(Lc.A.n * 32, 256), 256, 0, s>>>(gate_, dense_inv_.p, dense_n_, dense_ld(dense_n_), Lc.A.n,
-                                                                 b, x);
+            launch_chained(chain(), k_dense_gemv, nblk(Lc.A.n * 32, 256), 256, s, gate_, dense_inv_.p, dense_n_,
+                           dense_ld(dense_n_), Lc.A.n, b, x);
             xout[nl - 1] = x;
         } else {
             const unsigned g = nblk(Lc.A.n, 256);
@@ -3220,10 +3302,11 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
             a.long_part = lp;
             a.alpha = alpha_.p + l;
             a.ticket = tickets_.p + l;
-            launch_rows<kRowDots>(C, a, s);
+            launch_rows<kRowDots>(C, a, s, chain());
             al = alpha_.p + l;
         }
-        k_prolong<<<g, 256, 0, s>>>(gate_, L.A.n, L.agg.p, xout[l + 1], xi, al, opt_.alpha, l == 0 ? w0_used_ : nullptr);
+        launch_chained(chain(), k_prolong, g, 256, s, gate_, L.A.n, L.agg.p, xout[l + 1], xi, al, opt_.alpha,
+                       l == 0 ? w0_used_ : nullptr);
         float *other = xi == L.xa.p ? L.xb.p : L.xa.p;
         for (int k = 0; k < deg; ++k) {
             float *xo = (l == 0 && k == deg - 1) ? z : other;
@@ -3255,7 +3338,7 @@ cudaError_t Amg::coarse_correct(const float *v, float *out, cudaStream_t s) {
     k_restrict<<<nblk(C.A.n, 256), 256, 0, s>>>(g, L0.nc, C.A.n, L0.mem_start.p, L0.mem_rows.p, v, C.b.p, w0_used_);
     AMG_CK(cudaGetLastError());
     float *xc = nullptr;
-    cudaError_t e = cycle(1, nullptr, nullptr, nullptr, 0, s, nullptr, &xc);
+    cudaError_t e = cycle(1, nullptr, nullptr, nullptr, 0, s, nullptr, &xc, false);
     if (e != cudaSuccess) return e;
     k_prolong<<<nblk(n, 256), 256, 0, s>>>(g, n, L0.agg.p, xc, out, nullptr, 1.f, w0_used_);
     return cudaGetLastError();
@@ -3284,7 +3367,7 @@ cudaError_t Amg::smooth_fine(const float *b, float *x, cudaStream_t s) {
         a.dx = k == 1;
         a.wd = k + 1 < pre;
         a.agg = agg;
-        launch_rows<kRowStep>(L, a, s);
+        launch_rows<kRowStep>(L, a, s, false);
         std::swap(xi, xo);
     }
     AMG_CK(cudaGetLastError());

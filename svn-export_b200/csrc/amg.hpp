@@ -110,8 +110,10 @@ public:
     // z = M r over all rows of the solver space (one V-cycle); stream-ordered, capturable.
     // The kernels do nothing once *n_done >= n_inst (n_done may be null).
     // With prof, events are recorded around the cycle and its fine-level smoothing steps.
+    // follows: the launch before on s is a kernel that leaves the hierarchy as it is, so the
+    // cycle's first kernel may be brought up while it runs (pdl.hpp).
     cudaError_t apply(const float *r, float *z, const int32_t *n_done, int32_t n_inst, cudaStream_t s,
-                      AmgProf *prof = nullptr);
+                      AmgProf *prof = nullptr, bool follows = false);
     // smoothing steps on the fine level per cycle (none when the fine level is the coarsest)
     int fine_steps() const { return n_levels_ > 1 ? pre_degree() - 1 + std::max(1, opt_.cheb_degree) : 0; }
     int pre_degree() const { return opt_.pre_degree > 0 ? opt_.pre_degree : std::max(1, opt_.cheb_degree); }
@@ -168,7 +170,7 @@ private:
     // fixed pseudo-random start; deterministic sums), as |v_k|^2 and |v_{k-1}|^2 per level
     cudaError_t power_estimates(cudaStream_t s, int only_level = -1);
     cudaError_t cycle(int l0, const float *r, float *z, const int32_t *n_done, int32_t n_inst, cudaStream_t s,
-                      AmgProf *prof, float **x_l0);
+                      AmgProf *prof, float **x_l0, bool follows);
     cudaError_t scan_i32(const int32_t *in, int32_t *out, int64_t n, int64_t &total, cudaStream_t s);
     cudaError_t scan_i64(const int64_t *in, int64_t *out, int64_t n, int64_t &total, cudaStream_t s);
     // the same without reading the total back (out[n] holds it on the device)

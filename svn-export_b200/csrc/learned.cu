@@ -5,6 +5,7 @@
 
 #include "device_system.hpp"
 #include "learned.hpp"
+#include "pdl.hpp"
 
 namespace mh {
 
@@ -113,11 +114,9 @@ struct FcgStage {
     float dg, z, r, p, q;
 };
 
-__device__ __forceinline__ void fcg_stage_load(const SellView<float> &A, const float *__restrict__ z,
-                                               const float *__restrict__ r, const float *__restrict__ p,
-                                               const float *__restrict__ q, bool have, int tile, FcgStage &st) {
+__device__ __forceinline__ void fcg_stage_load(const SellView<float> &A, int tile, FcgStage &st) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t sl = (int64_t)tile * kWarpsPerBlock + warp, row = sl * kSliceRows + lane;
+    const int64_t sl = (int64_t)tile * kWarpsPerBlock + warp;
     st.off = A.slice_off[sl];
     st.w = (int)((A.slice_off[sl + 1] - st.off) / kSliceRows);
     st.dg = __ldcs(A.val + st.off + lane);  // a row's first slot is its diagonal
@@ -128,6 +127,10 @@ __device__ __forceinline__ void fcg_stage_load(const SellView<float> &A, const f
         st.c[j] = in ? __ldcs(A.col + slot) : 0;
         st.v[j] = in ? __ldcs(A.val + slot) : 0.f;
     }
+}
+__device__ __forceinline__ void fcg_stage_load_vec(const float *z, const float *r, const float *p, const float *q,
+                                                   bool have, int tile, FcgStage &st) {
+    const int64_t row = ((int64_t)tile * kWarpsPerBlock + (threadIdx.x >> 5)) * kSliceRows + (threadIdx.x & 31);
     st.z = z[row];
     st.r = r[row];
     st.p = have ? p[row] : 0.f;
@@ -135,28 +138,31 @@ __device__ __forceinline__ void fcg_stage_load(const SellView<float> &A, const f
 }
 
 __global__ void __launch_bounds__(kBlockThreads, 4)
-    k_fcg_spmv(SellView<float> A, const float *__restrict__ z, const float *__restrict__ r,
-               const float *__restrict__ p, const float *__restrict__ q, float *__restrict__ s,
-               double *__restrict__ partial, InstCtl *__restrict__ ctl, Plan plan, int32_t *n_done) {
+    k_fcg_spmv(SellView<float> A, const float *z, const float *r, const float *p, const float *q, float *s,
+               double *partial, InstCtl *ctl, Plan plan, int32_t *n_done) {
     const int inst = plan.inst[blockIdx.x];
     InstCtl *c = ctl + inst;
-    if (c->done) return;
-    const double pq_old = c->aux[0];
-    const bool have = c->aux[1] != 0.0 && pq_old != 0.0;  // else (p, q) may hold a broken direction
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // the instance's blocks take its tiles in turn, so that all of them gather from one moving window
     const int pb = plan.inst_blk[inst], nb = plan.inst_blk[inst + 1] - pb;
     const int tb = plan.tile_begin[pb] + ((int)blockIdx.x - pb), te = plan.tile_end[pb + nb - 1];
+    FcgStage st;
+    if (tb < te) fcg_stage_load(A, tb, st);
+    pdl_wait();
+    if (c->done) return;
+    const bool have = c->aux[1] != 0.0 && c->aux[0] != 0.0;  // else (p, q) may hold a broken direction
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int kJ = FcgStage::kJ;
     Sums<4> t = {{0.0, 0.0, 0.0, 0.0}};
-    FcgStage st;
-    if (tb < te) fcg_stage_load(A, z, r, p, q, have, tb, st);
+    if (tb < te) fcg_stage_load_vec(z, r, p, q, have, tb, st);
     for (int tile = tb; tile < te; tile += nb) {
         float g[kJ];
 #pragma unroll
         for (int j = 0; j < kJ; ++j) g[j] = z[st.c[j]];
         const FcgStage cur = st;
-        if (tile + nb < te) fcg_stage_load(A, z, r, p, q, have, tile + nb, st);
+        if (tile + nb < te) {
+            fcg_stage_load(A, tile + nb, st);
+            fcg_stage_load_vec(z, r, p, q, have, tile + nb, st);
+        }
         double y = (double)cur.dg * (double)cur.z;
 #pragma unroll
         for (int j = 0; j < kJ; ++j) y += (double)cur.v[j] * (double)g[j];
@@ -172,7 +178,7 @@ __global__ void __launch_bounds__(kBlockThreads, 4)
     }
     Sums<4> tot;
     if (block_finish<4>(t, partial, c, plan, inst, tot) && threadIdx.x == 0) {
-        const double beta = have ? tot.v[0] / pq_old : 0.0;
+        const double beta = have ? tot.v[0] / c->aux[0] : 0.0;  // (p.q of the iteration before)
         const double pr = tot.v[1] - beta * tot.v[2], pq = tot.v[3] - beta * tot.v[0];
         c->rho = pr;
         c->beta = beta;
@@ -186,11 +192,13 @@ __global__ void __launch_bounds__(kBlockThreads, 4)
 }
 
 __global__ void __launch_bounds__(kBlockThreads)
-    k_fcg_update(float4 *__restrict__ x, float4 *__restrict__ r, float4 *__restrict__ p, float4 *__restrict__ q,
-                 const float4 *__restrict__ z, const float4 *__restrict__ s, double *__restrict__ partial,
-                 InstCtl *__restrict__ ctl, Plan plan, int32_t *n_done) {
+    k_fcg_update(float4 *x, float4 *r, float4 *p, float4 *q, const float4 *z, const float4 *s, double *partial,
+                 InstCtl *ctl, Plan plan, int32_t *n_done) {
     const int inst = plan.inst[blockIdx.x];
     InstCtl *c = ctl + inst;
+    const int pb = plan.inst_blk[inst], nb = plan.inst_blk[inst + 1] - pb;
+    const int t0 = plan.tile_begin[pb], t1 = plan.tile_end[pb + nb - 1];
+    pdl_wait();
     if (c->done) return;
     const double alpha = c->alpha, beta = c->beta;
     double rr = 0.0;
@@ -204,9 +212,8 @@ __global__ void __launch_bounds__(kBlockThreads)
         rr += (double)rv * (double)rv;
     };
     // four rows a thread and turn: four tiles at a time of the instance's run, the blocks in turn
-    const int pb = plan.inst_blk[inst], nb = plan.inst_blk[inst + 1] - pb;
     constexpr int64_t kPer = kBlockThreads / 4;
-    const int64_t i0 = plan.tile_begin[pb] * kPer, end = plan.tile_end[pb + nb - 1] * kPer;
+    const int64_t i0 = t0 * kPer, end = t1 * kPer;
     for (int64_t i = i0 + ((int64_t)blockIdx.x - pb) * kBlockThreads + threadIdx.x; i < end;
          i += (int64_t)nb * kBlockThreads) {
         const float4 zv = __ldcs(z + i), sv = __ldcs(s + i);
@@ -336,17 +343,17 @@ cudaError_t launch_cheb_apply(const DevSystem &sys, const float *r, float *z0, f
     return cudaGetLastError();
 }
 
-cudaError_t launch_fcg_iteration(const DevSystem &sys, const float *z, cudaStream_t s) {
+cudaError_t launch_fcg_iteration(const DevSystem &sys, const float *z, cudaStream_t s, bool chained) {
     if (sys.rows_per_thread != 1) return cudaErrorInvalidValue;  // tiles of 256 rows
     const SellView<float> A = {sys.n_rows, sys.slice_off, sys.col, sys.val32};
     const unsigned g = (unsigned)sys.plan[1].n_blocks;
     auto v4 = [](float *v) { return reinterpret_cast<float4 *>(v); };  // rows start on cudaMalloc's boundary
-    k_fcg_spmv<<<g, kBlockThreads, 0, s>>>(A, z, sys.r32, sys.p32, sys.q32, sys.s32, sys.partial, sys.ctl, plan32(sys),
-                                           sys.n_done);
-    k_fcg_update<<<g, kBlockThreads, 0, s>>>(v4(sys.x32), v4(sys.r32), v4(sys.p32), v4(sys.q32),
-                                             reinterpret_cast<const float4 *>(z), v4(sys.s32), sys.partial, sys.ctl,
-                                             plan32(sys), sys.n_done);
-    return cudaGetLastError();
+    const cudaError_t e = launch_chained(chained, k_fcg_spmv, g, kBlockThreads, s, A, z, sys.r32, sys.p32, sys.q32, sys.s32,
+                                         sys.partial, sys.ctl, plan32(sys), sys.n_done);
+    if (e != cudaSuccess) return e;
+    return launch_chained(true, k_fcg_update, g, kBlockThreads, s, v4(sys.x32), v4(sys.r32), v4(sys.p32), v4(sys.q32),
+                          reinterpret_cast<const float4 *>(z), v4(sys.s32), sys.partial, sys.ctl, plan32(sys),
+                          sys.n_done);
 }
 
 cudaError_t launch_spectrum_bound(const DevSystem &sys, unsigned int *out, cudaStream_t s) {

@@ -951,7 +951,7 @@ int spectrum_bound(mh_handle *h, double &hi) {
 // One flexible-CG iteration: z = M(r) (network, Chebyshev polynomial or AMG V-cycle) with
 // beta = z.q_old / (p.q)_old, p = z - beta p, q = S^ p with alpha = p.r / p.q, x and r.
 cudaError_t fcg_iteration(mh_handle *h, Pc kind, int degree, double lo, double hi, cudaStream_t s,
-                          mh::AmgProf *prof = nullptr) {
+                          mh::AmgProf *prof = nullptr, bool follows = false) {
     mh::DevSystem &sys = h->sys;
     cudaError_t e;
     switch (kind) {
@@ -959,10 +959,10 @@ cudaError_t fcg_iteration(mh_handle *h, Pc kind, int degree, double lo, double h
             e = mh::launch_cheb_apply(sys, sys.r32, h->cheb_z0, h->cheb_z1, h->cheb_d, sys.z32, degree, lo, hi, s);
             break;
         default:
-            e = h->amg.apply(sys.r32, sys.z32, sys.n_done, sys.n_inst, s, prof);
+            e = h->amg.apply(sys.r32, sys.z32, sys.n_done, sys.n_inst, s, prof, follows);
             break;
     }
-    return e == cudaSuccess ? mh::launch_fcg_iteration(sys, sys.z32, s) : e;
+    return e == cudaSuccess ? mh::launch_fcg_iteration(sys, sys.z32, s, !prof) : e;
 }
 
 int fcg_kernels_per_iteration(mh_handle *h, Pc kind, int degree) {
@@ -1008,7 +1008,7 @@ int run_fcg(mh_handle *h, Pc kind, int degree, double lo, double hi, int ipg, in
                 [&](cudaStream_t cs) {
                     cudaError_t b = cudaSuccess;
                     for (int k = 0; k < ipg && b == cudaSuccess; ++k)
-                        b = fcg_iteration(h, kind, degree, lo, hi, cs, nullptr);
+                        b = fcg_iteration(h, kind, degree, lo, hi, cs, nullptr, k > 0);
                     return b;
                 },
                 &g);
@@ -1019,7 +1019,7 @@ int run_fcg(mh_handle *h, Pc kind, int degree, double lo, double hi, int ipg, in
         } else {
             CK(cudaStreamBeginCapture(h->own_stream, cudaStreamCaptureModeThreadLocal));
             for (int k = 0; k < ipg && e == cudaSuccess; ++k)
-                e = fcg_iteration(h, kind, degree, lo, hi, h->own_stream, prof ? &h->amg_prof[k] : nullptr);
+                e = fcg_iteration(h, kind, degree, lo, hi, h->own_stream, prof ? &h->amg_prof[k] : nullptr, k > 0);
             cudaError_t e2 = cudaStreamEndCapture(h->own_stream, &g);
             if (e != cudaSuccess || e2 != cudaSuccess) {
                 if (e2 == cudaSuccess) cudaGraphDestroy(g);

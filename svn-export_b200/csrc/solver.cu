@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 
 #include "device_system.hpp"
+#include "pdl.hpp"
 
 namespace mh {
 
@@ -620,8 +621,9 @@ __global__ void k_loop_init(cudaGraphConditionalHandle hnd, int32_t *__restrict_
     cudaGraphSetConditional(hnd, (*n_done < n_inst && loop[1] > 0) ? 1u : 0u);
 }
 
-__global__ void k_loop_next(cudaGraphConditionalHandle hnd, int32_t *__restrict__ loop,
-                            const int32_t *__restrict__ n_done, int32_t n_inst) {
+__global__ void k_loop_next(cudaGraphConditionalHandle hnd, int32_t *loop,
+                            const int32_t *n_done, int32_t n_inst) {
+    pdl_wait();
     const int32_t c = loop[0] + 1;
     loop[0] = c;
     cudaGraphSetConditional(hnd, (*n_done < n_inst && c < loop[1]) ? 1u : 0u);
@@ -633,8 +635,7 @@ cudaError_t launch_loop_init(const DevSystem &sys, cudaGraphConditionalHandle hn
 }
 
 cudaError_t launch_loop_next(const DevSystem &sys, cudaGraphConditionalHandle hnd, int32_t *loop, cudaStream_t s) {
-    k_loop_next<<<1, 1, 0, s>>>(hnd, loop, sys.n_done, sys.n_inst);
-    return cudaGetLastError();
+    return launch_chained(true, k_loop_next, 1, 1, s, hnd, loop, sys.n_done, sys.n_inst);
 }
 
 int krylov_target_blocks(int rows_per_thread, int prec) {
