@@ -111,6 +111,7 @@ template <typename T> __device__ __forceinline__ T block_incl_scan(T v, T *ws, T
 }
 
 template <typename T> __global__ void __launch_bounds__(1024) k_scan_block(const T *in, T *out, T *bsum, int64_t n) {
+    pdl_wait();
     __shared__ T ws[32];
     const int64_t i = (int64_t)blockIdx.x * 1024 + threadIdx.x;
     const T v = i < n ? in[i] : T(0);
@@ -121,6 +122,7 @@ template <typename T> __global__ void __launch_bounds__(1024) k_scan_block(const
 }
 
 template <typename T> __global__ void __launch_bounds__(1024) k_scan_sums(T *bsum, int64_t nb) {
+    pdl_wait();
     __shared__ T ws[32];
     T carry = 0;
     for (int64_t base = 0; base < nb; base += 1024) {
@@ -135,6 +137,7 @@ template <typename T> __global__ void __launch_bounds__(1024) k_scan_sums(T *bsu
 }
 
 template <typename T> __global__ void k_scan_add(T *out, const T *bsum, int64_t n, int64_t nb) {
+    pdl_wait();
     const int64_t i = (int64_t)blockIdx.x * 1024 + threadIdx.x;
     if (i < n) out[i] += bsum[blockIdx.x];
     if (i == 0) out[n] = bsum[nb];
@@ -143,6 +146,7 @@ template <typename T> __global__ void k_scan_add(T *out, const T *bsum, int64_t 
 // the whole scan in one block (small n: one launch instead of three)
 constexpr int64_t kScanOneMax = 8192;
 template <typename T> __global__ void __launch_bounds__(1024) k_scan_one(const T *in, T *out, int64_t n) {
+    pdl_wait();
     __shared__ T ws[32];
     T carry = 0;
     for (int64_t base = 0; base < n; base += 1024) {
@@ -160,15 +164,15 @@ template <typename T> __global__ void __launch_bounds__(1024) k_scan_one(const T
 template <typename T> cudaError_t launch_scan(const T *in, T *out, int64_t n, DBuf<T> &blk, cudaStream_t s) {
     if (n <= 0) return cudaMemsetAsync(out, 0, sizeof(T), s);
     if (n <= kScanOneMax) {
-        k_scan_one<T><<<1, 1024, 0, s>>>(in, out, n);
+        launch_chained(true, k_scan_one<T>, 1, 1024, s, in, out, n);
         return cudaGetLastError();
     }
     const int64_t nb = (n + 1023) / 1024;
     cudaError_t e = blk.ensure(nb + 1);
     if (e != cudaSuccess) return e;
-    k_scan_block<T><<<(unsigned)nb, 1024, 0, s>>>(in, out, blk.p, n);
-    k_scan_sums<T><<<1, 1024, 0, s>>>(blk.p, nb);
-    k_scan_add<T><<<(unsigned)nb, 1024, 0, s>>>(out, blk.p, n, nb);
+    launch_chained(true, k_scan_block<T>, (unsigned)nb, 1024, s, in, out, blk.p, n);
+    launch_chained(true, k_scan_sums<T>, 1, 1024, s, blk.p, nb);
+    launch_chained(true, k_scan_add<T>, (unsigned)nb, 1024, s, out, blk.p, n, nb);
     return cudaGetLastError();
 }
 
@@ -185,6 +189,7 @@ template <int G> __device__ __forceinline__ void split_row(int64_t &i, int &g) {
 // Gershgorin bound max_i sum_j |a_ij| / a_ii of D^-1 A.
 template <int G>
 __global__ void __launch_bounds__(256) k_level_diag(MatView A, float *inv_diag, float *isd, unsigned int *bound) {
+    pdl_wait();
     int64_t i;
     int g;
     split_row<G>(i, g);
@@ -202,8 +207,8 @@ __global__ void __launch_bounds__(256) k_level_diag(MatView A, float *inv_diag, 
             for (int k = 0; k < kB; ++k) {
                 const int j = j0 + k * G;
                 const int64_t slot = base + (int64_t)j * kS + ln;
-                c[k] = j < w ? __ldg(A.col + slot) : -1;
-                v[k] = j < w ? __ldg(A.val + slot) : 0.f;
+                c[k] = j < w ? A.col[slot] : -1;
+                v[k] = j < w ? A.val[slot] : 0.f;
             }
 #pragma unroll
             for (int k = 0; k < kB; ++k) {
@@ -284,8 +289,9 @@ __device__ void k_level_diag_long_row(MatView A, int64_t i, float *inv_diag, flo
     }
 }
 
-__global__ void __launch_bounds__(256) k_level_diag_long(MatView A, const int32_t *__restrict__ list, float *inv_diag,
+__global__ void __launch_bounds__(256) k_level_diag_long(MatView A, const int32_t *list, float *inv_diag,
                                                          float *isd, unsigned int *bound) {
+    pdl_wait();
     // list = [count, rows...]; the blocks stride over the rows
     for (int32_t k = blockIdx.x; k < list[0]; k += gridDim.x) {
         k_level_diag_long_row(A, list[1 + k], inv_diag, isd, bound);
@@ -299,6 +305,7 @@ __global__ void __launch_bounds__(256) k_level_diag_long(MatView A, const int32_
 // left without coupling, e.g. a whole batch instance reduced to one row) get agg = -1: they
 // leave the hierarchy and the smoother solves them exactly (x = b / a_ii).
 __global__ void k_pair_init(MatView A, const int32_t *row_edge, const float *isd, int32_t *mate) {
+    pdl_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= A.n) return;
     bool coupled = false;
@@ -343,6 +350,7 @@ __device__ __forceinline__ bool better(float s, int32_t c, float bw, int32_t bes
 template <int G>
 __global__ void __launch_bounds__(256) k_pair_want(MatView A, const float *isd, const int32_t *mate, int32_t *want,
                                                    int mix) {
+    pdl_wait();
     int64_t i;
     int g;
     split_row<G>(i, g);
@@ -361,8 +369,8 @@ __global__ void __launch_bounds__(256) k_pair_want(MatView A, const float *isd, 
             for (int k = 0; k < kB; ++k) {
                 const int j = j0 + k * G;
                 const int64_t slot = base + (int64_t)j * kS + ln;
-                c[k] = j < w ? __ldg(A.col + slot) : (int32_t)i;
-                v[k] = j < w ? __ldg(A.val + slot) : 0.f;
+                c[k] = j < w ? A.col[slot] : (int32_t)i;
+                v[k] = j < w ? A.val[slot] : 0.f;
             }
             int32_t mt[kB];
             float sc[kB];
@@ -403,6 +411,7 @@ __global__ void __launch_bounds__(256) k_pair_want(MatView A, const float *isd, 
 
 // Handshake: i and j pair when each is the other's choice; a row with no candidate is final.
 __global__ void k_pair_match(int64_t n, const int32_t *want, int32_t *mate) {
+    pdl_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || mate[i] != kUnmatched) return;
     const int32_t j = want[i];
@@ -414,6 +423,7 @@ __global__ void k_pair_match(int64_t n, const int32_t *want, int32_t *mate) {
 // low 32 bits 1 for a leader, high 32 bits the aggregate's member count.  The exclusive scan
 // then gives every leader its aggregate id (low) and member offset (high).
 __global__ void k_pair_pack(int64_t n, const int32_t *mate, int64_t *packed) {
+    pdl_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int32_t m = mate[i];
@@ -424,6 +434,7 @@ __global__ void k_pair_pack(int64_t n, const int32_t *mate, int64_t *packed) {
 // agg of every row, and the member lists (leader first, then its pair)
 __global__ void k_pair_finish(int64_t n, int64_t nc, int64_t members, const int32_t *mate, const int64_t *packed,
                               const int64_t *pscan, int32_t *agg, int32_t *mstart, int32_t *mrows) {
+    pdl_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) mstart[nc] = (int32_t)members;
     if (i >= n) return;
@@ -442,6 +453,7 @@ __global__ void k_pair_finish(int64_t n, int64_t nc, int64_t members, const int3
 
 // Two pairing passes composed: agg = agg2[agg1[i]], members of each final row in order.
 __global__ void k_compose_agg(int64_t n, const int32_t *agg1, const int32_t *agg2, int32_t *agg) {
+    pdl_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int32_t a = agg1[i];
@@ -449,6 +461,7 @@ __global__ void k_compose_agg(int64_t n, const int32_t *agg1, const int32_t *agg
 }
 
 __global__ void k_compose_count(int64_t nc, const int32_t *ms2, const int32_t *mr2, const int32_t *ms1, int32_t *cnt) {
+    pdl_wait();
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nc) return;
     int32_t k = 0;
@@ -458,6 +471,7 @@ __global__ void k_compose_count(int64_t nc, const int32_t *ms2, const int32_t *m
 
 __global__ void k_compose_fill(int64_t nc, const int32_t *ms2, const int32_t *mr2, const int32_t *ms1,
                                const int32_t *mr1, const int32_t *ms, int32_t *mr) {
+    pdl_wait();
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nc) return;
     int32_t p = ms[c];
@@ -721,8 +735,8 @@ __global__ void __launch_bounds__(kGalWarps * 32)
 }
 
 // Candidate bound of each coarse row: the summed lengths of its rows
-__global__ void k_cand_bound(MatView A, const int32_t *__restrict__ mstart, const int32_t *__restrict__ mrows,
-                             int64_t nc, int64_t *__restrict__ bound) {
+__global__ void k_cand_bound(MatView A, const int32_t *mstart, const int32_t *mrows, int64_t nc, int64_t *bound) {
+    pdl_wait();
     const int64_t I = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (I >= nc) return;
     int64_t b = 0;
@@ -736,10 +750,10 @@ __global__ void k_cand_bound(MatView A, const int32_t *__restrict__ mstart, cons
 }
 
 // SELL layout of the compact rows: entries, then padding slots (own column, value 0)
-__global__ void k_sell_fill(int64_t n_pad, int64_t nc, const int64_t *__restrict__ c_off,
-                            const int32_t *__restrict__ rowlen, const int64_t *__restrict__ t_off,
-                            const int32_t *__restrict__ t_col, const float *__restrict__ t_val,
-                            int32_t *__restrict__ c_col, float *__restrict__ c_val) {
+__global__ void k_sell_fill(int64_t n_pad, int64_t nc, const int64_t *c_off, const int32_t *rowlen,
+                            const int64_t *t_off, const int32_t *t_col, const float *t_val, int32_t *c_col,
+                            float *c_val) {
+    pdl_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_pad) return;
     const int64_t sl = i / kS;
@@ -761,6 +775,7 @@ __global__ void k_sell_fill(int64_t n_pad, int64_t nc, const int64_t *__restrict
 
 // slots of each slice: 32 x the longest row among its real rows
 __global__ void k_slice_width(int64_t n_slices, int64_t nc, const int32_t *rowlen, int64_t *width) {
+    pdl_wait();
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n_slices) return;
     int32_t m = 0;
@@ -793,7 +808,8 @@ constexpr int kCoarseMin = 160;  // pairing passes go on down to this many rows
 constexpr int kGjB = 32, kGjTile = 64;
 
 // the n x n part of A in the np x np matrix M (zeroed before; identity in the padding)
-__global__ void k_dense_scatter(MatView A, int n, int np, double *__restrict__ M) {
+__global__ void k_dense_scatter(MatView A, int n, int np, double *M) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= np) return;
     if (i >= n) {
@@ -819,8 +835,8 @@ __device__ __forceinline__ double quick_rcp(double x) {
     return fma(r, fma(-x, r, 1.0), r);
 }
 
-__global__ void __launch_bounds__(256) k_gj_step(const double *__restrict__ src, double *__restrict__ dst, int np,
-                                                 int k, int32_t *flag) {
+__global__ void __launch_bounds__(256) k_gj_step(const double *src, double *dst, int np, int k, int32_t *flag) {
+    pdl_wait();
     __shared__ double D[kGjB][kGjB + 1], rowb[2][kGjB], colb[2][kGjB];
     __shared__ double Ai[kGjTile][kGjB + 1], P[kGjB][kGjTile];
     const int t = threadIdx.x, kb = k * kGjB;
@@ -926,7 +942,8 @@ __global__ void __launch_bounds__(256) k_gj_step(const double *__restrict__ src,
 }
 
 // the inverse in FP32, rows of ld entries (a multiple of 4; zeros past n)
-__global__ void k_dense_store(int n, int np, int ld, const double *__restrict__ M, float *__restrict__ inv) {
+__global__ void k_dense_store(int n, int np, int ld, const double *M, float *inv) {
+    pdl_wait();
     const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= (int64_t)n * ld) return;
     const int i = (int)(q / ld), j = (int)(q % ld);
@@ -1212,10 +1229,12 @@ __global__ void k_prolong(Gate gate, int64_t n, const int32_t *__restrict__ agg,
 
 // long-row list: flags (1 where rlen > kLongRow) for a scan, then the compacted row indices
 __global__ void k_flag_long(int64_t n, const int32_t *rlen, int32_t *flag) {
+    pdl_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) flag[i] = rlen[i] > kLongRow ? 1 : 0;
 }
 __global__ void k_compact_long(int64_t n, const int32_t *flag, const int32_t *pos, int32_t *list, int32_t *count) {
+    pdl_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) list[0] = *count = pos[n];
     if (i < n && flag[i]) list[1 + pos[i]] = (int32_t)i;
@@ -2284,9 +2303,10 @@ cudaError_t Amg::level_stats(AmgLevel &L, unsigned int *bound, cudaStream_t s) {
     AMG_CK(L.inv_diag.ensure(n));
     AMG_CK(isd_.ensure(n));
     const int g = split_of(L.A, opt_.split, opt_.split_width);
-    level_diag_kernel(g)<<<split_blocks(n, g), 256, 0, s>>>(view(L.A), L.inv_diag.p, isd_.p, bound);
+    launch_chained(true, level_diag_kernel(g), split_blocks(n, g), 256, s, view(L.A), L.inv_diag.p, isd_.p, bound);
     if (L.A.long_count)
-        k_level_diag_long<<<148, 256, 0, s>>>(view(L.A), L.A.long_count, L.inv_diag.p, isd_.p, bound);
+        launch_chained(true, k_level_diag_long, 148, 256, s, view(L.A), L.A.long_count, L.inv_diag.p, isd_.p,
+                       bound);
     AMG_CK(cudaGetLastError());
     return cudaSuccess;
 }
@@ -2295,6 +2315,7 @@ cudaError_t Amg::level_stats(AmgLevel &L, unsigned int *bound, cudaStream_t s) {
 // The power iteration's steps y = D^-1 A x are the cycle's row kernels (kRowPower).  The start vector is a fixed pseudo-random sign pattern of amplitude in [0.5, 1)
 // (no scaling between steps: |D^-1 A| <= a few, so 12 steps stay far from FP32 overflow).
 __global__ void k_power_start(int64_t n, float *x) {
+    pdl_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     uint32_t h = (uint32_t)i * 2654435761u;
@@ -2306,8 +2327,8 @@ __global__ void k_power_start(int64_t n, float *x) {
 
 // per-block partial sums of x.x and y.y (fixed grid, fixed tree: deterministic)
 constexpr int kPowerBlocks = 296;
-__global__ void __launch_bounds__(256) k_power_norms(int64_t n, const float *__restrict__ x, const float *__restrict__ y,
-                                                     double *__restrict__ part) {
+__global__ void __launch_bounds__(256) k_power_norms(int64_t n, const float *x, const float *y, double *part) {
+    pdl_wait();
     double sx = 0.0, sy = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         sx += (double)x[i] * x[i];
@@ -2362,7 +2383,8 @@ __global__ void __launch_bounds__(256) k_fine_bound(MatView A, const float *__re
 }
 
 // the totals of the partials, by one warp in a fixed order
-__global__ void k_power_total(const double *__restrict__ part, int nb, double *__restrict__ out) {
+__global__ void k_power_total(const double *part, int nb, double *out) {
+    pdl_wait();
     double a = 0.0, b = 0.0;
     for (int k = threadIdx.x; k < nb; k += 32) {
         a += part[2 * k];
@@ -2392,13 +2414,13 @@ cudaError_t Amg::pair_pass(const AmgMatrix &A, const float *isd, const int32_t *
     AMG_CK(agg.ensure(n));
     const unsigned g = nblk(n, 256);
     const int gw = split_of(A, opt_.split, opt_.split_width);
-    k_pair_init<<<g, 256, 0, s>>>(V, row_edge, isd, mate_.p);
+    launch_chained(true, k_pair_init, g, 256, s, V, row_edge, isd, mate_.p);
     for (int r = 0; r < opt_.pair_rounds; ++r) {
-        pair_want_kernel(gw)<<<split_blocks(n, gw), 256, 0, s>>>(V, isd, mate_.p, want_.p,
-                                                                  row_edge ? 0 : opt_.mix_coarse);
-        k_pair_match<<<g, 256, 0, s>>>(n, want_.p, mate_.p);
+        launch_chained(true, pair_want_kernel(gw), split_blocks(n, gw), 256, s, V, isd, mate_.p, want_.p,
+                       row_edge ? 0 : opt_.mix_coarse);
+        launch_chained(true, k_pair_match, g, 256, s, n, want_.p, mate_.p);
     }
-    k_pair_pack<<<g, 256, 0, s>>>(n, mate_.p, packed_.p);
+    launch_chained(true, k_pair_pack, g, 256, s, n, mate_.p, packed_.p);
     AMG_CK(cudaGetLastError());
     int64_t tot = 0;
     cudaError_t e = scan_i64(packed_.p, pscan_.p, n, tot, s);  // the one host read of the pass
@@ -2407,8 +2429,8 @@ cudaError_t Amg::pair_pass(const AmgMatrix &A, const float *isd, const int32_t *
     const int64_t members = tot >> 32;
     AMG_CK(mstart.ensure(nc + 1));
     AMG_CK(mrows.ensure(std::max<int64_t>(members, 1)));
-    k_pair_finish<<<std::max(g, 1u), 256, 0, s>>>(n, nc, members, mate_.p, packed_.p, pscan_.p, agg.p, mstart.p,
-                                                  mrows.p);
+    launch_chained(true, k_pair_finish, std::max(g, 1u), 256, s, n, nc, members, mate_.p, packed_.p, pscan_.p,
+                   agg.p, mstart.p, mrows.p);
     AMG_CK(cudaGetLastError());
     return cudaSuccess;
 }
@@ -2426,7 +2448,7 @@ cudaError_t Amg::galerkin(const AmgMatrix &A, const int32_t *agg, int64_t nc, co
     const MatView V = view(A);
     AMG_CK(tbound_.ensure(nc + 1));
     AMG_CK(toff_.ensure(nc + 1));
-    if (nc > 0) k_cand_bound<<<nblk(nc, 256), 256, 0, s>>>(V, mstart, mrows, nc, tbound_.p);
+    if (nc > 0) launch_chained(true, k_cand_bound, nblk(nc, 256), 256, s, V, mstart, mrows, nc, tbound_.p);
     AMG_CK(cudaGetLastError());
     cudaError_t e = scan_i64_dev(tbound_.p, toff_.p, nc, s);
     if (e != cudaSuccess) return e;
@@ -2451,14 +2473,14 @@ cudaError_t Amg::galerkin(const AmgMatrix &A, const int32_t *agg, int64_t nc, co
     k_galerkin<kGalCapBig, kGalWarpsBig, true><<<148 * 2, kGalWarpsBig * 32, big_smem, s>>>(
         V, agg, mstart, mrows, nc, rowlen_.p, toff_.p, tcol_.p, tval_.p, overflow_, wt, big_list_.p, big_count_.p);
     AMG_CK(cudaGetLastError());
-    k_slice_width<<<nblk(n_sl, 256), 256, 0, s>>>(n_sl, nc, rowlen_.p, width_.p);
+    launch_chained(true, k_slice_width, nblk(n_sl, 256), 256, s, n_sl, nc, rowlen_.p, width_.p);
     AMG_CK(cudaGetLastError());
     int64_t slots = 0;
     if ((e = scan_i64(width_.p, c_off.p, n_sl, slots, s)) != cudaSuccess) return e;
     AMG_CK(c_col.ensure(std::max<int64_t>(slots, 1)));
     AMG_CK(c_val.ensure(std::max<int64_t>(slots, 1)));
-    k_sell_fill<<<nblk(n_pad, 256), 256, 0, s>>>(n_pad, nc, c_off.p, rowlen_.p, toff_.p, tcol_.p, tval_.p, c_col.p,
-                                                  c_val.p);
+    launch_chained(true, k_sell_fill, nblk(n_pad, 256), 256, s, n_pad, nc, c_off.p, rowlen_.p, toff_.p, tcol_.p,
+                   tval_.p, c_col.p, c_val.p);
     AMG_CK(cudaGetLastError());
     C.n = n_pad;
     C.n_slices = n_sl;
@@ -2472,14 +2494,15 @@ cudaError_t Amg::galerkin(const AmgMatrix &A, const int32_t *agg, int64_t nc, co
     C.rlen = c_rlen.p;
     AMG_CK(lflag_.ensure(n_pad));
     AMG_CK(lpos_.ensure(n_pad + 1));
-    k_flag_long<<<nblk(n_pad, 256), 256, 0, s>>>(n_pad, c_rlen.p, lflag_.p);
+    launch_chained(true, k_flag_long, nblk(n_pad, 256), 256, s, n_pad, c_rlen.p, lflag_.p);
     AMG_CK(cudaGetLastError());
     cudaError_t e2 = scan_i32_dev(lflag_.p, lpos_.p, n_pad, s);
     if (e2 != cudaSuccess) return e2;
     // the list holds its count in front: [count, rows...]; the host reads the counts of all
     // levels at the end of the setup
     AMG_CK(c_long.ensure(n_pad + 1));
-    k_compact_long<<<nblk(n_pad, 256), 256, 0, s>>>(n_pad, lflag_.p, lpos_.p, c_long.p, long_words_ + level);
+    launch_chained(true, k_compact_long, nblk(n_pad, 256), 256, s, n_pad, lflag_.p, lpos_.p, c_long.p,
+                   long_words_ + level);
     AMG_CK(cudaGetLastError());
     C.longrows = c_long.p + 1;
     C.long_count = c_long.p;
@@ -2494,12 +2517,14 @@ cudaError_t Amg::dense_coarse(const AmgMatrix &A, cudaStream_t s) {
     AMG_CK(dense_inv_.ensure((size_t)n * ld));
     for (auto &w : dense_work_) AMG_CK(w.ensure((size_t)np * np));
     AMG_CK(cudaMemsetAsync(dense_work_[0].p, 0, (size_t)np * np * sizeof(double), s));
-    k_dense_scatter<<<nblk(np, 128), 128, 0, s>>>(view(A), n, np, dense_work_[0].p);
+    launch_chained(true, k_dense_scatter, nblk(np, 128), 128, s, view(A), n, np, dense_work_[0].p);
     const unsigned tiles = nblk(np, kGjTile);
     int from = 0;
     for (int k = 0; k < np / kGjB; ++k, from ^= 1)
-        k_gj_step<<<dim3(tiles, tiles), 256, 0, s>>>(dense_work_[from].p, dense_work_[from ^ 1].p, np, k, dense_flag_);
-    k_dense_store<<<nblk(n * ld, 256), 256, 0, s>>>(n, np, (int)ld, dense_work_[from].p, dense_inv_.p);
+        launch_chained(true, k_gj_step, dim3(tiles, tiles), 256, s, dense_work_[from].p, dense_work_[from ^ 1].p,
+                       np, k, dense_flag_);
+    launch_chained(true, k_dense_store, nblk(n * ld, 256), 256, s, n, np, (int)ld, dense_work_[from].p,
+                   dense_inv_.p);
     AMG_CK(cudaGetLastError());
     return cudaSuccess;
 }
@@ -2596,23 +2621,26 @@ cudaError_t Amg::setup(const DevSystem &sys, const AmgOptions &o, cudaStream_t s
             // (the intermediate matrix's bound is not needed: its own slot past the levels')
             unsigned int *mb = bounds_.p + o.max_levels;
             const int gm = split_of(M, opt_.split, opt_.split_width);
-            level_diag_kernel(gm)<<<split_blocks(M.n, gm), 256, 0, s>>>(view(M), mid_invd_.p, isd_.p, mb);
+            launch_chained(true, level_diag_kernel(gm), split_blocks(M.n, gm), 256, s, view(M), mid_invd_.p, isd_.p,
+                           mb);
             if (M.long_count)
-                k_level_diag_long<<<148, 256, 0, s>>>(view(M), M.long_count, mid_invd_.p, isd_.p, mb);
+                launch_chained(true, k_level_diag_long, 148, 256, s, view(M), M.long_count, mid_invd_.p, isd_.p,
+                               mb);
             AMG_CK(cudaGetLastError());
             int64_t np = 0;
             if ((e = pair_pass(M, isd_.p, nullptr, tmp_agg_, np, tmp_ms_, tmp_mr_, s)) != cudaSuccess) return e;
             // compose: agg = agg_p[agg], members of each new aggregate in order
             AMG_CK(cnt_.ensure(np + 1));
             AMG_CK(cid_.ensure(np + 1));
-            k_compose_agg<<<nblk(L.A.n, 256), 256, 0, s>>>(L.A.n, L.agg.p, tmp_agg_.p, L.agg.p);
-            k_compose_count<<<nblk(np, 256), 256, 0, s>>>(np, tmp_ms_.p, tmp_mr_.p, L.mem_start.p, cnt_.p);
+            launch_chained(true, k_compose_agg, nblk(L.A.n, 256), 256, s, L.A.n, L.agg.p, tmp_agg_.p, L.agg.p);
+            launch_chained(true, k_compose_count, nblk(np, 256), 256, s, np, tmp_ms_.p, tmp_mr_.p, L.mem_start.p,
+                           cnt_.p);
             AMG_CK(cudaGetLastError());
             // member offsets by a device-side scan; the member lists hold at most A_l's rows
             if ((e = scan_i32_dev(cnt_.p, cid_.p, np, s)) != cudaSuccess) return e;
             AMG_CK(want_.ensure(std::max<int64_t>(L.A.n, 1)));
-            k_compose_fill<<<nblk(np, 256), 256, 0, s>>>(np, tmp_ms_.p, tmp_mr_.p, L.mem_start.p, L.mem_rows.p, cid_.p,
-                                                         want_.p);
+            launch_chained(true, k_compose_fill, nblk(np, 256), 256, s, np, tmp_ms_.p, tmp_mr_.p, L.mem_start.p,
+                           L.mem_rows.p, cid_.p, want_.p);
             AMG_CK(cudaGetLastError());
             std::swap(L.mem_start, cid_);  // the composed lists become the level's
             std::swap(L.mem_rows, want_);
@@ -2766,17 +2794,17 @@ cudaError_t Amg::power_estimates(cudaStream_t s, int only_level) {
         // smoother's row weights
         const float *invd = l == 0 ? fw() : L.inv_diag.p;
         float *x = pw_a_.p, *y = pw_b_.p;
-        k_power_start<<<nblk(n, 256), 256, 0, s>>>(n, x);
+        launch_chained(true, k_power_start, nblk(n, 256), 256, s, n, x);
         for (int k = 0; k < opt_.power_steps; ++k) {
             RowArgs a = {};
             a.x = x;
             a.out = y;
             a.invd = invd;
-            launch_rows<kRowPower>(L, a, s, false);
+            launch_rows<kRowPower>(L, a, s, k > 0);
             if (k + 1 < opt_.power_steps) std::swap(x, y);
         }
-        k_power_norms<<<kPowerBlocks, 256, 0, s>>>(n, x, y, pw_part_.p);
-        k_power_total<<<1, 32, 0, s>>>(pw_part_.p, kPowerBlocks, pw_sums_.p + 2 * l);
+        launch_chained(true, k_power_norms, kPowerBlocks, 256, s, n, x, y, pw_part_.p);
+        launch_chained(true, k_power_total, 1, 32, s, pw_part_.p, kPowerBlocks, pw_sums_.p + 2 * l);
         AMG_CK(cudaGetLastError());
     }
     return cudaSuccess;
@@ -3227,8 +3255,8 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
         if (l == 0 && tma0)
             launch_fine<kFineResid>(n_done, n_inst, b, nullptr, xi, L.r.p, nullptr, 0.f, 0.f, 0.f, s);
         else if (l == 0 && half0)
-            launch_chained(chain(), k_fine<kOpResid, false, false>, gf, 256, s, gate_, F, b, nullptr, xi, L.r.p, nullptr,
-                           0.f, 0.f, 0.f);
+            launch_chained(chain(), k_fine<kOpResid, false, false>, gf, 256, s, gate_, F, b, nullptr, xi, L.r.p,
+                           nullptr, 0.f, 0.f, 0.f);
         else {
             RowArgs a = {};
             a.gate = gate_;
@@ -3246,8 +3274,8 @@ cudaError_t Amg::cycle(int l0, const float *r, float *z, const int32_t *n_done, 
                            L.mem_rows.p, L.r.p, wt, C.inv_diag.p, (float)cc2[0], C.b.p, C.xa.p,
                            use_tail && l + 1 == tail_level_ ? C.d.p : nullptr, C.agg.p);
         } else {
-            launch_chained(chain(), k_restrict, nblk(C.A.n, 256), 256, s, gate_, L.nc, C.A.n, L.mem_start.p, L.mem_rows.p,
-                           L.r.p, C.b.p, wt);
+            launch_chained(chain(), k_restrict, nblk(C.A.n, 256), 256, s, gate_, L.nc, C.A.n, L.mem_start.p,
+                           L.mem_rows.p, L.r.p, C.b.p, wt);
         }
     }
     // coarsest: dense inverse, or (when coarsening stalled above the dense limit) a Chebyshev
