@@ -792,11 +792,14 @@ __global__ void k_slice_width(int64_t n_slices, int64_t nc, const int32_t *rowle
 // pivoting (it is SPD), blocks of 32, one launch per block step over 64 x 64 tiles of the padded
 // matrix, reading one copy and writing the other.  In step k, with D = A_kk^-1 and P = D A_k. (P_k
 // = D in block column k): row block k becomes P, the other rows A_i. - A_ik P (0 for A_ik in block
-// column k).  Every block inverts A_kk itself (32 pivots) and forms P for its columns, so a step
-// needs nothing from another block of the same launch.  flag = 1 on a non-positive or non-finite
-// pivot.
+// column k).  Every block forms P for its columns, so a step needs nothing from another block of the
+// same launch.  D comes from the launch before: the block that updates A_kk goes on to invert it (32
+// pivots in a row, the longest chain of a step, which would otherwise stand in front of every block's
+// work).  flag = 1 on a non-positive or non-finite pivot.
 // Measured (B200): the inverse of 130 rows 360 us by one block with the matrix in shared memory;
-// here 15 us a step at 477 rows (0.23 ms), 27 at 1120 (0.95 ms).
+// with every block inverting A_kk itself 15 us a step at 477 rows (0.23 ms), 27 at 1120 (0.95 ms); with D
+// from the launch before 15 and 17 (the chain of one block's update and 32 pivots; at 1120 rows
+// also the shared-memory reads of the update, three tiles to an SM).
 // kDenseMax: the limit was 160, what one SM's shared memory held.  An exact solve this high up
 // replaces one to three levels of seven latency-bound kernels each, in every cycle and in the setup,
 // and converges faster: n = 21 (1120 rows) 57 iterations of 145 us -> 40 of 113, n = 64 (847 rows)
@@ -835,25 +838,11 @@ __device__ __forceinline__ double quick_rcp(double x) {
     return fma(r, fma(-x, r, 1.0), r);
 }
 
-__global__ void __launch_bounds__(256) k_gj_step(const double *src, double *dst, int np, int k, int32_t *flag) {
-    pdl_wait();
-    __shared__ double D[kGjB][kGjB + 1], rowb[2][kGjB], colb[2][kGjB];
-    __shared__ double Ai[kGjTile][kGjB + 1], P[kGjB][kGjTile];
-    const int t = threadIdx.x, kb = k * kGjB;
-    const int i0 = blockIdx.y * kGjTile, j0 = blockIdx.x * kGjTile;
-    auto at = [&](int r, int c) { return r < np && c < np ? src[(size_t)r * np + c] : 0.0; };
-    // A_ik and A_kj are on their way while A_kk is inverted
-    for (int q = t; q < kGjTile * kGjB; q += 256) {
-        Ai[q / kGjB][q % kGjB] = at(i0 + q / kGjB, kb + q % kGjB);
-        P[q / kGjTile][q % kGjTile] = at(kb + q / kGjTile, j0 + q % kGjTile);
-    }
-    // D: thread t holds four entries of row r
-    const int r = t >> 3, c4 = (t & 7) * 4;
-    double m[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) m[q] = src[(size_t)(kb + r) * np + kb + c4 + q];
-    // pivot p: with a 1 in the pivot's place of row p, zeros left behind in row p and column p, and
-    // the factor -1 for row p, every entry is m -= f / pivot * row_p
+// The inverse of a 32 x 32 block by the 256 threads of a block: thread t holds m, four entries of
+// row r = t / 8 from column c4 = 4 (t % 8) on.  Pivot p: with a 1 in the pivot's place of row p, zeros
+// left behind in row p and column p, and the factor -1 for row p, every entry is m -= f / pivot * row_p.
+__device__ __forceinline__ void gj_invert(double (&m)[4], int r, int c4, double (*rowb)[kGjB], double (*colb)[kGjB],
+                                          int32_t *flag) {
     bool bad = false;
 #pragma unroll 1
     for (int p0 = 0; p0 < kGjB; p0 += 4) {
@@ -880,9 +869,36 @@ __global__ void __launch_bounds__(256) k_gj_step(const double *src, double *dst,
             for (int q = 0; q < 4; ++q) m[q] = fma(-g, rb[c4 + q], m[q]);
         }
     }
-    if (bad && t == 0) *flag = 1;
+    if (bad && r == 0 && c4 == 0) *flag = 1;
+}
+
+// D of the first step
+__global__ void __launch_bounds__(256) k_gj_first(const double *M, int np, double *dinv, int32_t *flag) {
+    pdl_wait();
+    __shared__ double rowb[2][kGjB], colb[2][kGjB];
+    const int r = threadIdx.x >> 3, c4 = (threadIdx.x & 7) * 4;
+    double m[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) D[r][c4 + q] = m[q];
+    for (int q = 0; q < 4; ++q) m[q] = M[(size_t)r * np + c4 + q];
+    gj_invert(m, r, c4, rowb, colb, flag);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) dinv[r * kGjB + c4 + q] = m[q];
+}
+
+// dinv: D of this step; dinv_next: of the next one, written by the block that holds it
+__global__ void __launch_bounds__(256) k_gj_step(const double *src, double *dst, int np, int k, const double *dinv,
+                                                 double *dinv_next, int32_t *flag) {
+    pdl_wait();
+    __shared__ double D[kGjB][kGjB + 1], rowb[2][kGjB], colb[2][kGjB];
+    __shared__ double Ai[kGjTile][kGjB + 1], P[kGjB][kGjTile];
+    const int t = threadIdx.x, kb = k * kGjB;
+    const int i0 = blockIdx.y * kGjTile, j0 = blockIdx.x * kGjTile;
+    auto at = [&](int r, int c) { return r < np && c < np ? src[(size_t)r * np + c] : 0.0; };
+    for (int q = t; q < kGjTile * kGjB; q += 256) {
+        Ai[q / kGjB][q % kGjB] = at(i0 + q / kGjB, kb + q % kGjB);
+        P[q / kGjTile][q % kGjTile] = at(kb + q / kGjTile, j0 + q % kGjTile);
+    }
+    for (int q = t; q < kGjB * kGjB; q += 256) D[q / kGjB][q % kGjB] = dinv[q];
     __syncthreads();
     // P = D A_kj (D itself in block column k): thread t takes column j and 8 of the 32 rows
     {
@@ -935,10 +951,22 @@ __global__ void __launch_bounds__(256) k_gj_step(const double *src, double *dst,
             const int j = j0 + tx + 16 * b;
             if (j >= np) continue;
             const bool in_r = i >= kb && i < kb + kGjB, in_c = j >= kb && j < kb + kGjB;
-            dst[(size_t)i * np + j] =
-                in_r ? P[i - kb][j - j0] : (in_c ? 0.0 : src[(size_t)i * np + j]) - acc[a][b];
+            const double v = in_r ? P[i - kb][j - j0] : (in_c ? 0.0 : src[(size_t)i * np + j]) - acc[a][b];
+            dst[(size_t)i * np + j] = v;
+            const int r = i - kb - kGjB, c = j - kb - kGjB;  // in the next step's A_kk
+            if (r >= 0 && r < kGjB && c >= 0 && c < kGjB) D[r][c] = v;
         }
     }
+    const int kn = kb + kGjB;
+    if (kn >= np || kn < i0 || kn >= i0 + kGjTile || i0 != j0) return;
+    __syncthreads();
+    const int r = t >> 3, c4 = (t & 7) * 4;
+    double m[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) m[q] = D[r][c4 + q];
+    gj_invert(m, r, c4, rowb, colb, flag);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) dinv_next[r * kGjB + c4 + q] = m[q];
 }
 
 // the inverse in FP32, rows of ld entries (a multiple of 4; zeros past n)
@@ -2259,6 +2287,7 @@ void Amg::release() {
     isd_.release();
     dense_inv_.release();
     for (auto &w : dense_work_) w.release();
+    dense_pivot_.release();
     bound_.release();
     tail_prog_.release();
     tail_levels_.release();
@@ -2519,10 +2548,13 @@ cudaError_t Amg::dense_coarse(const AmgMatrix &A, cudaStream_t s) {
     AMG_CK(cudaMemsetAsync(dense_work_[0].p, 0, (size_t)np * np * sizeof(double), s));
     launch_chained(true, k_dense_scatter, nblk(np, 128), 128, s, view(A), n, np, dense_work_[0].p);
     const unsigned tiles = nblk(np, kGjTile);
+    AMG_CK(dense_pivot_.ensure(2 * kGjB * kGjB));
+    double *const dinv[2] = {dense_pivot_.p, dense_pivot_.p + kGjB * kGjB};
+    launch_chained(true, k_gj_first, 1, 256, s, dense_work_[0].p, np, dinv[0], dense_flag_);
     int from = 0;
     for (int k = 0; k < np / kGjB; ++k, from ^= 1)
         launch_chained(true, k_gj_step, dim3(tiles, tiles), 256, s, dense_work_[from].p, dense_work_[from ^ 1].p,
-                       np, k, dense_flag_);
+                       np, k, dinv[from], dinv[from ^ 1], dense_flag_);
     launch_chained(true, k_dense_store, nblk(n * ld, 256), 256, s, n, np, (int)ld, dense_work_[from].p,
                    dense_inv_.p);
     AMG_CK(cudaGetLastError());

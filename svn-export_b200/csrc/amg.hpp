@@ -204,7 +204,7 @@ private:
     std::vector<int64_t> dots_long_off_;
     DBuf<float> isd_;
     DBuf<float> dense_inv_;         // inverse of the coarsest matrix, and the two copies it is made in
-    DBuf<double> dense_work_[2];
+    DBuf<double> dense_work_[2], dense_pivot_;
     DBuf<int32_t> flag_;
     DBuf<unsigned int> bound_;
     DBuf<double> dots_, alpha_;     // coarse-correction scaling: partials, factor per level
