@@ -243,12 +243,13 @@ __global__ void __launch_bounds__(kBlockThreads)
 // ---- Chebyshev-Jacobi polynomial preconditioner z = P_d(S^) r on [lo, hi] ---------------
 // step 0: d = r / theta, z = d;  step k: d = c1 d + c2 (r - S^ z_prev), z = z_prev + d.
 __global__ void __launch_bounds__(kBlockThreads)
-    k_cheb_step(SellView<float> A, const float *__restrict__ r, const float *__restrict__ z_prev,
-                float *__restrict__ z_next, float *__restrict__ d, double c1, double c2, int first,
-                const InstCtl *__restrict__ ctl, Plan plan) {
-    if (ctl[plan.inst[blockIdx.x]].done) return;
+    k_cheb_step(SellView<float> A, const float *r, const float *z_prev, float *z_next, float *d, double c1, double c2,
+                int first, const InstCtl *ctl, Plan plan) {
+    const int inst = plan.inst[blockIdx.x], tb = plan.tile_begin[blockIdx.x], te = plan.tile_end[blockIdx.x];
+    pdl_wait();
+    if (ctl[inst].done) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int tile = plan.tile_begin[blockIdx.x]; tile < plan.tile_end[blockIdx.x]; ++tile) {
+    for (int tile = tb; tile < te; ++tile) {
         const int64_t sl = (int64_t)tile * kWarpsPerBlock + warp;
         const int64_t row = sl * kSliceRows + lane;
         float zn;
@@ -319,7 +320,7 @@ inline unsigned blocks_for(int64_t n, int th) { return (unsigned)((n + th - 1) /
 }  // namespace
 
 cudaError_t launch_cheb_apply(const DevSystem &sys, const float *r, float *z0, float *z1, float *d, float *z_final,
-                              int degree, double lo, double hi, cudaStream_t s) {
+                              int degree, double lo, double hi, cudaStream_t s, bool follows) {
     if (sys.rows_per_thread != 1) return cudaErrorInvalidValue;  // tiles of 256 rows
     const SellView<float> A = {sys.n_rows, sys.slice_off, sys.col, sys.val32};
     const unsigned g = (unsigned)sys.plan[1].n_blocks;
@@ -337,7 +338,8 @@ cudaError_t launch_cheb_apply(const DevSystem &sys, const float *r, float *z0, f
         }
         const bool last = k == degree - 1;
         float *zn = last ? z_final : ((k % 2 == 0) ? z0 : z1);
-        k_cheb_step<<<g, kBlockThreads, 0, s>>>(A, r, zp, zn, d, c1, c2, k == 0 ? 1 : 0, sys.ctl, p);
+        launch_chained(follows || k > 0, k_cheb_step, g, kBlockThreads, s, A, r, zp, zn, d, c1, c2, k == 0 ? 1 : 0,
+                       sys.ctl, p);
         zp = zn;
     }
     return cudaGetLastError();

@@ -9,7 +9,7 @@
 namespace mh {
 
 cudaError_t launch_cheb_apply(const DevSystem &sys, const float *r, float *z0, float *z1, float *d, float *z_final,
-                              int degree, double lo, double hi, cudaStream_t s);
+                              int degree, double lo, double hi, cudaStream_t s, bool follows);
 // the rest of a flexible-CG iteration after z = M r (two kernels)
 cudaError_t launch_fcg_iteration(const DevSystem &sys, const float *z, cudaStream_t s, bool chained);
 cudaError_t launch_spectrum_bound(const DevSystem &sys, unsigned int *out, cudaStream_t s);

@@ -956,7 +956,8 @@ cudaError_t fcg_iteration(mh_handle *h, Pc kind, int degree, double lo, double h
     cudaError_t e;
     switch (kind) {
         case Pc::Cheb:
-            e = mh::launch_cheb_apply(sys, sys.r32, h->cheb_z0, h->cheb_z1, h->cheb_d, sys.z32, degree, lo, hi, s);
+            e = mh::launch_cheb_apply(sys, sys.r32, h->cheb_z0, h->cheb_z1, h->cheb_d, sys.z32, degree, lo, hi, s,
+                                      follows);
             break;
         default:
             e = h->amg.apply(sys.r32, sys.z32, sys.n_done, sys.n_inst, s, prof, follows);

@@ -5,6 +5,9 @@
 // -> with): 52k edges 83 -> 66, 115k 93 -> 78, 404k 151 -> 137, 1.35M 288 -> 243, 3.2M 498 -> 456,
 // 11M 2025 -> 1940.  Letting the next kernel come up behind the wait instead of before it gave 67, 78, 138,
 // 247, 460, 1946; at the kernel's very start 67, 80, 139, 245, 459, 1942.
+// The Chebyshev polynomial's steps: 28 -> 23 us an iteration (13k edges), 44 -> 38 (175k), 83 -> 73 (404k).
+// Not the two kernels of plain CG: 65.4 -> 61.7 ms for a batch of four small systems, but 32.8 -> 34.1 us an
+// iteration at 1.1M edges and 57.9 -> 59.9 (FP32) at 3.2M.
 // The multigrid setup's small kernels are chained too, with nothing read ahead: 1.93 -> 1.62 ms (52k
 // edges), 5.66 -> 5.16 (1.35M), 7.2 -> 6.6 (3.2M), 24.6 -> 23.3 (11M).
 #pragma once
