@@ -176,14 +176,16 @@ def algorithmic_bytes(kernel, N, Z):
     """Bytes each launch must move at minimum (every array once; no padding, no re-reads).
     spmv:    values + column indices of the Z nonzeros, p (gathered, counted once), r read, q written.
     update:  x, r, p read and written, q read.
-    smooth0: AMG Chebyshev step on the fine level (unit diagonal): values (FP16 copy, or FP32)
-             + indices, x (or b) gathered, b read, x and d written; d read by the steps that
-             continue a sequence (the fused first pre-smoothing pass and the first post-smoothing
-             step start one): mean over the 2d-1 fine steps of one cycle."""
+    smooth0: AMG Chebyshev step on the fine level (unit diagonal, not read): values (FP16 copy, or
+             FP32) + indices of the off-diagonals, x and b read, x written (the fused first pass:
+             b read, x written); d read by the steps that continue a sequence, written by those
+             that another one continues: mean over the 2d-1 fine steps of one cycle."""
     if kernel == "smooth0":
-        steps = 2 * AMG_DEGREE - 1
-        reads_d = max(0, AMG_DEGREE - 2) + (AMG_DEGREE - 1)
-        return Z * (4 + AMG_VALUE_BYTES) + 16 * N + 4 * N * reads_d / steps
+        d = AMG_DEGREE
+        vec = 2 + (d > 2)  # the first pass: two steps
+        vec += sum(3 + 1 + (k + 1 < d) for k in range(2, d))  # the other pre-smoothing steps
+        vec += sum(3 + (k > 0) + (k + 1 < d) for k in range(d))  # post-smoothing
+        return (Z - N) * (4 + AMG_VALUE_BYTES) + 4 * N * vec / (2 * d - 1)
     s = 8 if kernel.endswith("64") else 4
     if kernel.startswith("spmv"):
         return Z * (s + 4) + 3 * s * N
@@ -191,7 +193,7 @@ def algorithmic_bytes(kernel, N, Z):
 
 
 KERNEL_NAMES = {"spmv64": "k_cg_spmv<double>", "update64": "k_cg_update<double>", "spmv32": "k_cg_spmv<float>",
-                "update32": "k_cg_update<float>", "smooth0": "k_sm_step (AMG fine level)"}
+                "update32": "k_cg_update<float>", "smooth0": "k_fine (AMG fine level)"}
 
 
 def roofline(stats_list, N, Z, peaks):
