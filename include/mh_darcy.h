@@ -122,7 +122,8 @@ typedef struct mh_bc {
 typedef struct mh_solve_opts {
     int32_t method;         /* MH_SOLVER_*                                          */
     int32_t max_it;         /* cap on (inner) iterations, default 20000              */
-    double  r_tol;          /* relative tolerance (default 1e-10)                    */
+    double  r_tol;          /* relative tolerance (default 1e-10); at 1.8e-15 and below the
+                               multigrid methods end a decimal under it where FP64 can */
     double  a_tol;          /* absolute tolerance on |b - S x| (default 0)           */
     int32_t use_initial_guess;  /* start from the current edge pressures             */
     int32_t cheb_degree;    /* MH_SOLVER_CHEB: polynomial degree (default 4)         */

@@ -139,6 +139,7 @@ struct mh_handle {
     float *pair_r = nullptr, *pair_e = nullptr;  // training pairs, [cap][n_rows] each
     int pair_cap = 0;
     double *x_star = nullptr, *pair_acc = nullptr;
+    double *x_keep = nullptr;  // the solution before a segment that may be undone (polish)
     std::string err;
 };
 
@@ -1210,6 +1211,73 @@ int prepare_multigrid(mh_handle *h, Pc kind, double &ms_setup) {
 // kFallbackSegment iterations.
 constexpr int kFallbackSegment = 200;
 
+// One FP32 segment: flexible CG on S^ d = r / |r| for the instances that `sums` marks active, until
+// the residual is down by `rtol`, and x += |r| d.  fresh: a new direction sequence.
+int fcg_segment(mh_handle *h, const mh_solve_opts &o, Pc kind, int degree, double hi, const std::vector<double> &sums,
+                double rtol, int seg_max, bool fresh, std::vector<mh::InstCtl> &ctl) {
+    CK(cudaMemcpyAsync(h->sys.inst_sums, sums.data(), sizeof(double) * sums.size(), cudaMemcpyHostToDevice, h->stream));
+    CK(mh::launch_reset_ctl(h->sys, h->stream));
+    if (fresh)
+        CK(mh::launch_ir_start(h->sys, rtol * rtol, seg_max, h->stream));
+    else
+        CK(mh::launch_ir_continue(h->sys, rtol * rtol, seg_max, h->stream));
+    int rc = run_fcg(h, kind, degree, hi / 30.0, hi, o.iters_per_graph, seg_max, o.profile_kernels != 0);
+    if (rc) return rc;
+    CK(mh::launch_ir_correct(h->sys, h->stream));
+    h->n_launch += 2;
+    return read_ctl(h, ctl);
+}
+
+int most_iterations(const std::vector<mh::InstCtl> &ctl) {
+    int most = 0;
+    for (auto &c : ctl) most = std::max(most, c.iter);
+    return most;
+}
+
+// A tolerance of the order of the FP64 rounding asks for the pressures as exactly as they come; side
+// fluxes are differences of them and lose three to four more decimals.  A multigrid segment lowers the
+// residual by about 1e-3, so a solve to 1e-15 ends anywhere between r_tol and a hundredth of it, far
+// above what FP64 can reach (1e-18 of the right-hand side on 3.2M edges): flux vectors were off by 6e-8
+// (largest difference over the RMS) where it ended at 0.3-0.46 r_tol, and by 1e-8 at most below 0.1.
+// Such a solve ends a decimal below r_tol: an instance above that gets one more short segment, which
+// is undone if it does not lower the residual (FP64 rounding reached first).
+constexpr double kRoundingTol = 8.0 * std::numeric_limits<double>::epsilon();
+constexpr double kRoundingShare = 0.1;
+
+int polish(mh_handle *h, const mh_solve_opts &o, SolveResult &res, Pc kind, int degree, double hi,
+           std::vector<double> &sums, double worst) {
+    const int seg_max = std::min(o.inner_max_it, o.max_it - res.iterations);
+    const size_t bytes = (size_t)h->sys.n_rows * sizeof(double);
+    if (seg_max <= 0) return MH_OK;
+    if (!h->x_keep && !(h->x_keep = dalloc<double>(h, h->sys.n_rows))) {
+        cudaGetLastError();
+        return MH_OK;
+    }
+    const std::vector<int32_t> status = h->inst_status;
+    const std::vector<double> rel = h->inst_rel;
+    const SolveResult before = res;
+    mh_solve_opts tight = o;
+    tight.r_tol *= kRoundingShare;
+    bool finite;
+    evaluate(h, tight, sums, res, finite);  // marks the instances above
+    CK(cudaMemcpyAsync(h->x_keep, h->sys.x, bytes, cudaMemcpyDeviceToDevice, h->stream));
+    std::vector<mh::InstCtl> ctl;
+    int rc = fcg_segment(h, o, kind, degree, hi, sums, kRoundingShare, seg_max, false, ctl);
+    if (rc || (rc = true_residual(h, sums))) return rc;
+    for (size_t i = 0; i < ctl.size(); ++i) h->inst_iters[i] += ctl[i].iter;
+    h->inst_status = status;
+    const double now = evaluate(h, o, sums, res, finite);
+    if (!finite || !(now < worst)) {
+        CK(cudaMemcpyAsync(h->sys.x, h->x_keep, bytes, cudaMemcpyDeviceToDevice, h->stream));
+        h->inst_status = status;
+        h->inst_rel = rel;
+        res = before;
+    }
+    res.iterations = before.iterations + most_iterations(ctl);
+    res.outer = before.outer + 1;
+    return MH_OK;
+}
+
 int solve_fcg(mh_handle *h, const mh_solve_opts &o, SolveResult &res, Pc kind) {
     int rc = ensure_learned(h);
     if (rc) return rc;
@@ -1242,7 +1310,12 @@ int solve_fcg(mh_handle *h, const mh_solve_opts &o, SolveResult &res, Pc kind) {
         }
         res.outer = outer;
         res.iterations = total;
-        if (worst_ratio <= 1.0) return MH_OK;
+        if (worst_ratio <= 1.0) {
+            const bool multigrid = learned ? use_nn : kind == Pc::Amg;
+            if (outer > 0 && multigrid && o.r_tol <= kRoundingTol && worst_ratio > kRoundingShare)
+                return polish(h, o, res, kind, degree, hi, sums, worst_ratio);
+            return MH_OK;
+        }
         if (total >= o.max_it) {
             res.status = MH_NOT_CONVERGED;
             return MH_OK;
@@ -1263,33 +1336,20 @@ int solve_fcg(mh_handle *h, const mh_solve_opts &o, SolveResult &res, Pc kind) {
                 return MH_OK;
             }
         }
-        CK(cudaMemcpyAsync(h->sys.inst_sums, sums.data(), sizeof(double) * sums.size(), cudaMemcpyHostToDevice,
-                           h->stream));
-        CK(mh::launch_reset_ctl(h->sys, h->stream));
         // a fallback gets segments long enough to make progress whatever limit the learned
         // method was given
         const int seg_lim = learned && !use_nn ? std::max(o.inner_max_it, kFallbackSegment) : o.inner_max_it;
         const int seg_max = std::min(seg_lim, o.max_it - total);
-        // the direction sequence continues across replacements unless the preconditioner changed
-        if (outer == 0 || restart)
-            CK(mh::launch_ir_start(h->sys, o.inner_rtol * o.inner_rtol, seg_max, h->stream));
-        else
-            CK(mh::launch_ir_continue(h->sys, o.inner_rtol * o.inner_rtol, seg_max, h->stream));
-        restart = false;
         const Pc cur = learned ? (use_nn ? Pc::Nn : Pc::Cheb) : kind;
         if (cur == Pc::Cheb && hi == 0.0 && (rc = spectrum_bound(h, hi))) return rc;
-        if ((rc = run_fcg(h, cur, degree, hi / 30.0, hi, o.iters_per_graph, seg_max, o.profile_kernels != 0))) return rc;
-        CK(mh::launch_ir_correct(h->sys, h->stream));
-        h->n_launch += 2;
-        if ((rc = read_ctl(h, ctl))) return rc;
+        // the direction sequence continues across replacements unless the preconditioner changed
+        if ((rc = fcg_segment(h, o, cur, degree, hi, sums, o.inner_rtol, seg_max, outer == 0 || restart, ctl))) return rc;
+        restart = false;
         count_iterations(h, ctl);
-        int maxit = 0;
         bool seg_bad = false;  // an instance broke down or used up the segment's iterations
-        for (auto &c : ctl) {
-            maxit = std::max(maxit, c.iter);
+        for (auto &c : ctl)
             if (c.status != 0) seg_bad = true;
-        }
-        total += maxit;
+        total += most_iterations(ctl);
         if (seg_bad && use_nn) {
             use_nn = false;
             res.fell_back = 1;
