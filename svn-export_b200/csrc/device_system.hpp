@@ -71,9 +71,10 @@ struct DevSystem {
     double *b = nullptr;             // rhs (original scaling)
     double *bh = nullptr;            // D^-1/2 b
     // FP64 Krylov vectors (scaled space)
-    double *x = nullptr, *r = nullptr, *p = nullptr, *q = nullptr;
+    double *x = nullptr, *r = nullptr, *p = nullptr, *q = nullptr;  // (p, q: flexible CG's too)
+    double *s = nullptr;             // S^ z of flexible CG
     // FP32 inner vectors
-    float *x32 = nullptr, *r32 = nullptr, *p32 = nullptr, *q32 = nullptr, *z32 = nullptr, *s32 = nullptr;
+    float *x32 = nullptr, *r32 = nullptr, *p32 = nullptr, *q32 = nullptr, *z32 = nullptr;
     double *partial = nullptr;       // [max plan blocks * 4]
     InstCtl *ctl = nullptr;          // [n_inst]
     int32_t *n_done = nullptr;       // instances finished in the current Krylov run

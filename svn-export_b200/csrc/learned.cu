@@ -98,20 +98,23 @@ __device__ __forceinline__ float sell_row_dot(const SellView<float> &A, const fl
 //                 the last block forms beta = z.q / p.q, the new direction's p.r = z.r - beta p.r and
 //                 p.q = z.s - beta z.q (S^ is symmetric and z.S^ p = z.q), alpha = p.r / p.q;
 //   k_fcg_update: p = z - beta p, q = s - beta q, x += alpha p, r -= alpha q, r.r, stopping test.
-// q follows the direction's recurrence instead of a product with the new p: the same to a rounding
-// in FP32, and the FP64 residual at the end of the run does not use it.
-// Both move the bytes that the four did (60 a row and the matrix); the row entries go four to a
-// load in the update and are loaded a tile ahead with the slots in the product.
+// q follows the direction's recurrence instead of a product with the new p, so what p, q and s are
+// rounded to stays in q for the rest of the run: the three are FP64 (z, x and r are FP32).
+// Residual after one segment of 800 iterations (158k rows, recursion at 1.2e-8): 6.0e-8 with q a product of
+// FP32 vectors, 7.4e-8 with the recurrence in FP32, 5.9e-8 in FP64.  The row entries go two to a load in the
+// update; z and r are loaded a tile ahead with the slots in the product, p and q beside the gathers.
 // The blocks of an instance take its tiles in turn (solver.cu, Tiles).
 // Measured (B200, us an iteration without the preconditioner, four kernels over neighbouring tiles
-// -> these): 52k rows 20 -> 11, 3.2M 96 -> 68, 10.9M 381 -> 233 (the update at 6.3 TB/s).
+// -> two with all vectors FP32): 52k rows 20 -> 11, 3.2M 96 -> 68, 10.9M 381 -> 233.  The FP64 ones are 32
+// bytes a row more; a multigrid iteration with them, against all FP32: 67.0 us and 66.7 (52k edges), 119.4 and
+// 118.4 (405k), 251 and 246 (1.35M), 471 and 458 (3.2M), 2075 and 2019 (11M).
 struct FcgStage {
     static constexpr int kJ = 6;
     int64_t off;
     int w;
     int32_t c[kJ];
     float v[kJ];
-    float dg, z, r, p, q;
+    float dg, z, r;
 };
 
 __device__ __forceinline__ void fcg_stage_load(const SellView<float> &A, int tile, FcgStage &st) {
@@ -128,17 +131,14 @@ __device__ __forceinline__ void fcg_stage_load(const SellView<float> &A, int til
         st.v[j] = in ? __ldcs(A.val + slot) : 0.f;
     }
 }
-__device__ __forceinline__ void fcg_stage_load_vec(const float *z, const float *r, const float *p, const float *q,
-                                                   bool have, int tile, FcgStage &st) {
+__device__ __forceinline__ void fcg_stage_load_vec(const float *z, const float *r, int tile, FcgStage &st) {
     const int64_t row = ((int64_t)tile * kWarpsPerBlock + (threadIdx.x >> 5)) * kSliceRows + (threadIdx.x & 31);
     st.z = z[row];
     st.r = r[row];
-    st.p = have ? p[row] : 0.f;
-    st.q = have ? q[row] : 0.f;
 }
 
 __global__ void __launch_bounds__(kBlockThreads, 4)
-    k_fcg_spmv(SellView<float> A, const float *z, const float *r, const float *p, const float *q, float *s,
+    k_fcg_spmv(SellView<float> A, const float *z, const float *r, const double *p, const double *q, double *s,
                double *partial, InstCtl *ctl, Plan plan, int32_t *n_done) {
     const int inst = plan.inst[blockIdx.x];
     InstCtl *c = ctl + inst;
@@ -153,15 +153,17 @@ __global__ void __launch_bounds__(kBlockThreads, 4)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int kJ = FcgStage::kJ;
     Sums<4> t = {{0.0, 0.0, 0.0, 0.0}};
-    if (tb < te) fcg_stage_load_vec(z, r, p, q, have, tb, st);
+    if (tb < te) fcg_stage_load_vec(z, r, tb, st);
     for (int tile = tb; tile < te; tile += nb) {
         float g[kJ];
 #pragma unroll
         for (int j = 0; j < kJ; ++j) g[j] = z[st.c[j]];
+        const int64_t row = ((int64_t)tile * kWarpsPerBlock + warp) * kSliceRows + lane;
+        const double pv = have ? p[row] : 0.0, qv = have ? q[row] : 0.0;
         const FcgStage cur = st;
         if (tile + nb < te) {
             fcg_stage_load(A, tile + nb, st);
-            fcg_stage_load_vec(z, r, p, q, have, tile + nb, st);
+            fcg_stage_load_vec(z, r, tile + nb, st);
         }
         double y = (double)cur.dg * (double)cur.z;
 #pragma unroll
@@ -170,10 +172,10 @@ __global__ void __launch_bounds__(kBlockThreads, 4)
             const int64_t slot = cur.off + (int64_t)j * kSliceRows + lane;
             y += (double)__ldcs(A.val + slot) * (double)z[__ldcs(A.col + slot)];
         }
-        s[((int64_t)tile * kWarpsPerBlock + warp) * kSliceRows + lane] = (float)y;
-        t.v[0] += (double)cur.z * (double)cur.q;
+        s[row] = y;
+        t.v[0] += (double)cur.z * qv;
         t.v[1] += (double)cur.z * (double)cur.r;
-        t.v[2] += (double)cur.p * (double)cur.r;
+        t.v[2] += pv * (double)cur.r;
         t.v[3] += (double)cur.z * y;
     }
     Sums<4> tot;
@@ -192,7 +194,7 @@ __global__ void __launch_bounds__(kBlockThreads, 4)
 }
 
 __global__ void __launch_bounds__(kBlockThreads)
-    k_fcg_update(float4 *x, float4 *r, float4 *p, float4 *q, const float4 *z, const float4 *s, double *partial,
+    k_fcg_update(float2 *x, float2 *r, double2 *p, double2 *q, const float2 *z, const double2 *s, double *partial,
                  InstCtl *ctl, Plan plan, int32_t *n_done) {
     const int inst = plan.inst[blockIdx.x];
     InstCtl *c = ctl + inst;
@@ -203,25 +205,25 @@ __global__ void __launch_bounds__(kBlockThreads)
     const double alpha = c->alpha, beta = c->beta;
     double rr = 0.0;
     // beta = 0 starts a new direction sequence: p and q are not used (they may hold a broken one)
-    auto dir = [&](float a, float b) { return beta == 0.0 ? a : (float)((double)a - beta * (double)b); };
-    auto one = [&](float zv, float sv, float &pv, float &qv, float &xv, float &rv) {
-        pv = dir(zv, pv);
+    auto dir = [&](double a, double b) { return beta == 0.0 ? a : a - beta * b; };
+    auto one = [&](float zv, double sv, double &pv, double &qv, float &xv, float &rv) {
+        pv = dir((double)zv, pv);
         qv = dir(sv, qv);
-        xv = (float)((double)xv + alpha * (double)pv);
-        rv = (float)((double)rv - alpha * (double)qv);
+        xv = (float)((double)xv + alpha * pv);
+        rv = (float)((double)rv - alpha * qv);
         rr += (double)rv * (double)rv;
     };
-    // four rows a thread and turn: four tiles at a time of the instance's run, the blocks in turn
-    constexpr int64_t kPer = kBlockThreads / 4;
+    // two rows a thread and turn: two tiles at a time of the instance's run, the blocks in turn
+    constexpr int64_t kPer = kBlockThreads / 2;
     const int64_t i0 = t0 * kPer, end = t1 * kPer;
     for (int64_t i = i0 + ((int64_t)blockIdx.x - pb) * kBlockThreads + threadIdx.x; i < end;
          i += (int64_t)nb * kBlockThreads) {
-        const float4 zv = __ldcs(z + i), sv = __ldcs(s + i);
-        float4 pv = p[i], qv = q[i], xv = x[i], rv = r[i];
+        const float2 zv = __ldcs(z + i);
+        const double2 sv = __ldcs(s + i);
+        double2 pv = p[i], qv = q[i];
+        float2 xv = x[i], rv = r[i];
         one(zv.x, sv.x, pv.x, qv.x, xv.x, rv.x);
         one(zv.y, sv.y, pv.y, qv.y, xv.y, rv.y);
-        one(zv.z, sv.z, pv.z, qv.z, xv.z, rv.z);
-        one(zv.w, sv.w, pv.w, qv.w, xv.w, rv.w);
         p[i] = pv;
         q[i] = qv;
         x[i] = xv;
@@ -349,12 +351,14 @@ cudaError_t launch_fcg_iteration(const DevSystem &sys, const float *z, cudaStrea
     if (sys.rows_per_thread != 1) return cudaErrorInvalidValue;  // tiles of 256 rows
     const SellView<float> A = {sys.n_rows, sys.slice_off, sys.col, sys.val32};
     const unsigned g = (unsigned)sys.plan[1].n_blocks;
-    auto v4 = [](float *v) { return reinterpret_cast<float4 *>(v); };  // rows start on cudaMalloc's boundary
-    const cudaError_t e = launch_chained(chained, k_fcg_spmv, g, kBlockThreads, s, A, z, sys.r32, sys.p32, sys.q32, sys.s32,
+    // (rows start on cudaMalloc's boundary)
+    auto f2 = [](float *v) { return reinterpret_cast<float2 *>(v); };
+    auto d2 = [](double *v) { return reinterpret_cast<double2 *>(v); };
+    const cudaError_t e = launch_chained(chained, k_fcg_spmv, g, kBlockThreads, s, A, z, sys.r32, sys.p, sys.q, sys.s,
                                          sys.partial, sys.ctl, plan32(sys), sys.n_done);
     if (e != cudaSuccess) return e;
-    return launch_chained(true, k_fcg_update, g, kBlockThreads, s, v4(sys.x32), v4(sys.r32), v4(sys.p32), v4(sys.q32),
-                          reinterpret_cast<const float4 *>(z), v4(sys.s32), sys.partial, sys.ctl, plan32(sys),
+    return launch_chained(true, k_fcg_update, g, kBlockThreads, s, f2(sys.x32), f2(sys.r32), d2(sys.p), d2(sys.q),
+                          reinterpret_cast<const float2 *>(z), d2(sys.s), sys.partial, sys.ctl, plan32(sys),
                           sys.n_done);
 }
 

@@ -307,7 +307,7 @@ int device_setup(mh_handle *h) {
     s.r = dalloc<double>(h, nr);
     s.p = dalloc<double>(h, nr);
     s.q = dalloc<double>(h, nr);
-    s.s32 = dalloc<float>(h, nr);
+    s.s = dalloc<double>(h, nr);
     s.x32 = dalloc<float>(h, nr);
     s.r32 = dalloc<float>(h, nr);
     s.p32 = dalloc<float>(h, nr);
@@ -318,7 +318,7 @@ int device_setup(mh_handle *h) {
     s.n_done = dalloc<int32_t>(h, 1);
     s.inst_sums = dalloc<double>(h, mh::kSumStride * (size_t)s.n_inst);
     s.sum_ticket = dalloc<uint32_t>(h, s.n_inst);
-    if (!s.val_raw || !s.val64 || !s.val32 || !s.dsq || !s.b || !s.bh || !s.x || !s.r || !s.p || !s.q || !s.s32 ||
+    if (!s.val_raw || !s.val64 || !s.val32 || !s.dsq || !s.b || !s.bh || !s.x || !s.r || !s.p || !s.q || !s.s ||
         !s.x32 || !s.r32 || !s.p32 || !s.q32 || !s.z32 || !s.partial || !s.ctl || !s.n_done || !s.inst_sums ||
         !s.sum_ticket)
         return MH_ERR_NOMEM;
