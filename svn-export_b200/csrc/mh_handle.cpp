@@ -176,13 +176,16 @@ template <class T> T *dalloc(mh_handle *h, size_t n) {
     return (T *)p;
 }
 
+// On the handle's stream, which the legacy stream of the plain calls does not order (own_stream does
+// not wait for it): what the handle launches next finds the data there.
 template <class T> int upload(mh_handle *h, T *&dst, const std::vector<T> &src) {
     dst = dalloc<T>(h, src.size());
     if (!dst) {
         h->err = "cudaMalloc failed";
         return MH_ERR_NOMEM;
     }
-    if (!src.empty()) CK(cudaMemcpy(dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice));
+    if (!src.empty())
+        CK(cudaMemcpyAsync(dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice, h->stream));
     return MH_OK;
 }
 
@@ -199,6 +202,17 @@ double side_measure_host(const mh::MeshData &m, int64_t e, int s) {
     double v[3] = {X[2][0] - X[0][0], X[2][1] - X[0][1], X[2][2] - X[0][2]};
     double c[3] = {u[1] * v[2] - u[2] * v[1], u[2] * v[0] - u[0] * v[2], u[0] * v[1] - u[1] * v[0]};
     return 0.5 * std::sqrt(c[0] * c[0] + c[1] * c[1] + c[2] * c[2]);
+}
+
+__global__ void k_fill(double *dst, int64_t n, double v) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) dst[i] = v;
+}
+
+__global__ void k_scatter(int64_t n, const int32_t *__restrict__ to, const double *__restrict__ v,
+                          double *__restrict__ dst) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) dst[to[i]] = v[i];
 }
 
 int device_setup(mh_handle *h) {
@@ -327,30 +341,35 @@ int device_setup(mh_handle *h) {
         std::memset(&ctl[i], 0, sizeof(mh::InstCtl));
         ctl[i].done = 1;
     }
-    CK(cudaMemcpy(s.ctl, ctl.data(), sizeof(mh::InstCtl) * ctl.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemset(s.x, 0, nr * sizeof(double)));
-    CK(cudaMemset(s.x32, 0, nr * sizeof(float)));
-    CK(cudaMemset(s.sum_ticket, 0, s.n_inst * sizeof(uint32_t)));
-    CK(cudaMemset(s.inst_sums, 0, mh::kSumStride * s.n_inst * sizeof(double)));
+    CK(cudaMemcpyAsync(s.ctl, ctl.data(), sizeof(mh::InstCtl) * ctl.size(), cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemsetAsync(s.x, 0, nr * sizeof(double), h->stream));
+    CK(cudaMemsetAsync(s.x32, 0, nr * sizeof(float), h->stream));
+    CK(cudaMemsetAsync(s.sum_ticket, 0, s.n_inst * sizeof(uint32_t), h->stream));
+    CK(cudaMemsetAsync(s.inst_sums, 0, mh::kSumStride * s.n_inst * sizeof(double), h->stream));
     if (h->general) {
         // the slots outside the caller's pattern hold a unit diagonal (padding rows) or 0 for good
         if ((rc = upload(h, h->d_csr_slot, hs.csr_slot))) return rc;
         h->d_csr_val = dalloc<double>(h, hs.nnz);
         if (!h->d_csr_val) return MH_ERR_NOMEM;
-        CK(cudaMemset(s.val_raw, 0, hs.n_slots * sizeof(double)));
-        CK(cudaMemset(s.b, 0, nr * sizeof(double)));
-        std::vector<double> one(nr - t.n_edges(), 1.0);
-        std::vector<int32_t> at(hs.diag_slot.begin() + t.n_edges(), hs.diag_slot.end());
-        for (size_t k = 0; k < at.size(); ++k)  // fewer than kPadRows
-            CK(cudaMemcpy(s.val_raw + at[k], &one[k], sizeof(double), cudaMemcpyHostToDevice));
+        CK(cudaMemsetAsync(s.val_raw, 0, hs.n_slots * sizeof(double), h->stream));
+        CK(cudaMemsetAsync(s.b, 0, nr * sizeof(double), h->stream));
+        const int64_t n_pad = nr - t.n_edges();
+        if (n_pad > 0) {
+            // s.p is the staging: nothing has been solved yet
+            k_fill<<<(unsigned)((n_pad + 255) / 256), 256, 0, h->stream>>>(s.p, n_pad, 1.0);
+            k_scatter<<<(unsigned)((n_pad + 255) / 256), 256, 0, h->stream>>>(n_pad, s.diag_slot + t.n_edges(), s.p,
+                                                                              s.val_raw);
+            CK(cudaGetLastError());
+        }
     }
     const int64_t msize = t.n_sides() + m.n_el + t.n_edges();
     h->sol = dalloc<double>(h, msize);
     h->sol_prev = dalloc<double>(h, msize);
     h->d_loop = dalloc<int32_t>(h, 2);
     if (!h->sol || !h->sol_prev || !h->d_loop) return MH_ERR_NOMEM;
-    CK(cudaMemset(h->sol, 0, msize * sizeof(double)));
-    CK(cudaMemset(h->sol_prev, 0, msize * sizeof(double)));
+    CK(cudaMemsetAsync(h->sol, 0, msize * sizeof(double), h->stream));
+    CK(cudaMemsetAsync(h->sol_prev, 0, msize * sizeof(double), h->stream));
+    CK(cudaStreamSynchronize(h->stream));
     h->device = true;
     return MH_OK;
 }
@@ -421,17 +440,6 @@ int check_positive(const double *a, int64_t n) {
 #pragma omp parallel for reduction(&& : ok) schedule(static) if (n > (1 << 16))
     for (int64_t i = 0; i < n; ++i) ok = ok && a[i] > 0.0;
     return ok;
-}
-
-__global__ void k_fill(double *dst, int64_t n, double v) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = v;
-}
-
-__global__ void k_scatter(int64_t n, const int32_t *__restrict__ to, const double *__restrict__ v,
-                          double *__restrict__ dst) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dst[to[i]] = v[i];
 }
 
 // a field from the caller's host array, or its default value filled on the device
@@ -630,12 +638,10 @@ bool resident_ready(mh_handle *h, int prec) {
             const size_t np = 16 * (size_t)pl.n_blocks, nq = (prec == 64 ? 4 : 2) * (size_t)h->sys.n_rows;
             d.part = dalloc<double>(h, np);
             d.q = dalloc<double>(h, nq);
-            d.tag = dalloc<unsigned long long>(h, 1);
             d.err = dalloc<int32_t>(h, 1);
-            const unsigned long long first = 1;
-            if (!d.part || !d.q || !d.tag || !d.err || cudaMemset(d.part, 0, np * sizeof(double)) != cudaSuccess ||
-                cudaMemset(d.q, 0, nq * sizeof(double)) != cudaSuccess ||
-                cudaMemcpy(d.tag, &first, sizeof(first), cudaMemcpyHostToDevice) != cudaSuccess)
+            if (!d.part || !d.q || !d.err || upload(h, d.tag, std::vector<unsigned long long>{1}) ||
+                cudaMemsetAsync(d.part, 0, np * sizeof(double), h->stream) != cudaSuccess ||
+                cudaMemsetAsync(d.q, 0, nq * sizeof(double), h->stream) != cudaSuccess)
                 return false;
             pl.idx.clear();
             pl.idx.shrink_to_fit();
