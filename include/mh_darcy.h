@@ -376,7 +376,9 @@ int mh_create_mortar(const mh_mesh_desc *mesh, const mh_mortar_desc *mortar, mh_
 /* Autotuner: times `iterations` FP64 and FP32 CG iterations on the assembled system for
  * every launch shape (rows per thread R in {1, 2, 4}, blocks per SM from the occupancy of
  * that R's SpMV kernels) and keeps the fastest.  Writes the chosen R and the FP32 and FP64
- * microseconds per iteration (either pointer may be NULL). */
+ * microseconds per iteration (either pointer may be NULL).  These are the two-kernel
+ * iteration's: a single system that fits on the chip runs MH_SOLVER_PCG64 and _IR32 as one
+ * resident kernel, which has no such shape (about 3-8 us an iteration). */
 int mh_autotune(mh_handle *h, int32_t iterations, int32_t *rows_per_thread, double *us_per_iter);
 
 /* The launch shapes mh_autotune_ex chose. */

@@ -9,6 +9,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <limits>
 #include <memory>
 #include <random>
@@ -90,7 +91,6 @@ struct mh_handle {
     mh::ResidentPlan res_plan[2];
     int res_state[2] = {0, 0};
     mh::ResidentDev res_dev[2];
-    bool two_kernel = false;    // mh_autotune times the launch shapes of the two-kernel iteration
     int k1_group = 128;         // elements per K1 block (mh_autotune_ex)
     int amg_fine_passes = 0;    // pairing passes from the fine level chosen by mh_autotune_ex (0: default)
     bool host_loop = false;     // the current solve polls from the host instead (mh_solve_opts)
@@ -624,7 +624,8 @@ int run_krylov_loop(mh_handle *h, int prec, int ipg, int max_it) {
 }
 
 // The plan of the shared-memory-resident run, made once per handle and precision.  Batches keep
-// the two-kernel iteration: its launches are shared by all instances.
+// the two-kernel iteration: its launches are shared by all instances.  A plan whose buffers cannot be had
+// leaves nothing behind: no memory, and no error for the next launch to read as its own.
 bool resident_ready(mh_handle *h, int prec) {
     const int gi = prec == 64 ? 0 : 1;
     if (h->res_state[gi] == 0) {
@@ -632,45 +633,72 @@ bool resident_ready(mh_handle *h, int prec) {
         mh::ResidentPlan &pl = h->res_plan[gi];
         mh::ResidentDev &d = h->res_dev[gi];
         if (h->sys.n_inst == 1 && mh::plan_resident(h->hs.slice_off, h->hs.sell_col, h->hs.diag_slot, prec, pl)) {
-            if (upload(h, d.blk_slice, pl.blk_slice) || upload(h, d.halo_off, pl.halo_off) ||
-                upload(h, d.halo_row, pl.halo_row) || upload(h, d.idx, pl.idx))
-                return false;
+            const size_t mark = h->allocs.size();
+            const std::string err = h->err;
             const size_t np = 16 * (size_t)pl.n_blocks, nq = (prec == 64 ? 4 : 2) * (size_t)h->sys.n_rows;
             d.part = dalloc<double>(h, np);
             d.q = dalloc<double>(h, nq);
             d.err = dalloc<int32_t>(h, 1);
-            if (!d.part || !d.q || !d.err || upload(h, d.tag, std::vector<unsigned long long>{1}) ||
-                cudaMemsetAsync(d.part, 0, np * sizeof(double), h->stream) != cudaSuccess ||
-                cudaMemsetAsync(d.q, 0, nq * sizeof(double), h->stream) != cudaSuccess)
-                return false;
-            pl.idx.clear();
-            pl.idx.shrink_to_fit();
-            h->res_state[gi] = 1;
+            if (d.part && d.q && d.err && !upload(h, d.blk_slice, pl.blk_slice) &&
+                !upload(h, d.halo_off, pl.halo_off) && !upload(h, d.halo_row, pl.halo_row) &&
+                !upload(h, d.idx, pl.idx) && !upload(h, d.tag, std::vector<unsigned long long>{1}) &&
+                cudaMemsetAsync(d.part, 0, np * sizeof(double), h->stream) == cudaSuccess &&
+                cudaMemsetAsync(d.q, 0, nq * sizeof(double), h->stream) == cudaSuccess) {
+                h->res_state[gi] = 1;
+            } else {
+                cudaStreamSynchronize(h->stream);
+                for (size_t k = mark; k < h->allocs.size(); ++k) cudaFree(h->allocs[k]);
+                h->allocs.resize(mark);
+                h->err = err;
+                d = mh::ResidentDev();
+                cudaGetLastError();
+            }
         }
+        std::vector<uint16_t>().swap(pl.idx);
     }
     return h->res_state[gi] == 1;
 }
 
-int run_resident(mh_handle *h, int prec) {
+// How a Krylov run begins: what its caller has launched before it, once more.
+using Restart = std::function<cudaError_t()>;
+
+// The resident run.  done = false: its launch was refused (the chip is shared) or an exchange did not
+// complete in its bounded wait.  The run is then back at its start, x as it was, and the handle
+// keeps to the two-kernel iteration.  (MH_RESIDENT_POLLS: a shorter wait.)
+int run_resident(mh_handle *h, int prec, const Restart &restart, bool &done) {
     const int gi = prec == 64 ? 0 : 1;
-    CK(mh::launch_cg_resident(h->sys, h->res_plan[gi], h->res_dev[gi], h->stream));
-    h->n_launch += 1;
-    CK(cudaMemcpyAsync(h->h_done, h->res_dev[gi].err, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    if (*h->h_done) {
-        h->err = "Krylov run: a grid barrier did not complete (bounded wait timed out)";
-        return MH_ERR_CUDA;
+    const size_t bytes = (size_t)h->sys.n_rows * sizeof(double);
+    int polls = mh::kResidentPolls;
+    if (const char *e = getenv("MH_RESIDENT_POLLS")) polls = std::max(0, std::min(polls, atoi(e)));
+    // the FP64 run works on x itself; q is idle in it (the FP32 run leaves x alone)
+    if (prec == 64) CK(cudaMemcpyAsync(h->sys.q, h->sys.x, bytes, cudaMemcpyDeviceToDevice, h->stream));
+    const cudaError_t e = mh::launch_cg_resident(h->sys, h->res_plan[gi], h->res_dev[gi], polls, h->stream);
+    done = e == cudaSuccess;
+    if (done) {
+        h->n_launch += 1;
+        CK(cudaMemcpyAsync(h->h_done, h->res_dev[gi].err, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaStreamSynchronize(h->stream));
+        done = *h->h_done == 0;
     }
+    if (done) return MH_OK;
+    cudaGetLastError();
+    h->res_state[gi] = -1;
+    if (prec == 64) CK(cudaMemcpyAsync(h->sys.x, h->sys.q, bytes, cudaMemcpyDeviceToDevice, h->stream));
+    CK(restart());
     return MH_OK;
 }
 
 // Runs captured Krylov iterations until every instance reports done: in the device-side loop,
 // or (host_loop, or `prof`) as graphs of `ipg` iterations launched while the host sees an
 // instance running.  With `prof`, the kernels of the iterations that still did work are timed
-// from the in-graph events.
-int run_krylov(mh_handle *h, int prec, int ipg, int max_it, bool prof) {
+// from the in-graph events.  A system that fits on the chip runs there (with a `restart` to go back to).
+int run_krylov(mh_handle *h, int prec, int ipg, int max_it, bool prof, const Restart &restart = nullptr) {
     ipg = std::max(1, ipg);  // an empty graph would never make progress
-    if (!prof && !h->host_loop && !h->two_kernel && resident_ready(h, prec)) return run_resident(h, prec);
+    if (!prof && !h->host_loop && restart && resident_ready(h, prec)) {
+        bool done;
+        const int rc = run_resident(h, prec, restart, done);
+        if (rc || done) return rc;
+    }
     if (!prof && !h->host_loop && !h->loop_unavailable) {
         const int rc = run_krylov_loop(h, prec, ipg, max_it);
         if (rc != MH_ERR_CUDA || h->loop_graph[prec == 64 ? 0 : 1]) return rc;
@@ -771,10 +799,15 @@ int solve_pcg64(mh_handle *h, const mh_solve_opts &o, SolveResult &res) {
     double tau = o.r_tol;
     int total = 0;
     for (int run = 0; run < 12; ++run) {
-        CK(mh::launch_reset_ctl(h->sys, h->stream));
-        CK(mh::launch_cg_init(h->sys, tau * tau, 0.0, std::max(1, o.max_it - total), run > 0, h->stream));
-        h->n_launch += 1;
-        int rc = run_krylov(h, 64, o.iters_per_graph, o.max_it - total, o.profile_kernels != 0);
+        const Restart begin = [&] {
+            const cudaError_t e = mh::launch_reset_ctl(h->sys, h->stream);
+            h->n_launch += 1;
+            return e != cudaSuccess ? e
+                                    : mh::launch_cg_init(h->sys, tau * tau, 0.0, std::max(1, o.max_it - total), run > 0,
+                                                         h->stream);
+        };
+        CK(begin());
+        int rc = run_krylov(h, 64, o.iters_per_graph, o.max_it - total, o.profile_kernels != 0, begin);
         if (rc) return rc;
         if ((rc = read_ctl(h, ctl))) return rc;
         count_iterations(h, ctl);
@@ -864,7 +897,13 @@ int solve_ir32(mh_handle *h, const mh_solve_opts &o, SolveResult &res) {
             CK(mh::launch_ir_start(h->sys, o.inner_rtol * o.inner_rtol, seg_max, h->stream));
         else
             CK(mh::launch_ir_replace(h->sys, o.inner_rtol * o.inner_rtol, seg_max, h->stream));
-        if ((rc = run_krylov(h, 32, o.iters_per_graph, seg_max, o.profile_kernels != 0))) return rc;
+        // (a failed resident run has spoilt the direction: a new sequence)
+        const Restart again = [&] {
+            const cudaError_t e = mh::launch_reset_ctl(h->sys, h->stream);
+            return e != cudaSuccess ? e
+                                    : mh::launch_ir_start(h->sys, o.inner_rtol * o.inner_rtol, seg_max, h->stream);
+        };
+        if ((rc = run_krylov(h, 32, o.iters_per_graph, seg_max, o.profile_kernels != 0, again))) return rc;
         CK(mh::launch_ir_correct(h->sys, h->stream));
         h->n_launch += 2;
         if ((rc = read_ctl(h, ctl))) return rc;
@@ -2702,11 +2741,6 @@ int mh_autotune(mh_handle *h, int32_t iterations, int32_t *rows_per_thread, doub
     double best = 1e300, best32 = 0.0, best64 = 0.0;
     int best_r = h->hs.rows_per_thread;
     std::vector<double> sums;
-    h->two_kernel = true;  // the launch shapes are the two-kernel iteration's
-    struct Restore {
-        bool &flag;
-        ~Restore() { flag = false; }
-    } restore{h->two_kernel};
     for (int R : {1, 2, 4}) {
         const int targets[2] = {mh::krylov_target_blocks(R, 64), mh::krylov_target_blocks(R, 32)};
         if ((rc = apply_launch_shape(h, R, targets))) return rc;
@@ -2728,6 +2762,7 @@ int mh_autotune(mh_handle *h, int32_t iterations, int32_t *rows_per_thread, doub
             // warm the captured graph, then time
             if ((rc = capture_iterations(h, prec, ipg, false))) return rc;
             CK(cudaEventRecord(h->ev[0], h->stream));
+            // (no restart: the two-kernel iteration, whose launch shape this is about)
             if ((rc = run_krylov(h, prec, ipg, iterations, false))) return rc;
             CK(cudaEventRecord(h->ev[1], h->stream));
             CK(cudaStreamSynchronize(h->stream));

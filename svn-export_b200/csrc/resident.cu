@@ -20,7 +20,8 @@
 // Rows are cut into contiguous runs of 32-row slices, balanced by bytes; columns are 16-bit
 // indices into the block's own and halo entries, the diagonal is kept apart.
 // The launch is cooperative, so all blocks are on the chip together; every poll is bounded, and a
-// block that gives up sets *err and leaves.
+// block that gives up sets *err and leaves: the vectors and the exchange buffers are then worth
+// nothing, and the host starts the run again with the two-kernel iteration.
 // The smallest systems run in one thread-block cluster instead (k_cg_cluster below).
 // Measured (B200, us an iteration, two-kernel iteration -> this one): FP64, 6.9k edges 10.8 -> 2.8,
 // 52k 11.7 -> 3.1, 175k 15.5 -> 4.6, 273k 17.7 -> 5.3; FP32, 52k 12.8 -> 3.5, 244k 17.1 -> 4.8,
@@ -43,7 +44,6 @@ namespace {
 constexpr int kResThreads = 1024;
 constexpr int kResMaxBlocks = 256;
 constexpr int kResCluster = 16;    // blocks of a cluster at most
-constexpr int kResSpin = 1 << 21;  // polls of one value (about a second) before a block gives up
 
 struct ResArgs {
     const int64_t *slice_off;
@@ -56,6 +56,7 @@ struct ResArgs {
     double2 *part;             // [2][n_blocks][4] (sum, tag)
     unsigned long long *tag0;  // the launch's first tag; block 0 leaves the next launch's
     int32_t rows_cap;          // rows of the largest block (cluster)
+    int32_t polls;             // of one value at most, before a block gives up
     int32_t *n_done;
     int32_t *err;
 };
@@ -99,10 +100,10 @@ __device__ __forceinline__ double ld_pair(const double2 *p, unsigned long long w
     fresh = tag == want;
     return __longlong_as_double(v);
 }
-// polls one value, at most kResSpin times (late: it never came)
+// polls one value, at most `polls` times (late: it never came)
 template <typename P, typename T>
-__device__ __forceinline__ T await_pair(const P *p, T first, bool fresh, unsigned long long want, int &late) {
-    for (int spin = 0; !fresh && !late && spin < kResSpin; ++spin) first = ld_pair(p, want, fresh);
+__device__ __forceinline__ T await_pair(const P *p, T first, bool fresh, unsigned long long want, int polls, int &late) {
+    for (int spin = 0; !fresh && !late && spin < polls; ++spin) first = ld_pair(p, want, fresh);
     late |= !fresh;
     return first;
 }
@@ -333,12 +334,12 @@ __global__ void __launch_bounds__(kResThreads, 1)
         for (int k = threadIdx.x; k < 4 * nb; k += blockDim.x) {
             bool fresh;
             const double v = ld_pair(part + k, tag, fresh);
-            gath[k & 3][k >> 2] = await_pair(part + k, v, fresh, tag, late);
+            gath[k & 3][k >> 2] = await_pair(part + k, v, fresh, tag, a.polls, late);
         }
 #pragma unroll
         for (int i = 0; i < kH; ++i) {
             const int k = threadIdx.x + i * blockDim.x;
-            if (k < nh) hq[i] = await_pair(gq + hrow[k], hq[i], hf[i], tag, late);
+            if (k < nh) hq[i] = await_pair(gq + hrow[k], hq[i], hf[i], tag, a.polls, late);
         }
         ok = !__syncthreads_or(late);
         if (!ok) break;
@@ -362,7 +363,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
             if (k < nh) cg_step(hq[i], alpha, beta, hr[k], sp[nr + k]);
         }
         for (int k = threadIdx.x + kH * blockDim.x; k < nh; k += blockDim.x) {
-            const T qh = await_pair(gq + hrow[k], (T)0, false, tag, late);
+            const T qh = await_pair(gq + hrow[k], (T)0, false, tag, a.polls, late);
             cg_step(qh, alpha, beta, hr[k], sp[nr + k]);
         }
         rr_part = 0.0;
@@ -670,7 +671,8 @@ bool plan_resident(const std::vector<int64_t> &slice_off, const std::vector<int3
     return plan_blocks(slice_off, col, diag_slot, prec, false, plan);
 }
 
-cudaError_t launch_cg_resident(const DevSystem &sys, const ResidentPlan &plan, const ResidentDev &dev, cudaStream_t s) {
+cudaError_t launch_cg_resident(const DevSystem &sys, const ResidentPlan &plan, const ResidentDev &dev, int polls,
+                               cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(dev.err, 0, sizeof(int32_t), s);
     if (e != cudaSuccess) return e;
     ResArgs a;
@@ -693,6 +695,7 @@ cudaError_t launch_cg_resident(const DevSystem &sys, const ResidentPlan &plan, c
     float2 *qf0 = reinterpret_cast<float2 *>(dev.q), *qf1 = qf0 + sys.n_rows;
     void *args64[] = {&a, &v64, &x64, &r64, &p64, &qd0, &qd1}, *args32[] = {&a, &v32, &x32, &r32, &p32, &qf0, &qf1};
     a.rows_cap = plan.rows_cap;
+    a.polls = polls;
     if (plan.cluster) {
         cudaLaunchAttribute at[1];
         const cudaLaunchConfig_t cfg = cluster_config(plan, at, s);

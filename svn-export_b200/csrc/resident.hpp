@@ -43,8 +43,11 @@ struct ResidentDev {
 // Plans the run for the current device (prec: 64 or 32); false when the system does not fit.
 bool plan_resident(const std::vector<int64_t> &slice_off, const std::vector<int32_t> &col,
                    const std::vector<int32_t> &diag_slot, int prec, ResidentPlan &plan);
+// Polls of one value of an exchange (about a second) before a block gives up.
+constexpr int kResidentPolls = 1 << 21;
 // One Krylov run of a single-instance system, from the state k_cg_init / k_ir_start left, to the
-// end of the run.
-cudaError_t launch_cg_resident(const DevSystem &sys, const ResidentPlan &plan, const ResidentDev &dev, cudaStream_t s);
+// end of the run; *dev.err != 0 afterwards: an exchange did not complete, x, r, p are worth nothing.
+cudaError_t launch_cg_resident(const DevSystem &sys, const ResidentPlan &plan, const ResidentDev &dev, int polls,
+                               cudaStream_t s);
 
 }  // namespace mh
