@@ -413,7 +413,8 @@ __global__ void __launch_bounds__(kResThreads, 1)
     if (c->done) return;  // the same value in every block: it is written behind the last barrier
     cg::cluster_group cl = cg::this_cluster();
     extern __shared__ __align__(16) unsigned char rsm[];
-    __shared__ double sh[32][4], mail[2][kResCluster][4];
+    __shared__ double sh[32][4];
+    __shared__ double2 mail[2][kResCluster][2];  // a block's four sums in two stores of 16 bytes
     __shared__ RunState out;
     constexpr bool kReg = KR <= 2;
     RunState own;
@@ -464,16 +465,16 @@ __global__ void __launch_bounds__(kResThreads, 1)
 #pragma unroll
             for (int k = 0; k < 4; ++k) t[k] = __shfl_sync(0xffffffffu, w4, 8 * k);
             if (lane < nb) {
-                double2 *to = reinterpret_cast<double2 *>(cl.map_shared_rank(&mail[half][blockIdx.x][0], lane));
+                double2 *to = cl.map_shared_rank(&mail[half][blockIdx.x][0], lane);
                 to[0] = make_double2(t[0], t[1]);
                 to[1] = make_double2(t[2], t[3]);
             }
         }
         cl.sync();
         if (warp == 0) {
-            double t[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) t[k] = lane < nb ? mail[half][lane][k] : 0.0;
+            const double2 none = make_double2(0.0, 0.0);
+            const double2 m0 = lane < nb ? mail[half][lane][0] : none, m1 = lane < nb ? mail[half][lane][1] : none;
+            const double t[4] = {m0.x, m0.y, m1.x, m1.y};
             w4 = warp_sum4(t, lane);
             const double pq = __shfl_sync(0xffffffffu, w4, 0), rq = __shfl_sync(0xffffffffu, w4, 8),
                          qq = __shfl_sync(0xffffffffu, w4, 16), rr = __shfl_sync(0xffffffffu, w4, 24);
