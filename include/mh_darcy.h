@@ -490,6 +490,11 @@ int mh_amg_info(const mh_handle *h, int32_t *n_levels, int64_t *rows, int64_t *s
  * as one thread-block cluster launch, and the cluster's CTAs; 0 and 0 when every level runs
  * its own kernels. */
 int mh_amg_tail(const mh_handle *h, int32_t *level, int32_t *cluster_ctas);
+/* The coarsest level of that hierarchy: n rows solved by their dense inverse (FP32, [n][n] row by
+ * row, for the level's first n rows; may be NULL), or n = 0 where it is smoothed by a polynomial
+ * instead (too large, or not positive definite to FP32 rounding).  MH_ERR_STATE before the
+ * first multigrid solve. */
+int mh_amg_coarsest(const mh_handle *h, int64_t *n, float *inverse);
 /* One level of that hierarchy in CSR without zero entries (level 0 = the FP32 Jacobi-scaled
  * edge system in padded solver-row order), its aggregation agg [n] (coarse row of each row,
  * -1: none; not on the last level) and transfer weights [n]: level l+1 is P^T W A_l W P with

@@ -1,6 +1,7 @@
 // Aggregation multigrid preconditioner: GPU setup (pairwise aggregation, Galerkin products,
 // dense coarsest inverse) and the V-cycle.  See amg.hpp for the method.
 #include <algorithm>
+#include <cfloat>
 #include <climits>
 #include <cmath>
 #include <cstring>
@@ -795,7 +796,8 @@ __global__ void k_slice_width(int64_t n_slices, int64_t nc, const int32_t *rowle
 // column k).  Every block forms P for its columns, so a step needs nothing from another block of the
 // same launch.  D comes from the launch before: the block that updates A_kk goes on to invert it (32
 // pivots in a row, the longest chain of a step, which would otherwise stand in front of every block's
-// work).  flag = 1 on a non-positive or non-finite pivot.
+// work).  *flag: kPivotBad where a pivot is not positive or its reciprocal not finite; kPivotLost where one
+// is below the FP32 rounding of the row's diagonal, what the entries of A are known to.
 // Measured (B200): the inverse of 130 rows 360 us by one block with the matrix in shared memory;
 // with every block inverting A_kk itself 15 us a step at 477 rows (0.23 ms), 27 at 1120 (0.95 ms); with D
 // from the launch before 15 and 17 (the chain of one block's update and 32 pivots; at 1120 rows
@@ -810,13 +812,15 @@ constexpr int kHostWords = 256;  // pinned words of Amg's read-backs
 constexpr int kCoarseMin = 160;  // pairing passes go on down to this many rows
 constexpr int kGjB = 32, kGjTile = 64;
 
-// the n x n part of A in the np x np matrix M (zeroed before; identity in the padding)
-__global__ void k_dense_scatter(MatView A, int n, int np, double *M) {
+constexpr int kPivotBad = 1, kPivotLost = 2;
+
+// the n x n part of A in the np x np matrix M (zeroed before; identity in the padding), and its diagonal
+__global__ void k_dense_scatter(MatView A, int n, int np, double *M, double *diag) {
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= np) return;
     if (i >= n) {
-        M[(size_t)i * np + i] = 1.0;
+        M[(size_t)i * np + i] = diag[i] = 1.0;
         return;
     }
     int64_t base;
@@ -827,10 +831,12 @@ __global__ void k_dense_scatter(MatView A, int n, int np, double *M) {
         const int32_t c = A.col[slot];
         if (c < n) M[(size_t)i * np + c] += (double)A.val[slot];
     }
+    diag[i] = M[(size_t)i * np + i];
 }
 
-// 1 / x to the last bit or so: the hardware's 20-bit approximation and two Newton steps (a quarter of
-// the latency of the full division, which is the pivots' critical path)
+// 1 / x to the last bit or so, for x from 1e-300 to 1e300: the hardware's 20-bit approximation (subnormal
+// operands are zero to it) and two Newton steps (a quarter of the latency of the full division, which is
+// the pivots' critical path)
 __device__ __forceinline__ double quick_rcp(double x) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
@@ -841,9 +847,10 @@ __device__ __forceinline__ double quick_rcp(double x) {
 // The inverse of a 32 x 32 block by the 256 threads of a block: thread t holds m, four entries of
 // row r = t / 8 from column c4 = 4 (t % 8) on.  Pivot p: with a 1 in the pivot's place of row p, zeros
 // left behind in row p and column p, and the factor -1 for row p, every entry is m -= f / pivot * row_p.
+// diag: the block's rows' part of the matrix's own diagonal, in shared memory.
 __device__ __forceinline__ void gj_invert(double (&m)[4], int r, int c4, double (*rowb)[kGjB], double (*colb)[kGjB],
-                                          int32_t *flag) {
-    bool bad = false;
+                                          const double *diag, int32_t *flag) {
+    bool bad = false, lost = false;
 #pragma unroll 1
     for (int p0 = 0; p0 < kGjB; p0 += 4) {
 #pragma unroll
@@ -863,33 +870,36 @@ __device__ __forceinline__ void gj_invert(double (&m)[4], int r, int c4, double 
             }
             __syncthreads();
             const double piv = cb[p];
-            bad |= !(piv > 0.0 && piv < 1e300);
+            bad |= !(piv > 1e-300 && piv < 1e300);
+            lost |= !(piv > (double)FLT_EPSILON * diag[p]);
             const double g = (r == p ? -1.0 : cb[r]) * quick_rcp(piv);
 #pragma unroll
             for (int q = 0; q < 4; ++q) m[q] = fma(-g, rb[c4 + q], m[q]);
         }
     }
-    if (bad && r == 0 && c4 == 0) *flag = 1;
+    if ((bad || lost) && r == 0 && c4 == 0) atomicOr(flag, (bad ? kPivotBad : 0) | (lost ? kPivotLost : 0));
 }
 
 // D of the first step
-__global__ void __launch_bounds__(256) k_gj_first(const double *M, int np, double *dinv, int32_t *flag) {
+__global__ void __launch_bounds__(256) k_gj_first(const double *M, int np, const double *diag, double *dinv,
+                                                  int32_t *flag) {
     pdl_wait();
-    __shared__ double rowb[2][kGjB], colb[2][kGjB];
+    __shared__ double rowb[2][kGjB], colb[2][kGjB], dg[kGjB];
+    if (threadIdx.x < kGjB) dg[threadIdx.x] = diag[threadIdx.x];
     const int r = threadIdx.x >> 3, c4 = (threadIdx.x & 7) * 4;
     double m[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) m[q] = M[(size_t)r * np + c4 + q];
-    gj_invert(m, r, c4, rowb, colb, flag);
+    gj_invert(m, r, c4, rowb, colb, dg, flag);
 #pragma unroll
     for (int q = 0; q < 4; ++q) dinv[r * kGjB + c4 + q] = m[q];
 }
 
 // dinv: D of this step; dinv_next: of the next one, written by the block that holds it
-__global__ void __launch_bounds__(256) k_gj_step(const double *src, double *dst, int np, int k, const double *dinv,
-                                                 double *dinv_next, int32_t *flag) {
+__global__ void __launch_bounds__(256) k_gj_step(const double *src, double *dst, int np, int k, const double *diag,
+                                                 const double *dinv, double *dinv_next, int32_t *flag) {
     pdl_wait();
-    __shared__ double D[kGjB][kGjB + 1], rowb[2][kGjB], colb[2][kGjB];
+    __shared__ double D[kGjB][kGjB + 1], rowb[2][kGjB], colb[2][kGjB], dg[kGjB];
     __shared__ double Ai[kGjTile][kGjB + 1], P[kGjB][kGjTile];
     const int t = threadIdx.x, kb = k * kGjB;
     const int i0 = blockIdx.y * kGjTile, j0 = blockIdx.x * kGjTile;
@@ -959,12 +969,13 @@ __global__ void __launch_bounds__(256) k_gj_step(const double *src, double *dst,
     }
     const int kn = kb + kGjB;
     if (kn >= np || kn < i0 || kn >= i0 + kGjTile || i0 != j0) return;
+    if (t < kGjB) dg[t] = diag[kn + t];
     __syncthreads();
     const int r = t >> 3, c4 = (t & 7) * 4;
     double m[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) m[q] = D[r][c4 + q];
-    gj_invert(m, r, c4, rowb, colb, flag);
+    gj_invert(m, r, c4, rowb, colb, dg, flag);
 #pragma unroll
     for (int q = 0; q < 4; ++q) dinv_next[r * kGjB + c4 + q] = m[q];
 }
@@ -2288,6 +2299,7 @@ void Amg::release() {
     dense_inv_.release();
     for (auto &w : dense_work_) w.release();
     dense_pivot_.release();
+    dense_diag_.release();
     bound_.release();
     tail_prog_.release();
     tail_levels_.release();
@@ -2539,22 +2551,23 @@ cudaError_t Amg::galerkin(const AmgMatrix &A, const int32_t *agg, int64_t nc, co
     return cudaSuccess;
 }
 
-// *dense_flag_ != 0 afterwards: the matrix was not positive definite
+// *dense_flag_ afterwards: what was wrong with the pivots (kPivotBad, kPivotLost)
 cudaError_t Amg::dense_coarse(const AmgMatrix &A, cudaStream_t s) {
     const int n = (int)dense_n_, np = (int)round_up(n, kGjB);
     const int64_t ld = dense_ld(n);
     AMG_CK(dense_inv_.ensure((size_t)n * ld));
     for (auto &w : dense_work_) AMG_CK(w.ensure((size_t)np * np));
     AMG_CK(cudaMemsetAsync(dense_work_[0].p, 0, (size_t)np * np * sizeof(double), s));
-    launch_chained(true, k_dense_scatter, nblk(np, 128), 128, s, view(A), n, np, dense_work_[0].p);
+    AMG_CK(dense_diag_.ensure(np));
+    launch_chained(true, k_dense_scatter, nblk(np, 128), 128, s, view(A), n, np, dense_work_[0].p, dense_diag_.p);
     const unsigned tiles = nblk(np, kGjTile);
     AMG_CK(dense_pivot_.ensure(2 * kGjB * kGjB));
     double *const dinv[2] = {dense_pivot_.p, dense_pivot_.p + kGjB * kGjB};
-    launch_chained(true, k_gj_first, 1, 256, s, dense_work_[0].p, np, dinv[0], dense_flag_);
+    launch_chained(true, k_gj_first, 1, 256, s, dense_work_[0].p, np, dense_diag_.p, dinv[0], dense_flag_);
     int from = 0;
     for (int k = 0; k < np / kGjB; ++k, from ^= 1)
         launch_chained(true, k_gj_step, dim3(tiles, tiles), 256, s, dense_work_[from].p, dense_work_[from ^ 1].p,
-                       np, k, dinv[from], dinv[from ^ 1], dense_flag_);
+                       np, k, dense_diag_.p, dinv[from], dinv[from ^ 1], dense_flag_);
     launch_chained(true, k_dense_store, nblk(n * ld, 256), 256, s, n, np, (int)ld, dense_work_[from].p,
                    dense_inv_.p);
     AMG_CK(cudaGetLastError());
@@ -2725,14 +2738,13 @@ cudaError_t Amg::setup(const DevSystem &sys, const AmgOptions &o, cudaStream_t s
             err = "Galerkin row wider than the gather buffer";
             return cudaErrorInvalidValue;
         }
-        if (h_flag_[words - 1]) {
-            if (dense_n_ <= kCoarseMin) {
-                err = "coarsest matrix is not positive definite";
-                return cudaErrorInvalidValue;
-            }
-            // (a larger matrix can lose definiteness to its FP32 rounding: smoothed instead, on its
+        if (dense_n_ > kCoarseMin) {
+            // (a matrix this large can lose definiteness to its FP32 rounding: smoothed instead, on its
             // Gershgorin interval)
-            dense_n_ = 0;
+            if (h_flag_[words - 1]) dense_n_ = 0;
+        } else if (h_flag_[words - 1] & kPivotBad) {
+            err = "coarsest matrix is not positive definite";
+            return cudaErrorInvalidValue;
         }
         if (widest > 0) AMG_CK(prepare_fine_tma(widest, s));
         for (int l = 0; l < n_levels_; ++l) {
@@ -2794,6 +2806,14 @@ cudaError_t Amg::setup(const DevSystem &sys, const AmgOptions &o, cudaStream_t s
     AMG_CK(tickets_.ensure(n_levels_ + 1));
     AMG_CK(cudaMemsetAsync(tickets_.p, 0, (n_levels_ + 1) * sizeof(unsigned int), s));
     return build_tail(s);
+}
+
+cudaError_t Amg::dense_inverse(float *out, cudaStream_t s) const {
+    if (dense_n_ <= 0) return cudaSuccess;
+    const size_t row = dense_n_ * sizeof(float);
+    const cudaError_t e = cudaMemcpy2DAsync(out, row, dense_inv_.p, dense_ld(dense_n_) * sizeof(float), row, dense_n_,
+                                            cudaMemcpyDeviceToHost, s);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(s);
 }
 
 // whether the coarsest level gets a dense inverse: small enough, and never the fine level of a

@@ -123,6 +123,9 @@ public:
     const AmgLevel &level(int l) const { return lv_[l]; }
     int64_t coarse_rows() const { return n_levels_ ? lv_[n_levels_ - 1].A.n : 0; }
     // the first level of the coarse tail run as one cluster launch (0: none) and its CTAs
+    // rows of the coarsest level that is inverted (0: it gets a polynomial), and the inverse
+    int64_t dense_rows() const { return dense_n_; }
+    cudaError_t dense_inverse(float *out, cudaStream_t s) const;
     int tail_level() const { return tail_phases_ > 0 ? tail_level_ : 0; }
     // the fine level's kernels stream the matrix with TMA; a stage wait that timed out (read
     // back and cleared: the cycle's results are then not usable)
@@ -204,7 +207,7 @@ private:
     std::vector<int64_t> dots_long_off_;
     DBuf<float> isd_;
     DBuf<float> dense_inv_;         // inverse of the coarsest matrix, and the two copies it is made in
-    DBuf<double> dense_work_[2], dense_pivot_;
+    DBuf<double> dense_work_[2], dense_pivot_, dense_diag_;
     DBuf<int32_t> flag_;
     DBuf<unsigned int> bound_;
     DBuf<double> dots_, alpha_;     // coarse-correction scaling: partials, factor per level

@@ -2961,6 +2961,16 @@ int mh_amg_tail(const mh_handle *hc, int32_t *level, int32_t *cluster_ctas) {
     return MH_OK;
 }
 
+int mh_amg_coarsest(const mh_handle *hc, int64_t *n, float *inverse) {
+    mh_handle *h = const_cast<mh_handle *>(hc);
+    int rc = need_device(h);
+    if (rc) return rc;
+    if (h->amg.levels() == 0) return MH_ERR_STATE;
+    if (n) *n = h->amg.dense_rows();
+    if (inverse) CK(h->amg.dense_inverse(inverse, h->stream));
+    return MH_OK;
+}
+
 int mh_amg_level(const mh_handle *hc, int32_t level, int64_t *n, int64_t *nnz, int32_t *agg, float *weight,
                  int32_t *row_ptr, int32_t *col, float *val) {
     mh_handle *h = const_cast<mh_handle *>(hc);

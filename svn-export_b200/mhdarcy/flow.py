@@ -296,6 +296,17 @@ class MHSystem:
         check(lib.mh_amg_tail(self.h, ptr(lv, C.c_int32), ptr(cl, C.c_int32)), self.h)
         return dict(level=int(lv[0]), cluster=int(cl[0]))
 
+    def amg_coarsest(self):
+        """The dense inverse of the last AMG hierarchy's coarsest level ([n, n], FP32), or None where a
+        polynomial smooths that level instead."""
+        n = C.c_int64(0)
+        check(lib.mh_amg_coarsest(self.h, C.byref(n), None), self.h)
+        if n.value == 0:
+            return None
+        inv = np.zeros((n.value, n.value), np.float32)
+        check(lib.mh_amg_coarsest(self.h, None, ptr(inv, C.c_float)), self.h)
+        return inv
+
     def amg_level(self, level):
         """((row_ptr, col, val), agg, weight) of level `level` of the last AMG hierarchy."""
         n, nnz = C.c_int64(0), C.c_int64(0)
