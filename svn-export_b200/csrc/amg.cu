@@ -2212,14 +2212,13 @@ decltype(&k_pair_want<1>) pair_want_kernel(int g) {
 // blocks of 8 warps covering n rows (a multiple of 32) with G warps per slice
 unsigned split_blocks(int64_t n, int g) { return nblk(n / kS * g, 8); }
 unsigned row_blocks(const AmgLevel &L) { return L.pipe ? L.pipe : split_blocks(L.A.n, L.g); }
-constexpr unsigned kAheadBlocks = 4 * 148;
 template <int OP> void launch_rows(const AmgLevel &L, RowArgs a, cudaStream_t s, bool chained) {
     a.A = view(L.A);
     a.longrows = L.A.longrows;
     a.n_long = (int32_t)std::max<int64_t>(0, L.A.n_long);
     a.row_blocks = row_blocks(L);
     const unsigned grid = a.row_blocks + (unsigned)a.n_long;
-    const auto k = L.pipe ? k_rows_pipe<OP> : grid <= kAheadBlocks ? rows_kernel<OP, true>(L.g) : rows_kernel<OP, false>(L.g);
+    const auto k = L.pipe ? k_rows_pipe<OP> : L.ahead ? rows_kernel<OP, true>(L.g) : rows_kernel<OP, false>(L.g);
     launch_chained(chained, k, grid, 256, s, a);
 }
 // warps per slice for a matrix: the fewest with at most `width` slots per warp and row (one on
@@ -2755,6 +2754,8 @@ cudaError_t Amg::setup(const DevSystem &sys, const AmgOptions &o, cudaStream_t s
             // levels with at least two slices for every warp of the chip (three blocks of eight to
             // an SM): the persistent row kernels
             lv_[l].pipe = lv_[l].A.rlen && lv_[l].A.n_slices >= 2 * 8 * 3 * (int64_t)sms_ ? 3u * (unsigned)sms_ : 0u;
+            // one wave at four blocks an SM: the row kernels that load columns ahead (k_rows)
+            lv_[l].ahead = row_blocks(lv_[l]) + (unsigned)std::max(0, nlong[l]) <= 4u * (unsigned)sms_;
         }
         if ((e2 = power_estimates(s)) != cudaSuccess) return e2;
         if (opt_.power_steps > 0) {

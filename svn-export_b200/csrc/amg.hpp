@@ -93,6 +93,7 @@ struct AmgLevel {
     float gershgorin = 2.f;                    // Gershgorin bound of D^-1 A
     int g = 1;                                 // warps per slice in the row kernels (amg.cu)
     unsigned pipe = 0;                         // blocks of the persistent row kernels (0: not for this level)
+    bool ahead = false;                        // the row kernels load columns before they wait
 };
 
 // Events recorded inside a captured V-cycle (as external event nodes) to time it: the whole
