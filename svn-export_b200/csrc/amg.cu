@@ -834,16 +834,6 @@ __global__ void k_dense_scatter(MatView A, int n, int np, double *M, double *dia
     diag[i] = M[(size_t)i * np + i];
 }
 
-// 1 / x to the last bit or so, for x from 1e-300 to 1e300: the hardware's 20-bit approximation (subnormal
-// operands are zero to it) and two Newton steps (a quarter of the latency of the full division, which is
-// the pivots' critical path)
-__device__ __forceinline__ double quick_rcp(double x) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    r = fma(r, fma(-x, r, 1.0), r);
-    return fma(r, fma(-x, r, 1.0), r);
-}
-
 // The inverse of a 32 x 32 block by the 256 threads of a block: thread t holds m, four entries of
 // row r = t / 8 from column c4 = 4 (t % 8) on.  Pivot p: with a 1 in the pivot's place of row p, zeros
 // left behind in row p and column p, and the factor -1 for row p, every entry is m -= f / pivot * row_p.
@@ -872,7 +862,7 @@ __device__ __forceinline__ void gj_invert(double (&m)[4], int r, int c4, double 
             const double piv = cb[p];
             bad |= !(piv > 1e-300 && piv < 1e300);
             lost |= !(piv > (double)FLT_EPSILON * diag[p]);
-            const double g = (r == p ? -1.0 : cb[r]) * quick_rcp(piv);
+            const double g = (r == p ? -1.0 : cb[r]) / piv;
 #pragma unroll
             for (int q = 0; q < 4; ++q) m[q] = fma(-g, rb[c4 + q], m[q]);
         }
