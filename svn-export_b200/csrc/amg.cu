@@ -1407,7 +1407,7 @@ __device__ void dots_finish(const RowArgs &a, double xb, double xax, bool has_te
 // G warps per slice (split_row).  What the matrix says is loaded before the wait for the kernel
 // before: the row's extent and, AHEAD, its first columns.  Those cost registers, so AHEAD is for grids
 // that run in one wave at four blocks an SM; larger ones need eight (149k rows in 1164 blocks: 8.5 us a
-// pass at 40 registers, 5.4 at 32).
+// pass at 40 registers, 5.4 at 32, though kRowDots spills 36-44 bytes there).
 template <int G, int OP, bool AHEAD> __global__ void __launch_bounds__(256, AHEAD ? 4 : 8) k_rows(RowArgs a) {
     if (blockIdx.x >= a.row_blocks) {
         pdl_wait();
@@ -1572,7 +1572,7 @@ __device__ __forceinline__ float fine_step(float b, float w, float y, float d, f
 // offset of the one after are too.
 // Rows outside the hierarchy are one bit each (a word per slice).
 // Measured (B200, us a kernel, one row per thread with the diagonal read -> this): 3.19M rows 39-42 ->
-// 29 (52 bytes a row at 5.7 TB/s), 10.95M rows 139-150 -> 107-122.  16-bit columns relative to
+// 29 (52 bytes a row at 5.7 TB/s), 10.95M rows 139-150 -> 107-124.  16-bit columns relative to
 // two bases per slot position (26 bytes a row's slots instead of 36) were no faster unpipelined
 // (37-39, 154-163) and lost the pipeline where decoding waits for the bases.
 struct FineView {

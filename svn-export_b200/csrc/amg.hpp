@@ -50,7 +50,10 @@ struct AmgOptions {
     int coarse_degree = 12;     // Chebyshev degree of a smoothed (not inverted) coarsest level
     float coarse_ratio = 50.f;  // ... on [hi / coarse_ratio, hi]
     int stall_rows = 16384; // after two coarsenings in a row that kept more than half of the rows, a
-                            // next level of at most this many rows is the coarsest (0: off)
+                            // next level of at most this many rows is the coarsest (0: off).  Fractured
+                            // cubes, n = 72-96, 10 systems, ms to 1e-12 at 16384 / 32768: 112/105,
+                            // 86/86, 136/129, 145/133, 181/215, 664/664, 427/398, 323/348, 421/430,
+                            // 262/256: it turns on the system, by up to a fifth either way
     int fine_tma = 0;       // 1: the fine level's cycle kernels stream the matrix through shared
                             // memory with TMA bulk copies (with half_fine; amg.cu k_fine_tma)
     int fine_tma_stages = 4;  // ... in a ring of 2 or 4 stages

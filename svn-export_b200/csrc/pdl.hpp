@@ -3,7 +3,7 @@
 // A multigrid cycle is 23-70 kernels of 2-3 us on small levels, and of those 2-3 us about half is
 // the launch and the first dependent loads.  Measured (B200, us an iteration of the flexible CG without
 // -> with): 52k edges 83 -> 66, 115k 93 -> 78, 404k 151 -> 137, 1.35M 288 -> 243, 3.2M 498 -> 456,
-// 11M 2025 -> 1940.  Letting the next kernel come up behind the wait instead of before it gave 67, 78, 138,
+// 11M 2025 -> 1940 (all with FP32 vectors in the flexible CG, learned.cu).  Letting the next kernel come up behind the wait instead of before it gave 67, 78, 138,
 // 247, 460, 1946; at the kernel's very start 67, 80, 139, 245, 459, 1942.
 // The Chebyshev polynomial's steps: 28 -> 23 us an iteration (13k edges), 44 -> 38 (175k), 83 -> 73 (404k).
 // Not the two kernels of plain CG: 65.4 -> 61.7 ms for a batch of four small systems, but 32.8 -> 34.1 us an

@@ -128,8 +128,10 @@ template <typename T> __device__ __forceinline__ void cg_step(T q, double alpha,
 }
 
 // The run's scalars; only warp 0 works on them.  REG: rho, rr, tol2 and the counts in registers, which
-// saves 0.15 us an iteration of loads in a serial chain, but costs every thread ten; the kernels of three
-// and four rows a thread would spill for them (n = 35 FP32: 8.0 us an iteration against 7.6).
+// saves 0.15 us an iteration of loads in a serial chain, but costs every thread ten of the 64 that 1024
+// threads have.  The chip-wide kernels spill there: 32 bytes (FP64) and 16 (FP32) with two rows a thread,
+// 44 with three (FP64), 68 and 40 with four; those of three and four go without REG (n = 35 FP32: 8.0 us
+// an iteration with it against 7.6).
 struct RunState {
     double rho, rr, alpha, beta, tol2;
     int iter0, max_it, state;  // state 0: go on, 1: converged, 2: iteration cap, 3: breakdown, 4: not finite
