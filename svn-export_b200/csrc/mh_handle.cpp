@@ -669,7 +669,11 @@ int run_resident(mh_handle *h, int prec, const Restart &restart, bool &done) {
     const int gi = prec == 64 ? 0 : 1;
     const size_t bytes = (size_t)h->sys.n_rows * sizeof(double);
     int polls = mh::kResidentPolls;
-    if (const char *e = getenv("MH_RESIDENT_POLLS")) polls = std::max(0, std::min(polls, atoi(e)));
+    if (const char *e = getenv("MH_RESIDENT_POLLS")) {
+        char *end = nullptr;
+        const long v = std::strtol(e, &end, 10);
+        if (end != e && v >= 0 && v < polls) polls = (int)v;
+    }
     // the FP64 run works on x itself; q is idle in it (the FP32 run leaves x alone)
     if (prec == 64) CK(cudaMemcpyAsync(h->sys.q, h->sys.x, bytes, cudaMemcpyDeviceToDevice, h->stream));
     const cudaError_t e = mh::launch_cg_resident(h->sys, h->res_plan[gi], h->res_dev[gi], polls, h->stream);

@@ -55,3 +55,12 @@ def test_wait_that_runs_out_from_a_guess(gpu, monkeypatch):
         monkeypatch.setenv("MH_RESIDENT_POLLS", "0")
         st = s.solve(r_tol=1e-12, use_initial_guess=True)
         assert st["iterations"] == host["iterations"] and np.array_equal(s.solution(), xh)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("polls", ["", "many", "-1", "99999999999"])
+def test_only_a_smaller_number_shortens_the_wait(gpu, monkeypatch, polls):
+    monkeypatch.setenv("MH_RESIDENT_POLLS", polls)
+    with system(14) as s:
+        st = s.solve(r_tol=1e-10)
+        assert st["status"] == 0 and st["kernel_launches"] < st["iterations"]
